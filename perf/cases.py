@@ -133,7 +133,7 @@ def _options(case, seed):
 
 def _problem(case, seed):
     with tempfile.TemporaryDirectory() as tmp:
-        return Problem.load(_files(case, seed, tmp), _grid(case), fourthorder="pairs" in case, readiso=True)
+        return Problem.load(_files(case, seed, tmp), _grid(case), fourthorder="pairs" in case)
 
 
 def _lists(case, seed, prob, opts):
@@ -181,7 +181,7 @@ def run(s):
         (ks * s.kappa_bar).sum().backward()
         out = {"linewidth": lw.detach().numpy(), "kappa_sma": ks.detach().numpy(), "grad": fc3.grad.numpy()}
     elif s.case["op"] == "program":
-        prob = Problem.load(s.dir, _grid(s.case), readiso=True, device=0)
+        prob = Problem.load(s.dir, _grid(s.case), device=0)
         sr = ScatteringRates(prob)
         lw = sr.generate(s.opts)
         koff = sr.kappa_offdiag(s.opts)
