@@ -44,8 +44,9 @@ def listed():
         # mesh; three atoms, an odd mesh
         dict(name="fluorite11_mc_mixed", op="solve", cell="fluorite", mesh=11, it=2, precision="mixed", isotope=True,
              sub=6),
-        # four atoms, velocity-difference smearing, odd mesh, FP64
-        dict(name="l12_9_fp64", op="solve", cell="l12", mesh=9, it=6, precision="fp64", isotope=True),
+        # four atoms, velocity-difference smearing, odd mesh, FP64; without isotopes, whose terms
+        # between a mode at rest and itself outweigh everything else with this smearing
+        dict(name="l12_9_fp64", op="solve", cell="l12", mesh=9, it=6, precision="fp64", isotope=False),
         # five atoms in FP64: the reference run against which a mixed one is checked
         dict(name="perovskite8_fp64", op="solve", cell="perovskite", mesh=8, it=2, precision="fp64", isotope=False),
         # the benchmark's default workload: five atoms, 16^3, uneven samples per q1, mixed
