@@ -12,12 +12,6 @@ namespace {
 
 constexpr double kIsotopePrefactor = 3.141592653589793 / 4.0;
 
-__device__ __forceinline__ double lo_gauss(double x, double mu, double sigma) {
-    if (fabs(x - mu) > 8.0 * sigma) return 0.0;
-    const double invsig = 1.0 / sigma;
-    return exp(-(x - mu) * (x - mu) * 0.5 * invsig * invsig) * kSqrt2PiInv * invsig;
-}
-
 __device__ __forceinline__ double block_sum(double v, double *sh) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -30,58 +24,105 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
     return s;
 }
 
-// compute_isotope_scattering (scattering_isotope.f90:1-91): one thread per (q2, b2) of a row.
-__global__ void k_isotope(MeshDev m, PhononDev ph, RowsDev rows, const int32_t *row_q1, const int32_t *row_b1,
-                          const double *disorder, int32_t n_atom, double *gamma, double *xi) {
+// compute_isotope_scattering (scattering_isotope.f90:1-91). A CTA takes kIsoCols columns
+// (q2, b2) of one row: an FP32 screen of the one Gaussian against its 8-sigma window (the
+// margins of the three-phonon screen: a column it drops is exactly 0 in the reference), the
+// survivors compacted into a queue, then the strength, width and Gaussian in FP64 by full
+// warps. Bound: the FP64 pipe (2 lanes per clock and SM) for the survivors, a few per cent
+// of the columns with adaptive widths. Forming the strength of every column first, with its
+// 3 square roots per atom, cost 16.3 ms at perovskite 12^3 (32.6 M columns).
+// |conj(u) v| = |u| |v|: the magnitudes are made once per mode and component
+// (k_iso_mag), which leaves 3 products and 2 FMAs per atom.
+constexpr int kIsoCols = 2048;
+
+__global__ void k_iso_mag(int64_t ne, const double2 *egv, double *mag) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < ne) mag[i] = sqrt(egv[i].x * egv[i].x + egv[i].y * egv[i].y);
+}
+
+// Smearing width of -it 6 (scattering_isotope.f90:45-52): the velocity of (q2, b2) alone.
+__device__ __forceinline__ double iso_width6(const PhononDev &ph, int64_t j) {
+    const double *v = ph.vel + j * 3;
+    double mx = 0.0;
+    for (int jj = 0; jj < 3; ++jj) {
+        double s = 0.0;
+        for (int i = 0; i < 3; ++i) s += v[i] * ph.reclat_g[i + 3 * jj];
+        mx = fmax(mx, s * s);
+    }
+    return sqrt(mx * 0.5) + ph.thresh_sigma;
+}
+
+// What the screen reads of a column: omega2 (NaN below 1e-9 Ha, which no window holds) and
+// its share of the width (sigsq for -it 2, the width itself for -it 6).
+__global__ void k_iso_cols(MeshDev m, PhononDev ph, float2 *col) {
+    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= (int64_t)m.n_full * m.n_mode) return;
+    const int q2 = (int)(j / m.n_mode), b2 = (int)(j % m.n_mode);
+    float w = 0.f;
+    if (ph.integrationtype == 2) w = ph.sigsq32[(size_t)m.full_irr[q2] * m.n_mode + b2];
+    if (ph.integrationtype == 6) w = (float)iso_width6(ph, j);
+    col[j] = make_float2(ph.omega[j] < kFreqTolD ? __int_as_float(0x7fc00000) : ph.omega32[j], w);
+}
+
+__global__ void __launch_bounds__(256) k_isotope(MeshDev m, PhononDev ph, const int32_t *row_q1, const int32_t *row_b1,
+                                                 const float2 *col, const double *mag, const double *disorder,
+                                                 int32_t n_atom, double *gamma, double *xi) {
+    constexpr int kPer = kIsoCols / 256;
     __shared__ double sh[32];
-    const int n = m.n_mode;
+    __shared__ int wsum[33];
+    __shared__ uint16_t queue[kIsoCols];
+    const int n = m.n_mode, it = ph.integrationtype;
     const int r = blockIdx.y;
     const int q1 = row_q1[r], b1 = row_b1[r];
     const int f1 = m.irr_full[q1];
     const int64_t ld = (int64_t)m.n_full * n;
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    double f0 = 0.0;
-    if (j < ld) {
-        const int q2 = (int)(j / n), b2 = (int)(j % n);
-        const double om1 = ph.omega[(size_t)f1 * n + b1];
-        const double om2 = ph.omega[(size_t)q2 * n + b2];
-        if (!(om2 < kFreqTolD)) {
-            double sigma;
-            if (ph.integrationtype == 1) {
-                sigma = ph.sigma_fixed;
-            } else if (ph.integrationtype == 2) {
-                sigma = sqrt(ph.sigsq[(size_t)q1 * n + b1] + ph.sigsq[(size_t)m.full_irr[q2] * n + b2]);
-            } else {
-                const double *v = ph.vel + ((size_t)q2 * n + b2) * 3;
-                double mx = 0.0;
-                for (int jj = 0; jj < 3; ++jj) {
-                    double s = 0.0;
-                    for (int i = 0; i < 3; ++i) s += v[i] * ph.reclat_g[i + 3 * jj];
-                    mx = fmax(mx, s * s);
-                }
-                sigma = sqrt(mx * 0.5) + ph.thresh_sigma;
-            }
-            const double2 *e1 = ph.egv + ((size_t)f1 * n + b1) * n;
-            const double2 *e2 = ph.egv + ((size_t)q2 * n + b2) * n;
-            double f1s = 0.0;
-            for (int a = 0; a < n_atom; ++a) {
-                double fa = 0.0;
-                for (int x = 0; x < 3; ++x) {
-                    const double2 u = e1[a * 3 + x], v = e2[a * 3 + x];
-                    // |conjg(u) * v|
-                    const double re = u.x * v.x + u.y * v.y, im = u.x * v.y - u.y * v.x;
-                    fa += sqrt(re * re + im * im);
-                }
-                fa = fa * fa;
-                f1s += fa * disorder[a];
-            }
-            const double prefactor = kIsotopePrefactor * (1.0 / (double)m.n_full);
-            const double psisq = f1s * prefactor;
-            f0 = psisq * om1 * om2 * lo_gauss(om1, om2, sigma);
-            if (f0 != 0.0) xi[(int64_t)r * ld + j] += f0 * om2 / om1;
-        }
+    const int64_t j0 = (int64_t)blockIdx.x * kIsoCols;
+    const float fo1 = ph.omega32[(size_t)f1 * n + b1], fs1 = ph.sigsq32[(size_t)q1 * n + b1];
+    const float sigfix = (float)ph.sigma_fixed;
+    uint32_t live = 0u;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int64_t j = j0 + u * 256 + threadIdx.x;
+        if (j >= ld) continue;
+        const float2 c = __ldg(col + j);
+        const float sg = it == 1 ? sigfix : (it == 2 ? sqrt_screen(fs1 + c.y) : c.y);
+        if (fabsf(fo1 - c.x) <= 8.0f * sg * 1.001f + 1e-6f * (fo1 + c.x)) live |= 1u << u;
     }
-    const double s = block_sum(f0, sh);
+    int nq = 0;
+    int k = block_exclusive_scan(__popc(live), wsum, nq);
+    for (; live; live &= live - 1) queue[k++] = (uint16_t)((__ffs(live) - 1) * 256 + threadIdx.x);
+    __syncthreads();
+    if (nq == 0) return;
+    const double om1 = ph.omega[(size_t)f1 * n + b1], inv1 = ph.inv_omega[(size_t)f1 * n + b1];
+    const double *e1 = mag + ((size_t)f1 * n + b1) * n;
+    const double prefactor = kIsotopePrefactor * (1.0 / (double)m.n_full);
+    double sum = 0.0;
+    for (int i = threadIdx.x; i < nq; i += 256) {
+        const int64_t j = j0 + queue[i];
+        const double om2 = ph.omega[j];
+        double sigma;
+        if (it == 1) {
+            sigma = ph.sigma_fixed;
+        } else if (it == 2) {
+            const int q2 = (int)(j / n), b2 = (int)(j - (int64_t)q2 * n);
+            sigma = sqrt(ph.sigsq[(size_t)q1 * n + b1] + ph.sigsq[(size_t)m.full_irr[q2] * n + b2]);
+        } else {
+            sigma = iso_width6(ph, j);
+        }
+        if (fabs(om1 - om2) > 8.0 * sigma) continue;
+        const double invsig = 1.0 / sigma;
+        const double *e2 = mag + j * n;
+        double strength = 0.0;
+        for (int a = 0; a < n_atom; ++a) {
+            const double fa = e1[3 * a] * e2[3 * a] + e1[3 * a + 1] * e2[3 * a + 1] + e1[3 * a + 2] * e2[3 * a + 2];
+            strength = fma(fa * fa, disorder[a], strength);
+        }
+        const double dx = om1 - om2;
+        const double f0 = strength * prefactor * om1 * om2 * (exp_neg(dx * dx * 0.5 * invsig * invsig, ph.exp2tab) * kSqrt2PiInv * invsig);
+        if (f0 != 0.0) xi[(int64_t)r * ld + j] += f0 * om2 * inv1;
+        sum += f0;
+    }
+    const double s = block_sum(sum, sh);
     if (threadIdx.x == 0 && s != 0.0) atomicAdd(gamma + r, s);
 }
 
@@ -509,13 +550,20 @@ __global__ void k_xi_reduce(const double *part, int32_t n_row, int split, double
 
 }  // namespace
 
+cudaError_t launch_iso_mag(int64_t ne, const double2 *egv, double *mag, cudaStream_t s) {
+    if (ne <= 0) return cudaSuccess;
+    k_iso_mag<<<(unsigned)((ne + 255) / 256), 256, 0, s>>>(ne, egv, mag);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_isotope(const MeshDev &m, const PhononDev &ph, const RowsDev &rows, const int32_t *row_q1,
-                           const int32_t *row_b1, const double *disorder, int32_t n_atom, double *gamma,
-                           double *xi, cudaStream_t s) {
+                           const int32_t *row_b1, float2 *col, const double *mag, const double *disorder,
+                           int32_t n_atom, double *gamma, double *xi, cudaStream_t s) {
     if (rows.n_row <= 0) return cudaSuccess;
     const int64_t ld = (int64_t)m.n_full * m.n_mode;
-    dim3 grid((unsigned)((ld + 255) / 256), (unsigned)rows.n_row);
-    k_isotope<<<grid, 256, 0, s>>>(m, ph, rows, row_q1, row_b1, disorder, n_atom, gamma, xi);
+    k_iso_cols<<<(unsigned)((ld + 255) / 256), 256, 0, s>>>(m, ph, col);
+    dim3 grid((unsigned)((ld + kIsoCols - 1) / kIsoCols), (unsigned)rows.n_row);
+    k_isotope<<<grid, 256, 0, s>>>(m, ph, row_q1, row_b1, col, mag, disorder, n_atom, gamma, xi);
     return cudaGetLastError();
 }
 

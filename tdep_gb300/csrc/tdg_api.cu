@@ -210,6 +210,9 @@ struct tdg_ctx {
     DevBuf<float2> tw32;
     DevBuf<double> d_exp2tab, d_invom;
     DevBuf<float> d_om32, d_sigsq32;
+    // isotope scattering: magnitudes of the eigenvector components (first use), screen columns
+    DevBuf<double> d_iso_mag;
+    DevBuf<float2> d_iso_col;
     int L = 1, lmul[3] = {1, 1, 1};
     // scattering state
     int n_row = 0;
@@ -1304,6 +1307,13 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
             chk(c->d_list3.upload(ql->list3, ql->ptr3[nr], s));
         }
     }
+    if (o->isotope) {
+        chk(c->d_iso_col.alloc((size_t)ld));
+        if (c->d_iso_mag.n == 0) {
+            chk(c->d_iso_mag.alloc((size_t)ld * n));
+            if (e == cudaSuccess) chk(launch_iso_mag(ld * n, c->d_egv.p, c->d_iso_mag.p, s));
+        }
+    }
     if (o->fourthorder) {
         chk(c->d_cand4.upload(cand4.data(), cand4.size(), s));
         chk(c->d_mask4.upload(masks4.data(), masks4.size(), s));
@@ -1560,9 +1570,9 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
     }
     CUDA_TRY(cudaEventRecord(ev[4], s));
     if (o->isotope) {
-        CUDA_TRY(launch_isotope(mesh, ph, rows, c->d_row_q1.p, c->d_row_b1.p, c->d_disorder.p, c->na, c->d_gamma.p,
-                                c->d_xi.p, s));
-        ++launches;
+        CUDA_TRY(launch_isotope(mesh, ph, rows, c->d_row_q1.p, c->d_row_b1.p, c->d_iso_col.p, c->d_iso_mag.p,
+                                c->d_disorder.p, c->na, c->d_gamma.p, c->d_xi.p, s));
+        launches += 2;
     }
     CUDA_TRY(cudaEventRecord(ev[5], s));
     // ---- gamma to host; symmetrize_scatmat on the device meanwhile ----

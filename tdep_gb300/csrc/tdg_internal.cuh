@@ -282,10 +282,13 @@ cudaError_t launch_ln_batch(const LnBatch &b, cudaStream_t s);
 // gradient of the mass-weighted force constants added into grad_hi/grad_lo.
 cudaError_t launch_ln_adjoint_batch(const LnBatch &b, cudaStream_t s);
 
-// Isotope scattering (scattering_isotope.f90): adds into gamma and xi.
+// Isotope scattering (scattering_isotope.f90): adds into gamma and xi. mag: the magnitudes of
+// the eigenvector components ([n_full*n*n], launch_iso_mag, once per context); col: work
+// array of n_full*n entries.
+cudaError_t launch_iso_mag(int64_t ne, const double2 *egv, double *mag, cudaStream_t s);
 cudaError_t launch_isotope(const MeshDev &m, const PhononDev &ph, const RowsDev &rows, const int32_t *row_q1,
-                           const int32_t *row_b1, const double *disorder, int32_t n_atom, double *gamma,
-                           double *xi, cudaStream_t s);
+                           const int32_t *row_b1, float2 *col, const double *mag, const double *disorder,
+                           int32_t n_atom, double *gamma, double *xi, cudaStream_t s);
 
 // Context tables built on the device: the rotation table rot[op][q] (integer rotation of
 // fractional reciprocal coordinates on the mesh, -1 off the mesh) and the eigenvectors
