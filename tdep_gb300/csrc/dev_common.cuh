@@ -82,6 +82,25 @@ __device__ __forceinline__ float2 df_merge(float2 a, float2 b) {
     return make_float2(t, a.y + b.y + e);
 }
 
+// x = hi + lo by integer operations on the bits (double <-> float conversions run on the
+// FP64 pipe): hi keeps the leading 24 significant bits of x, lo the remaining 29 rounded to
+// 24, so hi + lo = x to 2^-48 relative. Zero and subnormal doubles give 0; magnitudes
+// outside [2^-74, 2^127) take the FP64 conversions.
+__device__ __forceinline__ float2 split_df(double x) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int e = (int)((b >> 52) & 0x7FF);
+    if (e == 0) return make_float2(0.f, 0.f);
+    if (e < 949 || e > 1150) {
+        const float h = (float)x;
+        return make_float2(h, (float)(x - (double)h));
+    }
+    const unsigned int sign = (unsigned int)(b >> 32) & 0x80000000u;
+    const float hi = __uint_as_float(sign | ((unsigned int)(e - 896) << 23) | (unsigned int)((b >> 29) & 0x7FFFFFu));
+    // remainder r * 2^(e - 1075), r < 2^29; the power of two is a normal float for e >= 949
+    const float lo = __uint2float_rn((unsigned int)(b & 0x1FFFFFFFu)) * __uint_as_float((unsigned int)(e - 948) << 23);
+    return make_float2(hi, sign ? -lo : lo);
+}
+
 // Square root by the hardware approximation (sqrt.approx.f32, a few ulp): for the FP32
 // screens, whose windows carry a relative margin of 1e-3.
 __device__ __forceinline__ float sqrt_screen(float x) {

@@ -243,7 +243,7 @@ struct tdg_ctx {
     DevBuf<QuartetRec> d_quart;
     DevBuf<unsigned char> d_scr4;
     // BTE buffers
-    DevBuf<double> d_buf, d_part;
+    DevBuf<double> d_part;
     DevBuf<float2> d_fbb;   // F as double-float pairs for the BTE product
     DevBuf<float4> d_xi_df;  // Xi as double-float row pairs (launch_split_xi)
     // state of the last tdg_scattering that the adjoint pass reuses
@@ -274,8 +274,8 @@ struct tdg_ctx {
     GraphSlot graph_bte;                  // a chunk of BTE iterations (tdg_kappa)
     int kappa_calls = 0;
     // BTE iteration state on the device
-    DevBuf<double> d_fnb, d_scf, d_qs_bte, d_F0, d_bte_part;
-    DevBuf<int32_t> d_deg_irr, d_dm_irr;
+    DevBuf<double> d_scf, d_qs_bte, d_F0, d_bte_change;
+    DevBuf<int32_t> d_deg_irr, d_dm_irr, d_chain, d_star_ptr, d_star, d_arrived;
     DevBuf<BteCtl> d_ctl;
     bool last_ln = false;  // the last tdg_scattering took the large-cell (tensor-core) path
     int last_ln_tune = 324;  // its launch shape (delta row block * 10 + GEMM stages)
@@ -1836,7 +1836,7 @@ extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double 
     int iters = 0;
     if (maxiter > 0) {
         const int64_t ncol = (int64_t)N * n;
-        const size_t nfn = (size_t)nirr * n * 3, nbuf = (size_t)nr * 3;
+        const size_t nfn = (size_t)nirr * n * 3;
         CUDA_TRY(c->d_fbb.alloc((size_t)ncol * 3));
         // the Xi.F products take Xi as double-float row pairs (k_xi_gemv; floats fail the
         // mixed iteration's convergence test)
@@ -1845,15 +1845,14 @@ extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double 
             CUDA_TRY(launch_split_xi(c->d_xi.p, nr, ncol, c->d_xi_df.p, s));
             c->xi_fmt = 1;
         }
-        CUDA_TRY(c->d_buf.alloc(nbuf));
         CUDA_TRY(c->d_part.alloc(xi_gemv_part_elems(nr)));
         CUDA_TRY(c->d_fn.alloc(nfn));
         if (c->d_full_op.n == 0) {
             CUDA_TRY(c->d_full_op.upload(c->full_op.data(), N, s));
             CUDA_TRY(c->d_op_cart.upload(c->op_cart.data(), c->op_cart.size(), s));
         }
-        // The whole iteration runs on the device (kappa.f90:382-490): foldout, the three Xi
-        // products and the scalar recurrences (k_bte_update), in chunks of kBteChunk
+        // The whole iteration runs on the device (kappa.f90:382-490): the three Xi
+        // products, then the scalar recurrences and the foldout (k_bte_update), in chunks of kBteChunk
         // iterations between host checks of the done flag; a chunk is replayed as a CUDA
         // graph from its second use. Fn goes up once and comes back once.
         if (c->d_deg_irr.n == 0) {
@@ -1866,13 +1865,23 @@ extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double 
                         dm[((size_t)q1 * n + b1) * n + j] = c->degen_mode[((size_t)f * n + b1) * n + j];
                 }
             }
+            std::vector<int32_t> chain((size_t)nirr * n), sp(nirr + 1, 0), star(N);
+            bte_chains(nirr, n, dg.data(), dm.data(), chain.data());
+            for (int q = 0; q < N; ++q) ++sp[c->full_irr[q]];
+            for (int q1 = 0; q1 < nirr; ++q1) sp[q1 + 1] += sp[q1];
+            std::vector<int32_t> at(sp.begin(), sp.end() - 1);
+            for (int q = 0; q < N; ++q) star[at[c->full_irr[q] - 1]++] = q;
             CUDA_TRY(c->d_deg_irr.upload(dg.data(), dg.size(), s));
             CUDA_TRY(c->d_dm_irr.upload(dm.data(), dm.size(), s));
+            CUDA_TRY(c->d_chain.upload(chain.data(), chain.size(), s));
+            CUDA_TRY(c->d_star_ptr.upload(sp.data(), sp.size(), s));
+            CUDA_TRY(c->d_star.upload(star.data(), star.size(), s));
         }
-        CUDA_TRY(c->d_fnb.alloc(nfn));
         CUDA_TRY(c->d_scf.alloc((size_t)maxiter));
         CUDA_TRY(c->d_ctl.alloc(1));
-        CUDA_TRY(c->d_bte_part.alloc((size_t)bte_part_elems(nirr)));
+        CUDA_TRY(c->d_bte_change.alloc(nirr));
+        CUDA_TRY(c->d_arrived.alloc(1));
+        CUDA_TRY(cudaMemsetAsync(c->d_arrived.p, 0, sizeof(int32_t), s));
         CUDA_TRY(c->d_qs_bte.upload(c->qs.data(), c->qs.size(), s));
         CUDA_TRY(c->d_F0.upload(c->F0.data(), nfn, s));
         CUDA_TRY(copy_async(c->d_fn.p, Fn.data(), sizeof(double) * nfn, cudaMemcpyHostToDevice, s));
@@ -1886,21 +1895,28 @@ extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double 
         bd.maxiter = maxiter;
         bd.tol = tol;
         bd.sqtol = kSqTol;
+        bd.part = c->d_part.p;
         bd.rowidx = c->d_rowidx.p;
-        bd.part = c->d_bte_part.p;
         bd.qs = c->d_qs_bte.p;
         bd.F0 = c->d_F0.p;
         bd.degen = c->d_deg_irr.p;
         bd.degen_mode = c->d_dm_irr.p;
+        bd.chain = c->d_chain.p;
+        bd.star_ptr = c->d_star_ptr.p;
+        bd.star = c->d_star.p;
+        bd.full_op = c->d_full_op.p;
+        bd.op_cart = c->d_op_cart.p;
         bd.fn = c->d_fn.p;
-        bd.fnb = c->d_fnb.p;
+        bd.fbb = c->d_fbb.p;
         bd.scf = c->d_scf.p;
+        bd.change = c->d_bte_change.p;
+        bd.arrived = c->d_arrived.p;
         bd.ctl = c->d_ctl.p;
         const int32_t *done = &c->d_ctl.p->done;
         // column split of the Xi products, autotuned per problem size on F0's foldout
         int split = 0;
+        CUDA_TRY(launch_bte_foldout(bd, s));
         {
-            CUDA_TRY(launch_foldout(N, n, c->d_full_op.p, c->d_full_irr.p, c->d_op_cart.p, c->d_fn.p, c->d_fbb.p, s));
             // shapes: rows per CTA (4, 8) * 100 + column ranges (the default, twice it)
             const int s0 = xi_gemv_default_split(nr, ncol, c->n_sm), smax = xi_gemv_max_split(ncol);
             std::vector<int> cand;
@@ -1913,19 +1929,18 @@ extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double 
             bool tuned = false;
             CUDA_TRY(tune_pick(tune_key(key.str().c_str(), n, 0, c->device), cand, 400 + s0,
                                [&](int v) {
-                                   return launch_xi_gemv(c->d_xi_df.p, nr, ncol, c->d_fbb.p, c->d_part.p,
-                                                         c->d_buf.p, c->n_sm, s, nullptr, v);
+                                   return launch_xi_gemv(c->d_xi_df.p, nr, ncol, c->d_fbb.p, c->d_part.p, s,
+                                                         nullptr, v);
                                },
                                s, split, tuned));
         }
+        // a decision read from a file may be any number
+        bd.split = std::min(std::max(split % 100, 1), xi_gemv_max_split(ncol));
+        split = (split / 100 == 8 ? 800 : 400) + bd.split;
         auto iterations = [&](int k) -> cudaError_t {
             for (int j = 0; j < k; ++j) {
-                cudaError_t e = launch_foldout(N, n, c->d_full_op.p, c->d_full_irr.p, c->d_op_cart.p, c->d_fn.p,
-                                               c->d_fbb.p, s, done);
-                if (e == cudaSuccess)
-                    e = launch_xi_gemv(c->d_xi_df.p, nr, ncol, c->d_fbb.p, c->d_part.p, c->d_buf.p, c->n_sm, s,
-                                       done, split);
-                if (e == cudaSuccess) e = launch_bte_update(bd, c->d_buf.p, s);
+                cudaError_t e = launch_xi_gemv(c->d_xi_df.p, nr, ncol, c->d_fbb.p, c->d_part.p, s, done, split);
+                if (e == cudaSuccess) e = launch_bte_update(bd, s);
                 if (e != cudaSuccess) return e;
             }
             return cudaSuccess;
@@ -1937,8 +1952,7 @@ extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double 
             std::ostringstream key;
             key << k << '/' << split << '/' << std::string(reinterpret_cast<const char *>(&bd), sizeof bd)
                 << '/'
-                << (const void *)c->d_xi_df.p << (const void *)c->d_fbb.p << (const void *)c->d_part.p
-                << (const void *)c->d_buf.p << (const void *)c->d_fn.p << ncol;
+                << (const void *)c->d_xi_df.p << ncol;
             // recorded only from the context's second kappa call on: a context that solves
             // once would pay for the recording without replaying it much
             CUDA_TRY(run_graph_region(c, c->graph_bte, key.str(), s, [&]() { return iterations(k); },

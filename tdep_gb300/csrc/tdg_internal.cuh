@@ -345,10 +345,9 @@ cudaError_t launch_sym_tile_adjoint(const MeshDev &m, const OrbitDev &o, int32_t
 size_t xi_pairs_elems(int32_t n_row, int64_t n_col);
 cudaError_t launch_split_xi(const double *xi, int32_t n_row, int64_t n_col, float4 *out, cudaStream_t s);
 size_t xi_gemv_part_elems(int32_t n_row);
-// shape: rows per CTA (4 or 8) * 100 + column ranges per row group (0: 4 rows and a default
-// split sized for about two waves).
+// shape: rows per CTA (4 or 8) * 100 + column ranges per row group.
 cudaError_t launch_xi_gemv(const float4 *xi, int32_t n_row, int64_t n_col, const float2 *fbb, double *part,
-                           double *buf, int n_sm, cudaStream_t s, const int32_t *skip = nullptr, int shape = 0);
+                           cudaStream_t s, const int32_t *skip, int shape);
 int xi_gemv_default_split(int32_t n_row, int64_t n_col, int n_sm);
 int xi_gemv_max_split(int64_t n_col);
 
@@ -356,13 +355,6 @@ int xi_gemv_max_split(int64_t n_col);
 // splits; variant selects the operand layout reading (diagnostic).
 cudaError_t launch_mma_check(int variant, int n, const float *a, const float *b, float *d, int *status,
                              cudaStream_t s);
-
-// foldout of the BTE: fbb[(q*n + b)*3 + d] = sign * (R fn[(irr(q)*n + b)*3 ..])_d, with
-// full_op signed 1-based operations (negative: time reversal) and full_irr 0-based; stored
-// as (hi, lo) float pairs (the Xi.F element format).
-cudaError_t launch_foldout(int32_t n_full, int32_t n_mode, const int32_t *full_op, const int32_t *full_irr,
-                           const double *op_cart, const double *fn, float2 *fbb, cudaStream_t s,
-                           const int32_t *skip = nullptr);
 
 // Device state of the BTE iteration (kappa.f90:326-495): the iteration counter, the mixing
 // factor and the done flag, which every kernel of an iteration checks first.
@@ -372,19 +364,34 @@ struct BteCtl {
 };
 struct BteDev {
     int32_t n_irr, n_mode, n_row, maxiter;
+    int32_t split;                    // partial sums per row and direction in part
     double tol, sqtol;
+    const double *part;               // [n_row][split][3] partial products of Xi and fbb
     const int32_t *rowidx;            // [n_irr*n] row of (q1, b1), -1 without one
     const double *qs;                 // [n_irr*n]
     const double *F0;                 // [n_irr*n*3]
     const int32_t *degen;             // [n_irr*n] degenerate-subspace sizes at the irreducible points
     const int32_t *degen_mode;        // [n_irr*n*n] its modes, 1-based
-    double *fn, *fnb;                 // [n_irr*n*3] current F and the new one
+    const int32_t *chain;             // [n_irr*n] bte_chains()
+    const int32_t *star_ptr;          // [n_irr+1] first point of each irreducible point's star
+    const int32_t *star;              // [n_full] the stars' points
+    const int32_t *full_op;           // [n_full] signed 1-based operation from the irreducible point
+    const double *op_cart;            // [n_op*9]
+    double *fn;                       // [n_irr*n*3] F
+    float2 *fbb;                      // [n_full*n*3] F on the full mesh as (hi, lo) float pairs
     double *scf;                      // [maxiter] relative changes
-    double *part;                     // [bte_part_elems(n_irr)] partial sums of the change
+    double *change;                   // [n_irr] change of each irreducible point
+    int32_t *arrived;                 // CTAs of the running update that are done (0 between kernels)
     BteCtl *ctl;
 };
-cudaError_t launch_bte_update(const BteDev &d, const double *buf, cudaStream_t s);
-int bte_part_elems(int32_t n_irr);
+// Order of distributeF within each irreducible point: chain[q1*n + b] = 1 + the next mode, in
+// ascending order, whose degenerate sets meet those of b, directly or through others
+// (0: none), plus kChainFirst where b is the lowest of them.
+constexpr int32_t kChainFirst = 1 << 30;
+void bte_chains(int n_irr, int n_mode, const int32_t *degen, const int32_t *degen_mode, int32_t *chain);
+// fbb = foldout of fn; then, per iteration after the products, the rest of it (k_bte.cu).
+cudaError_t launch_bte_foldout(const BteDev &d, cudaStream_t s);
+cudaError_t launch_bte_update(const BteDev &d, cudaStream_t s);
 
 // What an entry point compiled outside the context's own file needs of a context.
 // Off-diagonal kappa (k_offdiag.cu). Index tables 0-based.
