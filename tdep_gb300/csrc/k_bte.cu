@@ -1,7 +1,10 @@
-// The iterative BTE (kappa.f90:326-495) around its products with Xi: one kernel per iteration
-// for the scalar recurrences and the foldout of the new F onto the full mesh.
+// The iterative BTE (kappa.f90:326-495): three kernels per iteration, the sums of F over the
+// orbits (k_bte_sums), the products Xi F (k_bte_products) and the scalar recurrences with the
+// foldout of the new F onto the full mesh (k_bte_update).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <map>
 #include <vector>
 
 #include "dev_common.cuh"
@@ -10,6 +13,247 @@
 namespace tdg {
 
 namespace {
+
+// Two double-float accumulators (s, sl: high and low parts, one per column of a pair) +=
+// x * f for the columns' elements (x, xl) and F values (f, fl); nx = -x. The scalar form per component: p = x f, pe = fma(x, f, -p), cross = fma(x, fl,
+// xl f), TwoSum of s and p, sl += (e + pe) + cross. A subtraction a - b is fma(b, -1, a),
+// rounded once as a - b is.
+__device__ __forceinline__ void df2_fma(float2 &s, float2 &sl, float2 x, float2 nx, float2 xl, float2 f, float2 fl) {
+    const float2 m1 = make_float2(-1.f, -1.f);
+    const float2 p = __fmul2_rn(x, f);
+    const float2 npe = __ffma2_rn(nx, f, p);  // p - x f = -pe exactly
+    const float2 cross = __ffma2_rn(x, fl, __fmul2_rn(xl, f));
+    const float2 t = __fadd2_rn(s, p);
+    const float2 bb = __ffma2_rn(s, m1, t);                        // t - s
+    const float2 e1 = __ffma2_rn(__ffma2_rn(bb, m1, t), m1, s);    // s - (t - bb)
+    const float2 e = __fadd2_rn(e1, __ffma2_rn(bb, m1, p));       // + (p - bb)
+    s = t;
+    sl = __fadd2_rn(sl, __fadd2_rn(__ffma2_rn(npe, m1, e), cross));  // sl + ((e + pe) + cross)
+}
+
+// Three dot products per row of Xi (kappa.f90:411-413, the lo_gemv calls) over orbits.
+// symmetrize_scatmat leaves the entries of a row equal on every orbit of the little group of
+// its q1, so Xi F = sum over orbits and modes of Xi(orbit, b2) times the sum of F over the
+// orbit's points: of Xi only the representatives' columns are kept (k_bte_compact), N/48 of
+// N in all for a cubic crystal against the n_irr of the rows (0.52 of Xi at 16^3, 0.70 at
+// 24^3). Points with the same little group have the same orbits: their rows are laid out
+// together, and F is summed over the orbits once per group and iteration (k_bte_sums; some
+// 20 groups at 24^3, 14 MB), not by every CTA of the products: that cost as much as the
+// products, and 3 us of latency per chunk.
+//   Format. GB300's FP64 pipe (2 FMA per SM and clock) would bound an FP64 product with
+// three right-hand sides at ~1.2 TB/s of Xi, so it runs on the FP32 pipe: Xi and F as
+// (hi, lo) float pairs with hi + lo = x to ~2^-48, each term accumulated in double-float
+// (exact leading product by FMA, cross terms, TwoSum of the high parts); ~1e-14 relative,
+// the bytes of FP64. Two neighbouring columns of a row are one float4 (hi of both, lo of
+// both), so the arithmetic of the two runs in the packed FP32x2 instructions (__ffma2_rn,
+// __fadd2_rn, __fmul2_rn: per component the scalar IEEE operation). Floats for Xi (half the
+// bytes) fail the convergence test: the modes whose F is zero by symmetry (v = 0 at a
+// high-symmetry point) carry 1e-7 of the typical |F| from the rounding of Xi, above the
+// test's lo_sqtol floor, and rocksalt took 200 iterations, the limit, instead of 31-33.
+//   Shape. The work is dealt out in equal parts to two CTAs per SM (bte_plan): a CTA has a few
+// items, ranges of column pairs of up to kBteRows rows, and walks each in chunks of kBtePairs
+// pairs. Its G x S warps take three rows and a share of the pairs each, Xi through a ring of
+// kBteDepth steps that every lane fills for itself (cp.async, no barrier), the F sums from
+// shared memory (two buffers, one barrier per chunk). The partial sums of an item stay in
+// registers to its end and go to part[row][range][3] (FP64), added in range order by
+// k_bte_update, so the result does not depend on scheduling.
+//   Bound: HBM when Xi exceeds L2. Rocksalt 24^3: 1.15 GB in 217 us (5.3 TB/s, 0.79 of the
+// measured copy rate) against 330 us for the whole of Xi, four or eight rows to a CTA;
+// perovskite 16^3 96 us against 182; 40-atom supercell, no symmetry, 61 us against 72.
+constexpr int kBteRows = 30;
+constexpr int kBteThreads = 320;
+constexpr int kBtePairs = 256;
+constexpr int kBteDepth = 4;  // 10 warps x 4 steps x 1.5 KB and 24 KB of F sums: two CTAs per SM
+constexpr size_t kBteSmem = sizeof(float4) * (2 * 3 * kBtePairs + kBteThreads * 3 * kBteDepth);
+
+__device__ __forceinline__ void copy16(void *dst, const void *src, bool on) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+
+// Shares of the columns for G row groups of three: G S <= 10 warps, and kBteDepth steps of 32 S
+// pairs divide a chunk.
+__host__ __device__ constexpr int bte_share(int G) { return G <= 5 ? 2 : 1; }
+
+__device__ __forceinline__ void products_item(const BteDev &d, const BteItem &it, const float4 *__restrict__ xi,
+                                              float4 *smem) {
+    const int n = d.n_mode, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int G = (it.n_row + 2) / 3, S = bte_share(G);
+    const int g = w % G, s = w / G;
+    float2 ah[3][3], al[3][3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int x = 0; x < 3; ++x) ah[i][x] = al[i][x] = make_float2(0.f, 0.f);
+    // F sums of the chunk from pair p on, with the thread's next group of copies
+    auto fetch = [&](int p, float4 *buf) {
+        for (int c = tid; c < 3 * kBtePairs; c += kBteThreads) {
+            const int x = c / kBtePairs, pp = p + (c & (kBtePairs - 1));
+            copy16(buf + c, d.fsum + it.fsum + (int64_t)x * it.n_pair + min(pp, it.n_pair - 1), pp < it.n_pair);
+        }
+    };
+    // this warp's rows (the last one again past the item's); a lane's copies land in and are
+    // read from its own places of the ring
+    const float4 *xr[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) xr[i] = xi + it.xi + (int64_t)min(3 * g + i, it.n_row - 1) * it.n_pair;
+    float4 *ring = smem + 2 * 3 * kBtePairs + w * (32 * 3 * kBteDepth) + lane;
+    const bool work = s < S;
+    int pc = it.p0 + s * 32 + lane;  // the pair to copy next
+    auto copy = [&](int slot) {
+        const bool on = work && pc < it.p1;
+        const int at = min(pc, it.p1 - 1);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) copy16(ring + (slot * 3 + i) * 32, xr[i] + at, on);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        pc += 32 * S;
+    };
+    fetch(it.p0, smem);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int k = 0; k < kBteDepth - 1; ++k) copy(k);
+    int cur = 0;
+    for (int p = it.p0; p < it.p1; p += kBtePairs, cur ^= 1) {
+        // the chunk's F sums are in the oldest group but the ring's last kBteDepth - 1 (a chunk
+        // has at least kBteDepth steps; warps without rows have no ring)
+        if (work)
+            asm volatile("cp.async.wait_group %0;" ::"n"(kBteDepth - 1) : "memory");
+        else
+            asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();  // this chunk's sums are complete, the other buffer no longer read
+        if (p + kBtePairs < it.p1) fetch(p + kBtePairs, smem + (cur ^ 1) * (3 * kBtePairs));
+        if (work) {
+            const float4 *fp = smem + cur * (3 * kBtePairs) + s * 32 + lane;
+            for (int q = 0; q < kBtePairs && p + q < it.p1; q += 32 * kBteDepth * S) {
+#pragma unroll
+                for (int k = 0; k < kBteDepth; ++k) {
+                    asm volatile("cp.async.wait_group %0;" ::"n"(kBteDepth - 2) : "memory");
+                    float4 v[3];
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) v[i] = ring[(k * 3 + i) * 32];
+                    copy((k + kBteDepth - 1) % kBteDepth);
+#pragma unroll
+                    for (int x = 0; x < 3; ++x) {
+                        const float4 f = fp[x * kBtePairs];
+                        const float2 fh = make_float2(f.x, f.y), fl = make_float2(f.z, f.w);
+#pragma unroll
+                        for (int i = 0; i < 3; ++i)
+                            df2_fma(ah[i][x], al[i][x], make_float2(v[i].x, v[i].y), make_float2(-v[i].x, -v[i].y),
+                                    make_float2(v[i].z, v[i].w), fh, fl);
+                    }
+                    fp += 32 * S;
+                }
+            }
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    float2 *sh = reinterpret_cast<float2 *>(smem);  // [3 rows][S]
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            float2 a = df_merge(make_float2(ah[i][x].x, al[i][x].x), make_float2(ah[i][x].y, al[i][x].y));
+            for (int o = 16; o > 0; o >>= 1) {
+                float2 b;
+                b.x = __shfl_xor_sync(0xffffffffu, a.x, o);
+                b.y = __shfl_xor_sync(0xffffffffu, a.y, o);
+                a = df_merge(a, b);
+            }
+            if (lane == 0 && s < S) sh[((3 * g + i) * 3 + x) * S + s] = a;
+        }
+    __syncthreads();
+    if (tid < 3 * it.n_row) {
+        float2 a = sh[tid * S];
+        for (int k = 1; k < S; ++k) a = df_merge(a, sh[tid * S + k]);
+        const int row = d.rows_by_group[it.row + tid / 3];
+        d.part[((int64_t)row * d.split + it.range) * 3 + tid % 3] = (double)a.x + (double)a.y;
+    }
+}
+
+__global__ void __launch_bounds__(kBteThreads, 2) k_bte_products(BteDev d, const BteItem *items, const int32_t *first,
+                                                                 const float4 *__restrict__ xi) {
+    extern __shared__ float4 smem[];  // F sums of a chunk's column pairs per direction, twice; the ring
+    if (d.ctl->done) return;
+    for (int k = first[blockIdx.x]; k < first[blockIdx.x + 1]; ++k) {
+        __syncthreads();  // the previous item's sums are no longer read
+        products_item(d, items[k], xi, smem);
+    }
+}
+
+// The representatives' columns of Xi as double-float column pairs: pair p of a row holds
+// columns 2p and 2p + 1 of its (orbit, mode) list as (hi, hi, lo, lo); an odd last column
+// pairs with zero.
+__global__ void k_bte_compact(int n, int64_t ld, int n_row, const BteRow *rows, const int32_t *rep, const double *xi,
+                              float4 *out) {
+    for (int r = blockIdx.y; r < n_row; r += gridDim.y) {
+        const BteRow q = rows[r];
+        const double *xr = xi + (int64_t)r * ld;
+        float4 *o = out + q.xi;
+        for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < q.n_pair; p += gridDim.x * blockDim.x) {
+            float2 v[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int col = 2 * p + u, k = col / n;
+                v[u] = col < q.n_col ? split_df(__ldcs(xr + (int64_t)rep[q.rep0 + k] * n + (col - k * n)))
+                                     : make_float2(0.f, 0.f);
+            }
+            o[p] = make_float4(v[0].x, v[1].x, v[0].y, v[1].y);
+        }
+    }
+}
+
+// Points of every orbit of the groups, one orbit after another: orbit i of group g starts at
+// img_off[orb0 + i] (off: exclusive scan of the points per orbit over all q1; a q1's orbits
+// cover the mesh once).
+__global__ void k_bte_images(int n_full, int n_op, const BteGroup *grp, const int32_t *nuniq, const int32_t *img,
+                             const int32_t *off, int32_t *img_off, int32_t *out) {
+    const BteGroup g = grp[blockIdx.y];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= g.n_orb) return;
+    const int k = g.rep0 + i;
+    const int32_t *im = img + (size_t)k * n_op;
+    const int at = off[k] - off[g.rep0] + (int)blockIdx.y * n_full;
+    img_off[g.orb0 + i] = at;
+    if (i == g.n_orb - 1) img_off[g.orb0 + i + 1] = at + nuniq[k];
+    for (int u = 0; u < nuniq[k]; ++u) out[at + u] = im[u];
+}
+
+// F summed over the orbits of every group, as the products read it: [direction][column pair] of
+// (hi, hi, lo, lo). `lanes` consecutive threads share a column's points (a sixth of the
+// group's operations or so each: the chain of loads is what the kernel waits for).
+__global__ void __launch_bounds__(256) k_bte_sums(BteDev d, const BteGroup *grp) {
+    if (d.ctl->done) return;
+    const BteGroup g = grp[blockIdx.y];
+    const int n = d.n_mode, t = blockIdx.x * 256 + threadIdx.x;
+    const int col = t / g.lanes, part = t - col * g.lanes, n_pair = (g.n_orb * n + 1) / 2;
+    if ((blockIdx.x * 256) / g.lanes >= 2 * n_pair) return;
+    float2 a[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    if (col < g.n_orb * n) {
+        const int o = col / n, b = col - o * n;
+        const int i1 = d.img_off[g.orb0 + o + 1];
+#pragma unroll 4
+        for (int i = d.img_off[g.orb0 + o] + part; i < i1; i += g.lanes) {
+            const float2 *f = d.fbb + (d.img[i] * n + b) * (int64_t)3;
+#pragma unroll
+            for (int x = 0; x < 3; ++x) a[x] = df_merge(a[x], f[x]);
+        }
+    }
+    for (int o = 1; o < g.lanes; o <<= 1)
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            float2 v;
+            v.x = __shfl_xor_sync(0xffffffffu, a[x].x, o);
+            v.y = __shfl_xor_sync(0xffffffffu, a[x].y, o);
+            a[x] = df_merge(a[x], v);
+        }
+    if (part != 0 || col >= 2 * n_pair) return;
+    float *out = reinterpret_cast<float *>(d.fsum + g.fsum + (col >> 1)) + (col & 1);
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        out[(int64_t)4 * x * n_pair] = a[x].x;
+        out[(int64_t)4 * x * n_pair + 2] = a[x].y;
+    }
+}
 
 // foldout (kappa.f90:382-404): F of every point of the star of q1 from its irreducible point,
 // Fbb(q, b) = sign(op) * R_|op| Fn(irr(q), b), one (point, mode) per thread and trip.
@@ -63,7 +307,7 @@ __global__ void k_bte_update(BteDev d) {
         double v = 0.0;
         if (r >= 0 && !(q < kFreqTolD)) {
             const double *p = d.part + (int64_t)r * d.split * 3 + x;
-            for (int c = 0; c < d.split; ++c) v += p[c * 3];
+            for (int c = 0; c < d.ranges[r]; ++c) v += p[c * 3];
             v = -v / q;
         }
         fb[i] = v;
@@ -155,6 +399,129 @@ void bte_chains(int n_irr, int n_mode, const int32_t *degen, const int32_t *dege
             t = b;
         }
     }
+}
+
+BtePlan bte_plan(int n, int n_irr, int n_sm, const int32_t *rep_ptr, const int32_t *row_count, int n_op,
+                 const int32_t *irr_nop, const int32_t *irr_ops) {
+    BtePlan pl;
+    std::map<std::vector<int32_t>, int> ids;  // little group (its operations) -> group
+    std::vector<std::vector<int32_t>> rows;   // rows of each group
+    int row = 0;
+    for (int q = 0; q < n_irr; ++q) {
+        std::vector<int32_t> key(irr_ops + (size_t)q * n_op, irr_ops + (size_t)q * n_op + irr_nop[q]);
+        std::sort(key.begin(), key.end());
+        const auto at = ids.emplace(std::move(key), (int)pl.groups.size());
+        if (at.second) {
+            BteGroup g;
+            g.rep0 = rep_ptr[q];
+            g.n_orb = rep_ptr[q + 1] - rep_ptr[q];
+            g.orb0 = pl.n_orb;
+            g.fsum = pl.n_fsum;
+            pl.n_fsum += 3 * (((int64_t)g.n_orb * n + 1) / 2);
+            for (g.lanes = 1; g.lanes < 8 && 6 * g.lanes < irr_nop[q]; g.lanes *= 2) {}
+            pl.sum_threads = std::max(pl.sum_threads, ((int64_t)g.n_orb * n + 1) * g.lanes);
+            pl.n_orb += g.n_orb + 1;
+            pl.max_orb = std::max(pl.max_orb, g.n_orb);
+            pl.groups.push_back(g);
+            rows.emplace_back();
+        }
+        for (int k = 0; k < row_count[q]; ++k) rows[at.first->second].push_back(row++);
+    }
+    // Equal shares of a group's rows, in multiples of three.
+    auto share = [](int count) {
+        const int k = (count + kBteRows - 1) / kBteRows;
+        return ((count + k - 1) / k + 2) / 3 * 3;
+    };
+    // The row blocks one after another, each a number of units of columns (the steps between two
+    // turns of the ring), cut into equal parts for two CTAs per SM: a CTA's fill and drain, some
+    // 4 us, then come once or twice per iteration.
+    const auto unit_of = [](int h) { return 32 * kBteDepth * bte_share((h + 2) / 3); };
+    int64_t units = 0;
+    for (size_t g = 0; g < rows.size(); ++g) {
+        const int count = (int)rows[g].size();
+        const int64_t pairs = ((int64_t)pl.groups[g].n_orb * n + 1) / 2;
+        if (count == 0) continue;
+        const int h = share(count);
+        for (int k0 = 0; k0 < count; k0 += h) {
+            const int u = unit_of(std::min(h, count - k0));
+            units += (pairs + u - 1) / u;
+        }
+    }
+    const int64_t parts = std::max<int64_t>(1, std::min<int64_t>(units, 2 * (int64_t)n_sm));
+    int64_t done = 0;  // units dealt out
+    pl.first.push_back(0);
+    pl.rows.resize(row);
+    pl.ranges.assign(row, 0);
+    for (size_t g = 0; g < rows.size(); ++g) {
+        const BteGroup &gr = pl.groups[g];
+        const int count = (int)rows[g].size(), h = count ? share(count) : 3;
+        const int32_t n_col = gr.n_orb * n, n_pair = (n_col + 1) / 2;
+        for (int k0 = 0; k0 < count; k0 += h) {
+            BteItem it;
+            it.xi = pl.n_xi + (int64_t)k0 * n_pair;
+            it.row = (int32_t)pl.by_group.size() + k0;
+            it.n_row = std::min(h, count - k0);
+            it.fsum = gr.fsum;
+            it.n_pair = n_pair;
+            it.range = 0;
+            const int unit = unit_of(it.n_row);
+            for (int64_t p = 0; p < n_pair; ++it.range) {
+                // to the end of the part in hand or of the block
+                const int64_t end = units * (int64_t)pl.first.size() / parts;
+                const int64_t take = std::min<int64_t>(end - done, (n_pair - p + unit - 1) / unit);
+                it.p0 = (int32_t)p;
+                p = std::min<int64_t>(n_pair, p + take * unit);
+                it.p1 = (int32_t)p;
+                done += take;
+                pl.items.push_back(it);
+                if (done == end) pl.first.push_back((int32_t)pl.items.size());
+            }
+            for (int k = k0; k < k0 + it.n_row; ++k) pl.ranges[rows[g][k]] = it.range;
+            pl.split = std::max(pl.split, it.range);
+        }
+        for (int k = 0; k < count; ++k) {
+            BteRow &r = pl.rows[rows[g][k]];
+            r.xi = pl.n_xi + (int64_t)k * n_pair;
+            r.rep0 = gr.rep0;
+            r.n_col = n_col;
+            r.n_pair = n_pair;
+        }
+        pl.by_group.insert(pl.by_group.end(), rows[g].begin(), rows[g].end());
+        pl.n_xi += (int64_t)count * n_pair;
+    }
+    return pl;
+}
+
+cudaError_t launch_bte_images(int n_full, int n_op, int n_group, int max_orb, const BteGroup *grp, const OrbitDev &o,
+                              const int32_t *off, int32_t *img_off, int32_t *img, cudaStream_t s) {
+    if (n_group <= 0 || max_orb <= 0) return cudaSuccess;
+    dim3 grid((unsigned)((max_orb + 127) / 128), (unsigned)n_group);
+    k_bte_images<<<grid, 128, 0, s>>>(n_full, n_op, grp, o.nuniq, o.img, off, img_off, img);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_bte_compact(int n, int64_t ld, int n_row, const BteRow *rows, const int32_t *rep, const double *xi,
+                               float4 *out, cudaStream_t s) {
+    if (n_row <= 0) return cudaSuccess;
+    const int64_t bx = (ld / 2 + 255) / 256;
+    dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(bx, 64)), (unsigned)std::min(n_row, 65535));
+    k_bte_compact<<<grid, 256, 0, s>>>(n, ld, n_row, rows, rep, xi, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_bte_products(const BteDev &d, const BteItem *items, const int32_t *first, int n_part, const float4 *xi,
+                                cudaStream_t s) {
+    if (n_part <= 0) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(k_bte_products, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBteSmem);
+    if (e != cudaSuccess) return e;
+    k_bte_products<<<n_part, kBteThreads, kBteSmem, s>>>(d, items, first, xi);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_bte_sums(const BteDev &d, const BteGroup *grp, int n_group, int64_t threads, cudaStream_t s) {
+    if (n_group <= 0 || threads <= 0) return cudaSuccess;
+    k_bte_sums<<<dim3((unsigned)((threads + 255) / 256), (unsigned)n_group), 256, 0, s>>>(d, grp);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_bte_foldout(const BteDev &d, cudaStream_t s) {

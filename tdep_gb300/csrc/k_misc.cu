@@ -1,4 +1,4 @@
-// Isotope scattering, the two scattering-matrix symmetrisations and the BTE product.
+// Isotope scattering and the two scattering-matrix symmetrisations.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -365,160 +365,6 @@ __global__ void k_sample_bits(int32_t n_full, const int64_t *rbeg, const int32_t
     for (int i = threadIdx.x; i < nw; i += blockDim.x) br[i] = sb[i];
 }
 
-// K8: three dot products per row of Xi (kappa.f90:411-413, the lo_gemv calls).
-// Xi streams from HBM once per BTE iteration; F (3 x n_col) stays in L2. GB300's FP64 pipe
-// (2 FMA per SM and clock) would make an FP64 product with three right-hand sides
-// compute-bound at ~1.2 TB/s of Xi, so the product runs on the FP32 pipe: Xi and F as
-// (hi, lo) float pairs with hi + lo = x to ~2^-48 (converted once per kappa call, k_split_xi,
-// and per iteration for F, k_foldout), each term accumulated in double-float (exact leading
-// product by FMA, cross terms, TwoSum of the high parts); ~1e-14 relative, the bytes of FP64.
-// The rows go in pairs: pair p and column j are one float4 (hi of rows 2p and 2p + 1, lo of
-// both), so that the double-float arithmetic of the two rows runs in the packed FP32x2
-// instructions (__ffma2_rn, __fadd2_rn, __fmul2_rn: per component the scalar IEEE operation),
-// half the instructions of the scalar form, which left the product issue-bound at 0.58 of
-// the copy peak.
-// Floats for Xi (half the bytes) were the mixed-precision format until they failed the
-// convergence test: the modes whose F is zero by symmetry (v = 0 at a high-symmetry point)
-// carry 1e-7 of the typical |F| from the rounding of Xi, above the test's lo_sqtol floor,
-// and their relative change kept the sum of the last three checks above 1e-6 (rocksalt took
-// 200 iterations, the limit, instead of 31-33, with kappa already converged).
-// A CTA takes PAIRS row pairs (2 or 4, autotuned) and one of the column ranges (gridDim.y):
-// each F value read from L2 serves 2 PAIRS rows. Partial sums go to part[row][range][3]
-// (FP64) and are added in range order by k_bte_update, so the result does not depend on
-// scheduling. The in-CTA reduction stays in double-float too: FP64 shuffles and adds in
-// every CTA's epilogue cost more than the product itself once there are more than a few
-// ranges.
-constexpr int kGemvRows = 4;
-constexpr int kGemvMaxSplit = 32;
-
-// Ranges of at most 32768 columns, and enough CTAs for about two waves of 4 per SM.
-int gemv_split(int32_t n_row, int64_t n_col, int n_sm) {
-    const int64_t groups = (n_row + kGemvRows - 1) / kGemvRows;
-    int64_t k = (n_col + 32767) / 32768;
-    const int64_t w = (8 * (int64_t)n_sm + groups - 1) / groups;
-    if (w > k) k = w;
-    if (k > n_col / 256) k = n_col / 256;
-    return (int)(k < 1 ? 1 : (k > kGemvMaxSplit ? kGemvMaxSplit : k));
-}
-
-// (a.x + a.y) + (b.x + b.y) in double-float (TwoSum of the high parts)
-__device__ __forceinline__ float2 df_add(float2 a, float2 b) {
-    const float t = a.x + b.x;
-    const float bb = t - a.x;
-    const float e = (a.x - (t - bb)) + (b.x - bb);
-    return make_float2(t, a.y + b.y + e);
-}
-
-// Two double-float accumulators (s, sl: high and low parts of rows 2p and 2p + 1) += x * f
-// for the two rows' elements (x, xl) and one F value (f, fl, the same in both components);
-// nx = -x. The scalar form per component: p = x f, pe = fma(x, f, -p), cross = fma(x, fl,
-// xl f), TwoSum of s and p, sl += (e + pe) + cross. A subtraction a - b is fma(b, -1, a),
-// rounded once as a - b is.
-__device__ __forceinline__ void df2_fma(float2 &s, float2 &sl, float2 x, float2 nx, float2 xl, float2 f, float2 fl) {
-    const float2 m1 = make_float2(-1.f, -1.f);
-    const float2 p = __fmul2_rn(x, f);
-    const float2 npe = __ffma2_rn(nx, f, p);  // p - x f = -pe exactly
-    const float2 cross = __ffma2_rn(x, fl, __fmul2_rn(xl, f));
-    const float2 t = __fadd2_rn(s, p);
-    const float2 bb = __ffma2_rn(s, m1, t);                        // t - s
-    const float2 e1 = __ffma2_rn(__ffma2_rn(bb, m1, t), m1, s);    // s - (t - bb)
-    const float2 e = __fadd2_rn(e1, __ffma2_rn(bb, m1, p));       // + (p - bb)
-    s = t;
-    sl = __fadd2_rn(sl, __fadd2_rn(__ffma2_rn(npe, m1, e), cross));  // sl + ((e + pe) + cross)
-}
-
-// Xi as double-float row pairs: pair p, column j at p * n_col + j as (hi of row 2p, hi of
-// row 2p + 1, lo of row 2p, lo of row 2p + 1); an odd last row pairs with a zero row.
-__global__ void k_split_xi(const double *xi, int32_t n_row, int64_t n_col, float4 *out) {
-    const int n_pair = (n_row + 1) / 2;
-    for (int p = blockIdx.y; p < n_pair; p += gridDim.y) {
-        const double *r0 = xi + (int64_t)(2 * p) * n_col;
-        const bool two = 2 * p + 1 < n_row;
-        for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n_col; j += (int64_t)gridDim.x * blockDim.x) {
-            const float2 a = split_df(__ldcs(r0 + j));
-            const float2 b = two ? split_df(__ldcs(r0 + n_col + j)) : make_float2(0.f, 0.f);
-            out[(int64_t)p * n_col + j] = make_float4(a.x, b.x, a.y, b.y);
-        }
-    }
-}
-
-template <int PAIRS>
-__global__ void __launch_bounds__(256) k_xi_gemv(const float4 *__restrict__ xi, int32_t n_row, int64_t n_col,
-                                                 const float2 *__restrict__ fbb, double *part, const int32_t *skip) {
-    __shared__ float2 sh[2 * PAIRS * 3][8];
-    if (skip && *skip) return;
-    const int p0 = blockIdx.x * PAIRS;
-    const int np = min(PAIRS, (n_row + 1) / 2 - p0);
-    const int r0 = 2 * p0, nr = min(2 * PAIRS, n_row - r0);
-    const int64_t per = ((n_col + gridDim.y - 1) / gridDim.y + 7) / 8 * 8;
-    const int64_t c0 = min(n_col, per * blockIdx.y), c1 = min(n_col, c0 + per);
-    float2 ah[PAIRS][3], al[PAIRS][3];
-#pragma unroll
-    for (int k = 0; k < PAIRS; ++k)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) ah[k][d] = al[k][d] = make_float2(0.f, 0.f);
-    const float4 *xr[PAIRS];
-#pragma unroll
-    for (int k = 0; k < PAIRS; ++k) xr[k] = xi + (int64_t)(p0 + min(k, np - 1)) * n_col;
-    const int64_t step = blockDim.x;
-    int64_t j = c0 + threadIdx.x;
-    auto column = [&](const float4 (&x)[PAIRS], int64_t jj) {
-        float2 fh[3], fl[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const float2 t = __ldg(fbb + jj * 3 + d);
-            fh[d] = make_float2(t.x, t.x);
-            fl[d] = make_float2(t.y, t.y);
-        }
-#pragma unroll
-        for (int k = 0; k < PAIRS; ++k) {
-            const float2 xh = make_float2(x[k].x, x[k].y), xl = make_float2(x[k].z, x[k].w);
-            const float2 nx = make_float2(-x[k].x, -x[k].y);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) df2_fma(ah[k][d], al[k][d], xh, nx, xl, fh[d], fl[d]);
-        }
-    };
-    // four columns per thread and trip: 4 PAIRS 16-byte loads in flight
-    for (; j + 3 * step < c1; j += 4 * step) {
-        float4 x[4][PAIRS];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int k = 0; k < PAIRS; ++k)
-                x[u][k] = k < np ? __ldcs(xr[k] + j + u * step) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) column(x[u], j + u * step);
-    }
-    for (; j < c1; j += step) {
-        float4 x[PAIRS];
-#pragma unroll
-        for (int k = 0; k < PAIRS; ++k) x[k] = k < np ? __ldcs(xr[k] + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-        column(x, j);
-    }
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < 2 * PAIRS; ++k)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const float2 hp = ah[k / 2][d], lp = al[k / 2][d];
-            float2 v = (k & 1) ? make_float2(hp.y, lp.y) : make_float2(hp.x, lp.x);
-            for (int o = 16; o > 0; o >>= 1) {
-                float2 u;
-                u.x = __shfl_down_sync(0xffffffffu, v.x, o);
-                u.y = __shfl_down_sync(0xffffffffu, v.y, o);
-                v = df_add(v, u);
-            }
-            if (lane == 0) sh[k * 3 + d][w] = v;
-        }
-    __syncthreads();
-    if (threadIdx.x < nr * 3) {
-        float2 v = sh[threadIdx.x][0];
-        for (int i = 1; i < 8; ++i) v = df_add(v, sh[threadIdx.x][i]);
-        const int k = threadIdx.x / 3, d = threadIdx.x % 3;
-        part[((int64_t)(r0 + k) * gridDim.y + blockIdx.y) * 3 + d] = (double)v.x + (double)v.y;
-    }
-}
-
 }  // namespace
 
 cudaError_t launch_iso_mag(int64_t ne, const double2 *egv, double *mag, cudaStream_t s) {
@@ -611,39 +457,6 @@ cudaError_t launch_sym_tile(const MeshDev &m, const OrbitDev &o, int32_t n_row, 
     }
     dim3 grid((unsigned)o.max_tiles, (unsigned)n_row);
     k_sym_tile<<<grid, 256, sm, s>>>(m, o, row_q1, xi, sbits, dist ? 1 : 0, scat ? 1 : 0);
-    return cudaGetLastError();
-}
-
-size_t xi_gemv_part_elems(int32_t n_row) { return (size_t)n_row * kGemvMaxSplit * 3; }
-
-size_t xi_pairs_elems(int32_t n_row, int64_t n_col) { return (size_t)((n_row + 1) / 2) * (size_t)n_col; }
-
-cudaError_t launch_split_xi(const double *xi, int32_t n_row, int64_t n_col, float4 *out, cudaStream_t s) {
-    if (n_row <= 0 || n_col <= 0) return cudaSuccess;
-    const int n_pair = (n_row + 1) / 2;
-    const int64_t bx = (n_col + 255) / 256;
-    dim3 grid((unsigned)(bx < 64 ? bx : 64), (unsigned)(n_pair < 65535 ? n_pair : 65535));
-    k_split_xi<<<grid, 256, 0, s>>>(xi, n_row, n_col, out);
-    return cudaGetLastError();
-}
-
-int xi_gemv_default_split(int32_t n_row, int64_t n_col, int n_sm) { return gemv_split(n_row, n_col, n_sm); }
-
-int xi_gemv_max_split(int64_t n_col) {
-    const int64_t k = n_col / 256;
-    return (int)(k < 1 ? 1 : (k > kGemvMaxSplit ? kGemvMaxSplit : k));
-}
-
-cudaError_t launch_xi_gemv(const float4 *xi, int32_t n_row, int64_t n_col, const float2 *fbb, double *part,
-                           cudaStream_t s, const int32_t *skip, int shape) {
-    if (n_row <= 0) return cudaSuccess;
-    // shape = rows per CTA (4 or 8) * 100 + column ranges
-    const int rows = shape / 100, split = shape % 100;
-    dim3 grid((unsigned)((n_row + rows - 1) / rows), (unsigned)split);
-    if (rows == 8)
-        k_xi_gemv<4><<<grid, 256, 0, s>>>(xi, n_row, n_col, fbb, part, skip);
-    else
-        k_xi_gemv<2><<<grid, 256, 0, s>>>(xi, n_row, n_col, fbb, part, skip);
     return cudaGetLastError();
 }
 

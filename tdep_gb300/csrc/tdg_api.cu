@@ -245,7 +245,16 @@ struct tdg_ctx {
     // BTE buffers
     DevBuf<double> d_part;
     DevBuf<float2> d_fbb;   // F as double-float pairs for the BTE product
-    DevBuf<float4> d_xi_df;  // Xi as double-float row pairs (launch_split_xi)
+    DevBuf<float4> d_xi_df;  // the representatives' columns of Xi as double-float pairs (launch_bte_compact)
+    // the products' division (bte_plan) and the points of every orbit, built by the first solve
+    int bte_parts = 0, bte_split = 0, bte_groups = 0;
+    int64_t bte_n_xi = 0, bte_sum_threads = 0;
+    DevBuf<BteGroup> d_bte_groups;
+    DevBuf<float4> d_fsum;
+    DevBuf<BteItem> d_bte_items;
+    DevBuf<BteRow> d_bte_rows;
+    DevBuf<int32_t> d_bte_first, d_bte_ranges, d_by_group, d_img_off, d_bte_img;
+    std::vector<int32_t> orb_rep_ptr;  // host copy of orbits.rep_ptr
     // state of the last tdg_scattering that the adjoint pass reuses
     PhononDev last_ph{};
     RowsDev last_rows{};
@@ -726,6 +735,7 @@ extern "C" int tdg_create(tdg_ctx **out, const tdg_problem *p, int device) {
             mx = std::max(mx, rp[q + 1] - rp[q]);
             mt = std::max(mt, sym_tile_count(rp[q + 1] - rp[q], c->irr_nop[q], c->n));
         }
+        c->orb_rep_ptr = rp;
         c->orbits.max_rep = mx;
         c->orbits.tile_pts = sym_tile_points(c->n);
         c->orbits.max_tiles = mt;
@@ -1838,14 +1848,40 @@ extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double 
         const int64_t ncol = (int64_t)N * n;
         const size_t nfn = (size_t)nirr * n * 3;
         CUDA_TRY(c->d_fbb.alloc((size_t)ncol * 3));
-        // the Xi.F products take Xi as double-float row pairs (k_xi_gemv; floats fail the
-        // mixed iteration's convergence test)
+        if (c->d_bte_items.n == 0) {
+            std::vector<int32_t> count(nirr, 0);
+            for (int r = 0; r < nr; ++r) ++count[c->row_q1[r] - 1];
+            const BtePlan pl = bte_plan(n, nirr, c->n_sm, c->orb_rep_ptr.data(), count.data(), c->nop,
+                                        c->irr_nop.data(), c->irr_ops.data());
+            const int32_t nrep = c->orb_rep_ptr[nirr], ng = (int32_t)pl.groups.size();
+            DevBuf<int32_t> off, tmp;
+            CUDA_TRY(off.alloc((size_t)nrep + 1));
+            CUDA_TRY(tmp.alloc(exclusive_scan_tmp_elems(nrep)));
+            CUDA_TRY(c->d_bte_groups.upload(pl.groups.data(), pl.groups.size(), s));
+            CUDA_TRY(c->d_img_off.alloc((size_t)pl.n_orb));
+            CUDA_TRY(c->d_bte_img.alloc((size_t)ng * N));
+            CUDA_TRY(exclusive_scan_i32(c->orbits.nuniq, off.p, nrep, tmp.p, s));
+            CUDA_TRY(launch_bte_images(N, c->nop, ng, pl.max_orb, c->d_bte_groups.p, c->orbits, off.p, c->d_img_off.p,
+                                       c->d_bte_img.p, s));
+            CUDA_TRY(c->d_bte_rows.upload(pl.rows.data(), pl.rows.size(), s));
+            CUDA_TRY(c->d_bte_ranges.upload(pl.ranges.data(), pl.ranges.size(), s));
+            CUDA_TRY(c->d_by_group.upload(pl.by_group.data(), pl.by_group.size(), s));
+            c->bte_parts = (int)pl.first.size() - 1;
+            CUDA_TRY(c->d_bte_first.upload(pl.first.data(), pl.first.size(), s));
+            c->bte_split = pl.split;
+            c->bte_groups = ng;
+            c->bte_sum_threads = pl.sum_threads;
+            CUDA_TRY(c->d_fsum.alloc((size_t)pl.n_fsum));
+            c->bte_n_xi = pl.n_xi;
+            CUDA_TRY(c->d_bte_items.upload(pl.items.data(), pl.items.size(), s));
+        }
+        // the products take the representatives' columns of Xi as double-float pairs
         if (c->xi_fmt != 1) {
-            CUDA_TRY(c->d_xi_df.alloc(xi_pairs_elems(nr, ncol)));
-            CUDA_TRY(launch_split_xi(c->d_xi.p, nr, ncol, c->d_xi_df.p, s));
+            CUDA_TRY(c->d_xi_df.alloc((size_t)c->bte_n_xi));
+            CUDA_TRY(launch_bte_compact(n, ncol, nr, c->d_bte_rows.p, c->orbits.rep, c->d_xi.p, c->d_xi_df.p, s));
             c->xi_fmt = 1;
         }
-        CUDA_TRY(c->d_part.alloc(xi_gemv_part_elems(nr)));
+        CUDA_TRY(c->d_part.alloc((size_t)nr * c->bte_split * 3));
         CUDA_TRY(c->d_fn.alloc(nfn));
         if (c->d_full_op.n == 0) {
             CUDA_TRY(c->d_full_op.upload(c->full_op.data(), N, s));
@@ -1895,7 +1931,12 @@ extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double 
         bd.maxiter = maxiter;
         bd.tol = tol;
         bd.sqtol = kSqTol;
+        bd.split = c->bte_split;
         bd.part = c->d_part.p;
+        bd.ranges = c->d_bte_ranges.p;
+        bd.rows_by_group = c->d_by_group.p;
+        bd.img_off = c->d_img_off.p;
+        bd.img = c->d_bte_img.p;
         bd.rowidx = c->d_rowidx.p;
         bd.qs = c->d_qs_bte.p;
         bd.F0 = c->d_F0.p;
@@ -1908,38 +1949,17 @@ extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double 
         bd.op_cart = c->d_op_cart.p;
         bd.fn = c->d_fn.p;
         bd.fbb = c->d_fbb.p;
+        bd.fsum = c->d_fsum.p;
         bd.scf = c->d_scf.p;
         bd.change = c->d_bte_change.p;
         bd.arrived = c->d_arrived.p;
         bd.ctl = c->d_ctl.p;
-        const int32_t *done = &c->d_ctl.p->done;
-        // column split of the Xi products, autotuned per problem size on F0's foldout
-        int split = 0;
         CUDA_TRY(launch_bte_foldout(bd, s));
-        {
-            // shapes: rows per CTA (4, 8) * 100 + column ranges (the default, twice it)
-            const int s0 = xi_gemv_default_split(nr, ncol, c->n_sm), smax = xi_gemv_max_split(ncol);
-            std::vector<int> cand;
-            for (int rows : {4, 8})
-                for (int v : {s0, 2 * s0})
-                    if (v <= smax && std::find(cand.begin(), cand.end(), rows * 100 + v) == cand.end())
-                        cand.push_back(rows * 100 + v);
-            std::ostringstream key;
-            key << "xigemv2/r" << nr << "/c" << ncol;
-            bool tuned = false;
-            CUDA_TRY(tune_pick(tune_key(key.str().c_str(), n, 0, c->device), cand, 400 + s0,
-                               [&](int v) {
-                                   return launch_xi_gemv(c->d_xi_df.p, nr, ncol, c->d_fbb.p, c->d_part.p, s,
-                                                         nullptr, v);
-                               },
-                               s, split, tuned));
-        }
-        // a decision read from a file may be any number
-        bd.split = std::min(std::max(split % 100, 1), xi_gemv_max_split(ncol));
-        split = (split / 100 == 8 ? 800 : 400) + bd.split;
         auto iterations = [&](int k) -> cudaError_t {
             for (int j = 0; j < k; ++j) {
-                cudaError_t e = launch_xi_gemv(c->d_xi_df.p, nr, ncol, c->d_fbb.p, c->d_part.p, s, done, split);
+                cudaError_t e = launch_bte_sums(bd, c->d_bte_groups.p, c->bte_groups, c->bte_sum_threads, s);
+                if (e == cudaSuccess)
+                    e = launch_bte_products(bd, c->d_bte_items.p, c->d_bte_first.p, c->bte_parts, c->d_xi_df.p, s);
                 if (e == cudaSuccess) e = launch_bte_update(bd, s);
                 if (e != cudaSuccess) return e;
             }
@@ -1950,9 +1970,9 @@ extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double 
         for (int it0 = 0; it0 < maxiter; it0 += kBteChunk) {
             const int k = std::min(kBteChunk, maxiter - it0);
             std::ostringstream key;
-            key << k << '/' << split << '/' << std::string(reinterpret_cast<const char *>(&bd), sizeof bd)
+            key << k << '/' << std::string(reinterpret_cast<const char *>(&bd), sizeof bd)
                 << '/'
-                << (const void *)c->d_xi_df.p << ncol;
+                << (const void *)c->d_xi_df.p;
             // recorded only from the context's second kappa call on: a context that solves
             // once would pay for the recording without replaying it much
             CUDA_TRY(run_graph_region(c, c->graph_bte, key.str(), s, [&]() { return iterations(k); },

@@ -338,19 +338,6 @@ cudaError_t launch_sym_tile(const MeshDev &m, const OrbitDev &o, int32_t n_row, 
 // cotangent w in place, the distribution's active entries given by the raw terms od_raw.
 cudaError_t launch_sym_tile_adjoint(const MeshDev &m, const OrbitDev &o, int32_t n_row, const int32_t *row_q1,
                                     const double *od_raw, double *w, const uint32_t *sbits, cudaStream_t s);
-// K8: buf[r*3+a] = sum_j xi[r, j] * fbb[j*3 + a] on the FP32 pipe, xi and fbb as (hi, lo)
-// float pairs accumulated in double-float. launch_split_xi converts the FP64 Xi into row
-// pairs (xi_pairs_elems(n_row, n_col) float4: hi of rows 2p and 2p + 1, lo of both); part:
-// xi_gemv_part_elems(n_row) doubles.
-size_t xi_pairs_elems(int32_t n_row, int64_t n_col);
-cudaError_t launch_split_xi(const double *xi, int32_t n_row, int64_t n_col, float4 *out, cudaStream_t s);
-size_t xi_gemv_part_elems(int32_t n_row);
-// shape: rows per CTA (4 or 8) * 100 + column ranges per row group.
-cudaError_t launch_xi_gemv(const float4 *xi, int32_t n_row, int64_t n_col, const float2 *fbb, double *part,
-                           cudaStream_t s, const int32_t *skip, int shape);
-int xi_gemv_default_split(int32_t n_row, int64_t n_col, int n_sm);
-int xi_gemv_max_split(int64_t n_col);
-
 // One-tile tcgen05 self-check: d (128 x n) = a (128 x 16) b (16 x n) through BF16 hi/lo
 // splits; variant selects the operand layout reading (diagnostic).
 cudaError_t launch_mma_check(int variant, int n, const float *a, const float *b, float *d, int *status,
@@ -362,11 +349,53 @@ struct BteCtl {
     int32_t done, iter;
     double mixing;
 };
+// Irreducible points with one little group: its orbits in the orbit table (n_orb from rep0),
+// the first of their offsets into the points' list, its F sums (float4 index) and the threads
+// that share a column's points.
+struct BteGroup {
+    int64_t fsum;
+    int32_t rep0, n_orb, orb0, lanes;
+};
+// A row in the compacted Xi: its first float4, representatives, columns (representatives x
+// modes) and float4.
+struct BteRow {
+    int64_t xi;
+    int32_t rep0, n_col, n_pair;
+};
+// Work item of the products: n_row rows from by_group[row] on (xi: float4 index of the first),
+// column pairs [p0, p1) of n_pair, the group's F sums, the range's number.
+struct BteItem {
+    int64_t xi, fsum;
+    int32_t row, n_row, n_pair, p0, p1, range;
+};
+// The products' division, fixed by the crystal, the mesh and the rows: groups, rows in group
+// order, items and the first of each CTA (and their end), ranges per row and the most of
+// them, float4 of the compacted Xi and of the F sums, most threads of a group's sums.
+struct BtePlan {
+    std::vector<BteGroup> groups;
+    std::vector<BteRow> rows;
+    std::vector<int32_t> by_group, ranges, first;
+    std::vector<BteItem> items;
+    int32_t split = 1, n_orb = 0, max_orb = 0;
+    int64_t n_xi = 0, n_fsum = 0, sum_threads = 0;
+};
+BtePlan bte_plan(int n, int n_irr, int n_sm, const int32_t *rep_ptr, const int32_t *row_count, int n_op,
+                 const int32_t *irr_nop, const int32_t *irr_ops);
+// Points of every orbit of the groups (off: exclusive scan of o.nuniq over all q1).
+struct OrbitDev;
+cudaError_t launch_bte_images(int n_full, int n_op, int n_group, int max_orb, const BteGroup *grp, const OrbitDev &o,
+                              const int32_t *off, int32_t *img_off, int32_t *img, cudaStream_t s);
+// The representatives' columns of the symmetrised Xi as double-float column pairs.
+cudaError_t launch_bte_compact(int n, int64_t ld, int n_row, const BteRow *rows, const int32_t *rep, const double *xi,
+                               float4 *out, cudaStream_t s);
 struct BteDev {
     int32_t n_irr, n_mode, n_row, maxiter;
     int32_t split;                    // partial sums per row and direction in part
     double tol, sqtol;
-    const double *part;               // [n_row][split][3] partial products of Xi and fbb
+    double *part;                     // [n_row][split][3] partial products of Xi and fbb
+    const int32_t *ranges;            // [n_row] partial sums of the row
+    const int32_t *rows_by_group;     // [n_row] BtePlan::by_group
+    const int32_t *img_off, *img;     // points of every orbit (launch_bte_images)
     const int32_t *rowidx;            // [n_irr*n] row of (q1, b1), -1 without one
     const double *qs;                 // [n_irr*n]
     const double *F0;                 // [n_irr*n*3]
@@ -379,6 +408,7 @@ struct BteDev {
     const double *op_cart;            // [n_op*9]
     double *fn;                       // [n_irr*n*3] F
     float2 *fbb;                      // [n_full*n*3] F on the full mesh as (hi, lo) float pairs
+    float4 *fsum;                     // its sums over the orbits of every group (launch_bte_sums)
     double *scf;                      // [maxiter] relative changes
     double *change;                   // [n_irr] change of each irreducible point
     int32_t *arrived;                 // CTAs of the running update that are done (0 between kernels)
@@ -389,6 +419,11 @@ struct BteDev {
 // (0: none), plus kChainFirst where b is the lowest of them.
 constexpr int32_t kChainFirst = 1 << 30;
 void bte_chains(int n_irr, int n_mode, const int32_t *degen, const int32_t *degen_mode, int32_t *chain);
+// fsum = fbb summed over the orbits of every group.
+cudaError_t launch_bte_sums(const BteDev &d, const BteGroup *grp, int n_group, int64_t threads, cudaStream_t s);
+// part = products of the compacted Xi (items and parts of bte_plan) and fsum.
+cudaError_t launch_bte_products(const BteDev &d, const BteItem *items, const int32_t *first, int n_part, const float4 *xi,
+                                cudaStream_t s);
 // fbb = foldout of fn; then, per iteration after the products, the rest of it (k_bte.cu).
 cudaError_t launch_bte_foldout(const BteDev &d, cudaStream_t s);
 cudaError_t launch_bte_update(const BteDev &d, cudaStream_t s);

@@ -1,6 +1,6 @@
 """Iterative BTE on the device against the oracle where its kernels can go wrong: degenerate
 sets of one to three modes, sets that overlap without being equal (each mode's set is the
-caller's), fewer modes than a warp and more than one, meshes of one and of many points."""
+caller's), fewer modes than a warp and more than one."""
 import numpy as np
 import pytest
 
@@ -20,15 +20,20 @@ def _overlapping(prob):
     prob.degen, prob.degen_mode = dg, dm
 
 
-# (cell, mesh, overlapping sets): 3, 6, 15 and 30 modes
-@pytest.mark.parametrize("name,mesh,overlap", [("fcc", 5, False), ("fcc", 6, True), ("rocksalt", 6, False),
-                                               ("rocksalt", 5, True), ("perovskite", 4, False),
-                                               ("perovskite", 4, True)])
+# 3 to 30 modes; meshes on which operations of a point's little group leave the mesh (unequal
+# dimensions); the identity alone and rows in two items (30 modes); columns of one
+# and of many chunks, even and odd in number
+@pytest.mark.parametrize("name,mesh,overlap", [
+    ("fcc", (5, 5, 5), False), ("fcc", (6, 6, 6), True), ("fcc", (3, 4, 5), False), ("fcc", (16, 16, 16), False),
+    ("rocksalt", (6, 6, 6), False), ("rocksalt", (5, 5, 5), True), ("rocksalt", (6, 6, 4), False),
+    ("rocksalt", (13, 13, 13), False), ("fluorite", (5, 5, 5), False), ("l12", (4, 4, 4), False),
+    ("perovskite", (4, 4, 4), False), ("perovskite", (4, 4, 3), True), ("supercell", (3, 3, 3), False)])
 def test_iterative_solution_matches_the_oracle(configs, name, mesh, overlap):
-    prob = Problem.load(configs[name], (mesh,) * 3)
+    prob = Problem.load(configs[name], mesh)
     if overlap:
         _overlapping(prob)
-    opts = Options(integrationtype=2, isotopescattering=False, itertol=1e-7, itermaxsteps=60)
+    opts = Options(integrationtype=2, isotopescattering=False, itertol=1e-7, itermaxsteps=60,
+                   precision="mixed" if prob.n_mode > 18 else "fp64")
     lists = QLists.monte_carlo(prob, opts)
     sr = ScatteringRates(prob)
     lw = sr.generate(opts, lists)
