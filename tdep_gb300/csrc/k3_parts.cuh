@@ -167,18 +167,19 @@ __device__ __forceinline__ void k3_enqueue(const K3Smem &S, int b1b2, int k, uin
     }
 }
 
-// FP64 delta weights and occupations of the nq queued survivors, by full warps: F[idx] =
-// perm |Psi|^2 ((n2 - n3) d0 + (n2 + n3 + 1) d1) (the adjoint keeps dF/d|Psi|^2: psisq(idx)
-// returns 1) and the row/column bits of the non-zero entries. F must be zero beforehand.
-template <int N, typename PsiSq>
-__device__ __forceinline__ void k3_survivors(const K3Smem &S, const PhononDev &P, int nq, double perm,
-                                             PsiSq psisq) {
+// FP64 delta weights and occupations of the survivors q0 <= s < q1 of the queue, by full
+// warps: put(entry, F) with F = perm |Psi|^2 ((n2 - n3) d0 + (n2 + n3 + 1) d1), psisq(entry)
+// the |Psi|^2 of a survivor whose weights are not zero, width6(b1, b2, b3) its -it 6 width.
+// The low 16 bits of an entry are the (b1 b2 b3) index, the next four its live Gaussians.
+template <int N, typename Width6, typename PsiSq, typename Put>
+__device__ __forceinline__ void k3_survivors(const K3Smem &S, const PhononDev &P, int q0, int q1, double perm,
+                                             Width6 width6, PsiSq psisq, Put put) {
     constexpr int N2 = N * N;
     const int it = P.integrationtype;
-    for (int s = threadIdx.x; s < nq; s += blockDim.x) {
+    for (int s = q0 + threadIdx.x; s < q1; s += blockDim.x) {
         const uint32_t qv = S.Q[s];
         const int idx = (int)(qv & 0xffffu);
-        const uint32_t live = qv >> 16;
+        const uint32_t live = (qv >> 16) & 15u;
         const int b1 = idx / N2, b2 = (idx / N) % N, b3 = idx % N;
         const double o1 = S.om1[b1], o2 = S.om2[b2], o3 = S.om3[b3];
         double sigma, invsig;
@@ -190,48 +191,55 @@ __device__ __forceinline__ void k3_survivors(const K3Smem &S, const PhononDev &P
             invsig = rsqrt(sq);
             sigma = sq * invsig;
         } else {
-            sigma = adaptive_pair(S.v1 + 3 * b1, S.v2 + 3 * b2, P.reclat_g) / 3.0;
-            sigma += adaptive_pair(S.v1 + 3 * b1, S.v3 + 3 * b3, P.reclat_g) / 3.0;
-            sigma += adaptive_pair(S.v2 + 3 * b2, S.v3 + 3 * b3, P.reclat_g) / 3.0;
-            sigma += P.thresh_sigma;
+            sigma = width6(b1, b2, b3);
             invsig = 1.0 / sigma;
         }
         const double win8 = 8.0 * sigma, h = 0.5 * invsig * invsig, cg = kSqrt2PiInv * invsig;
         double d0, d1;
         dirac3(live, o1, o2, o3, win8, h, cg, P.exp2tab, d0, d1);
         if (nonzero(d0) || nonzero(d1)) {
-            const double pq = kThreePhononPrefactor * psisq(idx) * S.wrow[b1];
+            const double pq = kThreePhononPrefactor * psisq(qv) * S.wrow[b1];
             const double n2 = S.be2[b2], n3 = S.be3[b3];
             const double f0 = perm * pq * (n2 - n3) * d0;
             const double f1 = perm * pq * (n2 + n3 + 1.0) * d1;
-            const double fsum = f0 + f1;
-            S.F[idx] = fsum;
-            if (nonzero(fsum)) {
-                atomicOr(S.rowbits + b1 * N + b2, 1u << b3);
-                atomicOr(S.colbits + b1 * N + b3, 1u << b2);
-            }
+            put(qv, f0 + f1);
         }
     }
+}
+
+// Row and column bits of a survivor whose F is not zero.
+template <int N>
+__device__ __forceinline__ void k3_mark(const K3Smem &S, int idx) {
+    const int b1 = idx / (N * N), b2 = (idx / N) % N, b3 = idx % N;
+    atomicOr(S.rowbits + b1 * N + b2, 1u << b3);
+    atomicOr(S.colbits + b1 * N + b3, 1u << b2);
+}
+
+// The -it 6 width of a mode triplet from its velocities.
+__device__ __forceinline__ double k3_width6(const K3Smem &S, const PhononDev &P, int b1, int b2, int b3) {
+    double sigma = adaptive_pair(S.v1 + 3 * b1, S.v2 + 3 * b2, P.reclat_g) / 3.0;
+    sigma += adaptive_pair(S.v1 + 3 * b1, S.v3 + 3 * b3, P.reclat_g) / 3.0;
+    sigma += adaptive_pair(S.v2 + 3 * b2, S.v3 + 3 * b3, P.reclat_g) / 3.0;
+    return sigma + P.thresh_sigma;
 }
 
 // The same in FP32 for the mixed-precision kernels: the centre differences om1 - (+-om2 +-
 // om3) from FP32 pairs (centre_diff_f32, as accurate as the FP64 difference rounded to
 // FP32), the width, the exponent and the Gaussian in FP32 (expf), the occupation factors
-// and row weight from FP32 copies made once per mode, F in FP32 stored as a double for the
-// FP64 sums. Relative error of a weight about 1e-6, against the 1e-5 of the BF16x3
+// and row weight from FP32 copies made once per mode, F in FP32. Relative error of a weight about 1e-6, against the 1e-5 of the BF16x3
 // contraction.
-template <int N, bool FLOAT_F = false, typename PsiSq>
-__device__ __forceinline__ void k3_survivors_f32(const K3Smem &S, const PhononDev &P, int nq, float perm,
-                                                 PsiSq psisq) {
+template <int N, typename Width6, typename PsiSq, typename Put>
+__device__ __forceinline__ void k3_survivors_f32(const K3Smem &S, const PhononDev &P, int q0, int q1, float perm,
+                                                 Width6 width6, PsiSq psisq, Put put) {
     constexpr int N2 = N * N;
     constexpr float kSqrt2PiInvF = 0.3989422804014327f;
     const int it = P.integrationtype;
     const float sfix = (float)P.sigma_fixed;
     const float pref = (float)kThreePhononPrefactor;
-    for (int s = threadIdx.x; s < nq; s += blockDim.x) {
+    for (int s = q0 + threadIdx.x; s < q1; s += blockDim.x) {
         const uint32_t qv = S.Q[s];
         const int idx = (int)(qv & 0xffffu);
-        uint32_t live = qv >> 16;
+        uint32_t live = (qv >> 16) & 15u;
         const int b1 = idx / N2, b2 = (idx / N) % N, b3 = idx % N;
         float sigma;
         if (it == 1) {
@@ -239,9 +247,7 @@ __device__ __forceinline__ void k3_survivors_f32(const K3Smem &S, const PhononDe
         } else if (it == 2) {
             sigma = sqrtf(S.fs1[b1] + S.fs2[b2] + S.fs3[b3]);
         } else {
-            sigma = (float)(adaptive_pair(S.v1 + 3 * b1, S.v2 + 3 * b2, P.reclat_g) / 3.0 +
-                            adaptive_pair(S.v1 + 3 * b1, S.v3 + 3 * b3, P.reclat_g) / 3.0 +
-                            adaptive_pair(S.v2 + 3 * b2, S.v3 + 3 * b3, P.reclat_g) / 3.0 + P.thresh_sigma);
+            sigma = (float)width6(b1, b2, b3);
         }
         const float invsig = 1.0f / sigma;
         const float win8 = 8.0f * sigma, h = 0.5f * invsig * invsig, cg = kSqrt2PiInvF * invsig;
@@ -262,17 +268,9 @@ __device__ __forceinline__ void k3_survivors_f32(const K3Smem &S, const PhononDe
         }
         const float d0 = g[0] - g[1], d1 = g[2] - g[3];
         if (d0 != 0.f || d1 != 0.f) {
-            const float pq = pref * psisq(idx) * S.fw1[b1];
+            const float pq = pref * psisq(qv) * S.fw1[b1];
             const float n2 = S.fb2[b2], n3 = S.fb3[b3];
-            const float fsum = perm * pq * ((n2 - n3) * d0 + (n2 + n3 + 1.0f) * d1);
-            if constexpr (FLOAT_F)
-                S.Ff[idx] = fsum;
-            else
-                S.F[idx] = (double)fsum;
-            if (fsum != 0.f) {
-                atomicOr(S.rowbits + b1 * N + b2, 1u << b3);
-                atomicOr(S.colbits + b1 * N + b3, 1u << b2);
-            }
+            put(qv, perm * pq * ((n2 - n3) * d0 + (n2 + n3 + 1.0f) * d1));
         }
     }
 }
@@ -280,8 +278,8 @@ __device__ __forceinline__ void k3_survivors_f32(const K3Smem &S, const PhononDe
 // Row sums over b3 (R2) and column sums over b2 (R3) of the non-zero F, Gamma of every
 // sampling row times the nred equivalent triplets, then the Xi row terms 2 F om/om1 added
 // for each equivalent triplet (scattering_threephonon.f90:115-135). Starts and ends with
-// barriers of its own.
-template <int N, bool FLOAT_F = false>
+// barriers of its own. F of (b1, b2, b3) lies at b1 FS + b2 N + b3.
+template <int N, bool FLOAT_F = false, int FS = N * N>
 __device__ __forceinline__ void k3_sums_scatter(const K3Smem &S, const ThreePhArgs &a, int nred) {
     constexpr int N2 = N * N;
     const int tid = threadIdx.x, bd = blockDim.x;
@@ -295,7 +293,7 @@ __device__ __forceinline__ void k3_sums_scatter(const K3Smem &S, const ThreePhAr
         float2 dsum = make_float2(0.f, 0.f);
         if (e < N2) {
             for (uint32_t bits = S.rowbits[e]; bits; bits &= bits - 1) {
-                const int i = e * N + __ffs(bits) - 1;
+                const int i = (e / N) * FS + (e % N) * N + __ffs(bits) - 1;
                 if constexpr (FLOAT_F)
                     df_acc(dsum, S.Ff[i]);
                 else
@@ -305,7 +303,7 @@ __device__ __forceinline__ void k3_sums_scatter(const K3Smem &S, const ThreePhAr
         } else {
             const int e3 = e - N2, b1 = e3 / N, b3 = e3 % N;
             for (uint32_t bits = S.colbits[e3]; bits; bits &= bits - 1) {
-                const int i = (b1 * N + __ffs(bits) - 1) * N + b3;
+                const int i = b1 * FS + (__ffs(bits) - 1) * N + b3;
                 if constexpr (FLOAT_F)
                     df_acc(dsum, S.Ff[i]);
                 else

@@ -15,18 +15,26 @@
 // lattice vectors, so q.lv = sum_d g_d lv_d / N_d and exp(-2 pi i q.lv) is one entry of a
 // table of exp(-2 pi i K / L), L = lcm of the mesh dimensions.
 //
-// Delta weights stay FP64 as in the reference. GB300's FP64 pipe is narrow and the mode
-// triplets whose Gaussians fall inside the 8-sigma window of lo_gauss are sparse, so:
-//   1. the reference's skip rules become per-triplet bit masks (3 n^2 FP64 compares);
-//   2. every mode triplet and each of the four Gaussians of get_dirac is screened in FP32
-//      against the window, with a relative margin of 1e-3 and an absolute margin far
-//      above FP32 rounding (a Gaussian the screen drops is exactly 0 in the reference);
-//   3. the survivors are compacted into a shared-memory queue (block scan) and evaluated
-//      in FP64 by full warps, with the reference's own window test and formulas.
+// With adaptive widths few mode triplets have a Gaussian inside its 8-sigma window (2 % at
+// rocksalt 24^3, 3-12 % at 9 to 15 modes), and at two atoms 59 % of the q-triplets have none,
+// so the screen comes before the contraction and the contraction is driven by it:
+//   1. every mode triplet and each of the four Gaussians of get_dirac is screened in FP32
+//      against the window, with a relative margin of 1e-3 and an absolute margin far above
+//      FP32 rounding (a Gaussian the screen drops is exactly 0 in the reference); the
+//      reference's skip rules are tests of the same loop. A q-triplet without survivors ends
+//      here: its terms are exactly 0;
+//   2. pretransform and the first stage (n^4 complex MACs), in place;
+//   3. the second stage for the (b1, b2) that have a survivor, the third for the survivors
+//      alone, a thread each, followed by their weights with the reference's own window test
+//      and formulas.
+// Each value that is formed is the same sum in the same order as in the full contraction.
+// Bound: FP64 runs the FP64 pipe (2 lanes per clock and SM): perovskite 8^3 5.6 -> 3.1 ms,
+// L1_2 9^3 (-it 6) 6.4 -> 2.2 ms; mixed precision at n = 6 instruction issue and the latency
+// of the phases: rocksalt 24^3 14.6 -> 4.3 ms.
 //
 // Everything for one triplet lives in shared memory. Precision R is double (FP64 path)
-// or float (mixed path: FP32 pretransform and contraction, FP64 delta weights,
-// occupations and accumulation).
+// or float (mixed path: FP32 pretransform and contraction, FP32 delta weights,
+// occupations and FP64 accumulation).
 #include <cuda_runtime.h>
 
 #include "dev_common.cuh"
@@ -39,14 +47,17 @@ namespace {
 
 constexpr int kPhaseChunk = 512;
 // Phase factors held in shared memory at a time: at least kPhaseChunk, more when the survivor
-// queue, which later reuses the eigenvector and phase region, is larger anyway (n = 15 in
-// FP32: 1008, so that 1115 force-constant triplets take two passes instead of three at no
-// cost in shared memory).
-__host__ __device__ constexpr int phase_chunk(int n, int cs) {
-    const int ez = (cs * n * n + 15) / 16 * 16;
-    const int qsz = (4 * n * n * n + 15) / 16 * 16;
-    const int room = (qsz - 3 * ez) / cs / 16 * 16;
+// queue, which takes their place afterwards, is larger anyway (n = 15 in FP32: 1680; in the
+// adjoint, where it takes that of two eigenvector matrices as well, 1232).
+__host__ __device__ constexpr int phase_chunk(int n, int cs, bool adj) {
+    const int room = (4 * n * n * n - (adj ? 2 * cs * n * n : 0)) / cs / 16 * 16;
     return room > kPhaseChunk ? room : kPhaseChunk;
+}
+// b1 per pass of the second and third stages: all of them where their two n^3 buffers leave
+// CTAs enough on an SM, else so many that they do (FP64 at n = 15: one buffer of n^3 and one
+// of n^3 / 3, two CTAs instead of one). The adjoint needs both buffers whole.
+__host__ __device__ constexpr int b1_pass(int n, int cs, bool adj) {
+    return adj || cs == 8 || n < 12 ? n : (n == 15 ? 5 : 6);
 }
 
 template <typename R>
@@ -112,11 +123,10 @@ __device__ __forceinline__ C phase3(const Fc3Dev &fc, const MeshDev &m, const in
 
 // Shared-memory layout (bytes) for mode count n and complex size cs.
 struct Layout {
-    size_t om1, om2, om3, inv1, be2, be3, s1, s2, s3, v1, v2, v3, wrow, r2, f32, masks, E1, E2, E3, ph, Q, A, B,
-        rowid, red, wsum, xb, total;
+    size_t om1, om2, om3, inv1, be2, be3, s1, s2, s3, wrow, w6, r2, f32, bits, E1, E2, E3, ph, Q, pairs, A, B, rowid,
+        red, wsum, xb, total;
 };
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
-// adj: the adjoint's extra n^2 doubles (column sums of the scattering-matrix cotangent).
 __host__ __device__ inline Layout make_layout(int n, int cs, bool adj = false) {
     Layout L;
     size_t o = 0;
@@ -131,37 +141,41 @@ __host__ __device__ inline Layout make_layout(int n, int cs, bool adj = false) {
     L.s1 = o; o += dn;
     L.s2 = o; o += dn;
     L.s3 = o; o += dn;
-    L.v1 = o; o += 3 * dn;
-    L.v2 = o; o += 3 * dn;
-    L.v3 = o; o += 3 * dn;
     L.wrow = o; o += dn;
     L.r2 = o; o += align16(sizeof(double) * n2);
     L.f32 = o; o += align16(sizeof(float) * n * 12);           // om1..3, s1..3, om lo parts, be2, be3, wrow in FP32
-    L.masks = o; o += align16(sizeof(uint32_t) * (3 * n + 2 + 2 * n2));  // m12, m13, m23, z2, z3, row/col bits
-    // E1..E3 and the phase chunk are dead once Psi is formed: the survivor queue reuses them.
+    L.bits = o; o += align16(sizeof(uint32_t) * 2 * n2);       // row/col bits of the non-zero F
     const size_t ez = align16(cs * n2);
-    L.E1 = o;
-    L.E2 = o + ez;
-    L.E3 = o + 2 * ez;
-    L.ph = o + 3 * ez;
-    const size_t eph = 3 * ez + align16((size_t)cs * phase_chunk(n, cs));
-    const size_t qsz = align16(sizeof(uint32_t) * n3);
-    L.Q = o;
-    o += eph > qsz ? eph : qsz;
-    // A and B each hold n^3 complex values and at least n^3 doubles.
-    const size_t csz = (size_t)cs > sizeof(double) ? (size_t)cs : sizeof(double);
-    const size_t buf = align16(csz * n3);
-    L.A = o; o += buf;
-    L.B = o; o += buf;
+    const size_t eph = align16((size_t)cs * phase_chunk(n, cs, adj)), qsz = align16(sizeof(uint32_t) * n3);
+    if (adj) {
+        // the queue, filled after the second stage, takes the place of E1, E2 and the phases
+        // (the back-contraction loads the matrices again): at n = 18 in FP64 the two n^3
+        // buffers leave no more room
+        L.E3 = o; o += ez;
+        L.Q = L.E1 = o;
+        L.E2 = o + ez;
+        L.ph = o + 2 * ez;
+        o += 2 * ez + eph > qsz ? 2 * ez + eph : qsz;
+    } else {
+        // the phases are dead after the pretransform: the survivor queue takes their place
+        L.E1 = o; o += ez;
+        L.E2 = o; o += ez;
+        L.E3 = o; o += ez;
+        L.Q = L.ph = o; o += eph > qsz ? eph : qsz;
+        L.w6 = o; o += align16(sizeof(double) * 3 * n2);       // -it 6: widths of the mode pairs
+    }
+    L.pairs = o; o += align16(sizeof(uint16_t) * n2);          // the (b1, b2) with survivors
+    // A: n^3 complex values, then (dense F, a slab of n^2 complex per b1) n^3 doubles; B: the
+    // second stage of the b1 of a pass (the adjoint: of all), then 3 n^2 doubles
+    L.A = o; o += align16(cs * n3);
+    if (adj) L.w6 = L.A;                                       // for the screen only
+    const size_t bsz = (size_t)cs * b1_pass(n, cs, adj) * n2, dsz = sizeof(double) * 3 * n2;
+    L.B = o; o += align16(bsz > dsz ? bsz : dsz);
     L.rowid = o; o += align16(sizeof(int) * n);
     L.red = o; o += align16(sizeof(int2) * kMaxRed);
-    L.wsum = o; o += align16(sizeof(int) * 33);
-    // The adjoint's xi_bar sums over b2 (n^2 doubles) live in the survivor-queue region: they
-    // are written after the survivors are done and read before the eigenvectors are loaded
-    // there again (4 n^3 >= 8 n^2 bytes). Keeping them separate cost 1.8 KB at n = 15 and
-    // the third CTA per SM.
-    L.xb = L.Q;
-    (void)adj;
+    L.wsum = o; o += align16(sizeof(int) * 48);                // block scan [33], pass starts in queue and pairs
+    // the adjoint does not mark rows and columns: its xi_bar sums over b2 (n^2 doubles)
+    L.xb = L.bits;
     L.total = o;
     return L;
 }
@@ -174,7 +188,8 @@ __host__ __device__ constexpr int threads_for(int n) { return ((n * n + 31) / 32
 __host__ __device__ constexpr int min_blocks_for(int n, bool dbl, bool adj) {
     return n <= 3 ? 16
                   : (n <= 6 ? (adj || dbl ? 12 : 16)
-                            : (n <= 9 ? 6 : (dbl ? (n <= 12 ? 2 : 1) : (n <= 15 ? 3 : 2))));
+                            : (n <= 9 ? 6 : (dbl ? (adj ? (n <= 12 ? 2 : 1) : (n <= 12 ? 3 : (n <= 15 ? 2 : 1)))
+                                                 : (n <= 15 ? 3 : 2))));
 }
 
 // ADJ = false: Gamma and the Xi row terms. ADJ = true: the adjoint pass, which recomputes
@@ -184,50 +199,38 @@ __global__ void __launch_bounds__(threads_for(N), min_blocks_for(N, sizeof(R) ==
     using C = typename CT<R>::C;
     constexpr int N2 = N * N, N3 = N2 * N;
     constexpr int NA = N / 3;
-    constexpr uint32_t kAll = (N >= 32) ? 0xffffffffu : ((1u << N) - 1u);
+    constexpr int NB1 = b1_pass(N, sizeof(C), ADJ), PASSES = N / NB1;
+    static_assert(PASSES * NB1 == N, "passes of equal size");
+    constexpr int FS = N2 * (int)(sizeof(C) / sizeof(double));  // doubles per b1 slab of A
     extern __shared__ __align__(16) unsigned char smem[];
     const Layout L = make_layout(N, sizeof(C), ADJ);
-    double *om1 = (double *)(smem + L.om1);
-    double *om2 = (double *)(smem + L.om2);
-    double *om3 = (double *)(smem + L.om3);
-    double *inv1 = (double *)(smem + L.inv1);
-    double *be2 = (double *)(smem + L.be2);
-    double *be3 = (double *)(smem + L.be3);
-    double *s1 = (double *)(smem + L.s1);
-    double *s2 = (double *)(smem + L.s2);
-    double *s3 = (double *)(smem + L.s3);
-    double *v1 = (double *)(smem + L.v1);
-    double *v2 = (double *)(smem + L.v2);
-    double *v3 = (double *)(smem + L.v3);
-    double *wrow = (double *)(smem + L.wrow);
-    double *R2 = (double *)(smem + L.r2);
-    float *fo1 = (float *)(smem + L.f32);
-    float *fo2 = fo1 + N, *fo3 = fo2 + N, *fs1 = fo3 + N, *fs2 = fs1 + N, *fs3 = fs2 + N;
-    uint32_t *m12 = (uint32_t *)(smem + L.masks);
-    uint32_t *m13 = m12 + N, *m23 = m13 + N, *zmask = m23 + N;  // zmask[0]: omega2 < tol, zmask[1]: omega3 < tol
-    // b3 with a non-zero F for each (b1, b2), and b2 for each (b1, b3): the row and column sums
-    // then add only those terms (adding an exact zero changes nothing)
-    uint32_t *rowbits = zmask + 2, *colbits = rowbits + N2;
+    float *f32 = (float *)(smem + L.f32);
     C *E1 = (C *)(smem + L.E1);
     C *E2 = (C *)(smem + L.E2);
     C *E3 = (C *)(smem + L.E3);
     C *ph = (C *)(smem + L.ph);
-    uint32_t *Q = (uint32_t *)(smem + L.Q);
+    uint16_t *pairs = (uint16_t *)(smem + L.pairs);
     C *A = (C *)(smem + L.A);
     C *B = (C *)(smem + L.B);
-    int *rowid = (int *)(smem + L.rowid);
-    int2 *red = (int2 *)(smem + L.red);
-    int *wsum = (int *)(smem + L.wsum);
+    double *F = (double *)A;
+    double *W6 = (double *)(smem + L.w6);
     K3Smem S;
-    S.om1 = om1; S.om2 = om2; S.om3 = om3; S.inv1 = inv1; S.be2 = be2; S.be3 = be3;
-    S.s1 = s1; S.s2 = s2; S.s3 = s3; S.v1 = v1; S.v2 = v2; S.v3 = v3; S.wrow = wrow;
-    S.R2 = R2; S.R3 = (double *)B; S.F = (double *)A; S.Ff = nullptr;
-    S.R2s = S.R3 + N2; S.R3s = S.R2s + N2;  // B (8 n^3 or more bytes) is free when the sums start
-    S.fo1 = fo1; S.fo2 = fo2; S.fo3 = fo3; S.fs1 = fs1; S.fs2 = fs2; S.fs3 = fs3;
-    S.fl1 = fs3 + N; S.fl2 = fs3 + 2 * N; S.fl3 = fs3 + 3 * N; S.fb2 = fs3 + 4 * N; S.fb3 = fs3 + 5 * N;
-    S.fw1 = fs3 + 6 * N;
-    S.m12 = m12; S.m13 = m13; S.m23 = m23; S.zmask = zmask; S.rowbits = rowbits; S.colbits = colbits;
-    S.Q = Q; S.rowid = rowid; S.red = red; S.wsum = wsum;
+    S.om1 = (double *)(smem + L.om1); S.om2 = (double *)(smem + L.om2); S.om3 = (double *)(smem + L.om3);
+    S.inv1 = (double *)(smem + L.inv1); S.be2 = (double *)(smem + L.be2); S.be3 = (double *)(smem + L.be3);
+    S.s1 = (double *)(smem + L.s1); S.s2 = (double *)(smem + L.s2); S.s3 = (double *)(smem + L.s3);
+    S.wrow = (double *)(smem + L.wrow);
+    S.R2 = (double *)(smem + L.r2);
+    S.R3 = (double *)B; S.R2s = S.R3 + N2; S.R3s = S.R2s + N2;  // B is free when the sums start
+    S.F = F;
+    S.fo1 = f32; S.fo2 = f32 + N; S.fo3 = f32 + 2 * N; S.fs1 = f32 + 3 * N; S.fs2 = f32 + 4 * N; S.fs3 = f32 + 5 * N;
+    S.fl1 = f32 + 6 * N; S.fl2 = f32 + 7 * N; S.fl3 = f32 + 8 * N; S.fb2 = f32 + 9 * N; S.fb3 = f32 + 10 * N;
+    S.fw1 = f32 + 11 * N;
+    S.rowbits = (uint32_t *)(smem + L.bits); S.colbits = S.rowbits + N2;
+    S.Q = (uint32_t *)(smem + L.Q);
+    S.rowid = (int *)(smem + L.rowid);
+    S.red = (int2 *)(smem + L.red);
+    S.wsum = (int *)(smem + L.wsum);
+    int *qstart = S.wsum + 33, *pstart = qstart + 7;  // first entry of each pass, and the ends
     const int tid = threadIdx.x, bd = blockDim.x;
     const MeshDev &m = a.mesh;
     const PhononDev &P = a.ph;
@@ -255,7 +258,96 @@ __global__ void __launch_bounds__(threads_for(N), min_blocks_for(N, sizeof(R) ==
         const int i2 = m.full_irr[q2], i3 = m.full_irr[q3];
         const int nred = rec.red_cnt;
         const double perm = (q2 == q3) ? 1.0 : 2.0;
-        k3_load_modes<N>(S, a, rec, f1, q2, q3, i2, i3);
+        // ---- what the screen reads: omega (NaN where no survivor may be: below 1e-9 Ha, or a
+        // row that does not sample q2) and sigsq, FP32; -it 6: the widths of the mode pairs ----
+        for (int i = tid; i < 3 * N; i += bd) {
+            const int which = i / N, b = i - which * N;
+            const int q = which == 0 ? f1 : (which == 1 ? q2 : q3);
+            const float2 w = P.omega_hl[(size_t)q * N + b];
+            bool on = true;
+            if (which == 0) {
+                const uint32_t mask = a.cand_mask[(size_t)rec.cand * 4 + (b >> 5)];
+                const int r = (mask >> (b & 31)) & 1u ? a.rows.rowidx[(size_t)rec.q1 * N + b] : -1;
+                S.rowid[b] = r;
+                on = r >= 0;
+            }
+            f32[i] = on ? w.x : __int_as_float(0x7fc00000);
+            f32[6 * N + i] = w.y;
+            f32[3 * N + i] = P.sigsq32[(size_t)(which == 0 ? rec.q1 : (which == 1 ? i2 : i3)) * N + b];
+        }
+        if (it == 6)
+            for (int i = tid; i < 3 * N2; i += bd) {
+                const int which = i / N2, x = (i - which * N2) / N, y = i % N;
+                W6[i] = adaptive_pair(P.vel + ((size_t)(which == 2 ? q2 : f1) * N + x) * 3,
+                                      P.vel + ((size_t)(which == 0 ? q2 : q3) * N + y) * 3, P.reclat_g) / 3.0;
+            }
+        __syncthreads();
+        const auto width6 = [&](int b1, int b2, int b3) {
+            return W6[b1 * N + b2] + W6[N2 + b1 * N + b3] + W6[2 * N2 + b2 * N + b3] + P.thresh_sigma;
+        };
+        const auto width6_again = [&](int b1, int b2, int b3) {  // once A holds something else
+            const double *v1 = P.vel + ((size_t)f1 * N + b1) * 3, *v2 = P.vel + ((size_t)q2 * N + b2) * 3,
+                         *v3 = P.vel + ((size_t)q3 * N + b3) * 3;
+            const double w12 = adaptive_pair(v1, v2, P.reclat_g) / 3.0, w13 = adaptive_pair(v1, v3, P.reclat_g) / 3.0;
+            return w12 + w13 + adaptive_pair(v2, v3, P.reclat_g) / 3.0 + P.thresh_sigma;
+        };
+        // ---- screen: a thread per (b1, b2), its live bits kept in registers ----
+        uint32_t live_lo = 0u, live_hi = 0u, live_x = 0u;  // 4 bits for b3 = 0..7, 8..15, 16..17
+        int nsurv = 0;
+        if (tid < N2) {
+            const int b1 = tid / N, b2 = tid - b1 * N;
+            const float o1 = S.fo1[b1], o2 = S.fo2[b2], l1 = S.fl1[b1], l2 = S.fl2[b2];
+            const float s12 = S.fs1[b1] + S.fs2[b2], p12 = o1 + o2, d12 = o1 - o2;
+            // |omega - omega'| < 1e-9 (scattering_threephonon.f90:90-101) where the high parts
+            // are that near, decided on the pairs
+            const float near1 = 1e-9f + 3e-7f * o1, near2 = 1e-9f + 3e-7f * o2;
+            if (o1 == o1 && o2 == o2 && !close_f32(o1, l1, o2, l2)) {
+#pragma unroll
+                for (int b3 = 0; b3 < N; ++b3) {
+                    const float o3 = S.fo3[b3];
+                    float sg = sigfix32;
+                    if (it == 2) sg = sqrt_screen(s12 + S.fs3[b3]);
+                    else if (it == 6) sg = (float)width6(b1, b2, b3);
+                    const float win = 8.0f * sg * 1.001f + 1e-6f * (p12 + o3);
+                    uint32_t live = (fabsf(p12 - o3) <= win ? 1u : 0u) | (fabsf(d12 + o3) <= win ? 2u : 0u) |
+                                    (fabsf(d12 - o3) <= win ? 4u : 0u) | (p12 + o3 <= win ? 8u : 0u);
+                    if ((fabsf(o1 - o3) < near1 && close_f32(o1, l1, o3, S.fl3[b3])) ||
+                        (fabsf(o2 - o3) < near2 && close_f32(o2, l2, o3, S.fl3[b3])))
+                        live = 0u;
+                    if (live) {
+                        ++nsurv;
+                        if (b3 < 8) live_lo |= live << (4 * b3);
+                        else if (b3 < 16) live_hi |= live << (4 * (b3 - 8));
+                        else live_x |= live << (4 * (b3 - 16));
+                    }
+                }
+            }
+        }
+        // survivors in the low half, (b1, b2) with any in the high half (n^3 <= 5832 entries)
+        int total = 0;
+        const int off = block_exclusive_scan(nsurv | (nsurv ? 1 << 16 : 0), S.wsum, total);  // contains barriers
+        if (total == 0) continue;
+        // ---- the rest of the mode data, eigenvectors, equivalent triplets ----
+        for (int b = tid; b < N; b += bd) {
+            S.om1[b] = P.omega[(size_t)f1 * N + b];
+            S.om2[b] = P.omega[(size_t)q2 * N + b];
+            S.om3[b] = P.omega[(size_t)q3 * N + b];
+            S.inv1[b] = P.inv_omega[(size_t)f1 * N + b];
+            S.be2[b] = P.be[(size_t)i2 * N + b];
+            S.be3[b] = P.be[(size_t)i3 * N + b];
+            S.wrow[b] = a.rows.w3q[(size_t)rec.q1 * N + b];
+            if constexpr (sizeof(R) == 8) {
+                S.s1[b] = P.sigsq[(size_t)rec.q1 * N + b];
+                S.s2[b] = P.sigsq[(size_t)i2 * N + b];
+                S.s3[b] = P.sigsq[(size_t)i3 * N + b];
+            } else {
+                S.fb2[b] = (float)S.be2[b];
+                S.fb3[b] = (float)S.be3[b];
+                S.fw1[b] = (float)S.wrow[b];
+            }
+        }
+        for (int i = tid; i < nred && i < kMaxRed; i += bd) S.red[i] = a.red[rec.red_off + i];
+        for (int i = tid; i < 2 * N2; i += bd) S.rowbits[i] = 0u;
         for (int i = tid; i < 3 * N2; i += bd) {
             const int which = i / N2, e = i % N2;
             const int r = e / N, b = e % N;  // element (r) of mode b
@@ -263,10 +355,18 @@ __global__ void __launch_bounds__(threads_for(N), min_blocks_for(N, sizeof(R) ==
             C *E = which == 0 ? E1 : (which == 1 ? E2 : E3);
             E[r * N + b] = egvs[((size_t)q * N + b) * N + r];
         }
-        for (int i = tid; i < N3; i += bd) A[i] = czero<C>();
-        __syncthreads();
-        // ---- skip rules of scattering_threephonon.f90:90-101 as bit masks ----
-        k3_skip_masks<N>(S);
+        if (tid < N2) {
+            const int b1 = tid / N;
+            if (tid == b1 * N && b1 % NB1 == 0) {
+                qstart[b1 / NB1] = off & 0xffff;
+                pstart[b1 / NB1] = off >> 16;
+            }
+            if (nsurv) pairs[off >> 16] = (uint16_t)tid;
+            if (tid == 0) {
+                qstart[PASSES] = total & 0xffff;
+                pstart[PASSES] = total >> 16;
+            }
+        }
         // ---- K2: pretransform into A ----
         int gi2[3], gi3[3];
         {
@@ -278,15 +378,15 @@ __global__ void __launch_bounds__(threads_for(N), min_blocks_for(N, sizeof(R) ==
                 gi3[d] *= m.lmul[d];
             }
         }
-        constexpr int PC = phase_chunk(N, sizeof(C));
+        constexpr int PC = phase_chunk(N, sizeof(C), ADJ);
         bool planned = false;
         if constexpr (sizeof(R) == 4) {
             // FP32 with a pretransform plan (all phase factors at once; k_threephonon_tc.cu
             // explains the plan): each thread's slots, 8 values and 8 words in flight, the
-            // sums in the triplets' order as below
+            // sums in the triplets' order as below; it writes the blocks that have triplets
             if (a.plan_slots > 0) {
                 planned = true;
-                __syncthreads();
+                for (int i = tid; i < N3; i += bd) A[i] = czero<C>();
                 // four triplets per thread in flight: their lattice vectors, then their table entries
                 for (int i0 = tid; i0 < fc.n + 4; i0 += 4 * bd) {
                     int kk[4];
@@ -343,28 +443,43 @@ __global__ void __launch_bounds__(threads_for(N), min_blocks_for(N, sizeof(R) ==
         }
         for (int c0 = 0; !planned && c0 < fc.n; c0 += PC) {
             const int cn = min(PC, fc.n - c0);
-            __syncthreads();
+            if (c0) __syncthreads();
             for (int i = tid; i < cn; i += bd) ph[i] = phase3<C>(fc, m, gi2, gi3, c0 + i);
             __syncthreads();
             for (int idx = tid; idx < N3; idx += bd) {
                 const int blk = idx / 27, ijk = idx % 27;
                 const int lo = max(fc.blk_ptr[blk], c0), hi = min(fc.blk_ptr[blk + 1], c0 + cn);
-                if (lo >= hi) continue;
+                if (c0 && lo >= hi) continue;
                 const int a1 = blk / (NA * NA), a2 = (blk / NA) % NA, a3 = blk % NA;
                 const int ii = ijk % 3, jj = (ijk / 3) % 3, kk = ijk / 9;
                 const int pa = 3 * a1 + ii, pb = 3 * a2 + jj, pc = 3 * a3 + kk;
-                C acc = A[(pa * N + pb) * N + pc];
+                C *out = A + (pa * N + pb) * N + pc;
+                C acc = c0 ? *out : czero<C>();
                 for (int tt = lo; tt < hi; ++tt) {
                     const R mv = __ldg(mwm + (size_t)tt * 27 + ijk);
                     const C p = ph[tt - c0];
                     acc.x = fma(mv, p.x, acc.x);
                     acc.y = fma(mv, p.y, acc.y);
                 }
-                A[(pa * N + pb) * N + pc] = acc;
+                *out = acc;
             }
         }
         __syncthreads();
-        // ---- K3: T1 into B, T2 into A ----
+        // ---- the queue, in the phases' place: (b1 b2 b3) | live << 16 | place of (b1, b2) in
+        // its pass << 20 ----
+        const auto enqueue = [&]() {
+            if (!nsurv) return;
+            int k = off & 0xffff;
+            const uint32_t place = (uint32_t)((off >> 16) - pstart[tid / N / NB1]) << 20;
+#pragma unroll
+            for (int b3 = 0; b3 < N; ++b3) {
+                const uint32_t live = b3 < 8 ? (live_lo >> (4 * b3)) & 15u
+                                             : (b3 < 16 ? (live_hi >> (4 * (b3 - 8))) & 15u : (live_x >> (4 * (b3 - 16))) & 15u);
+                if (live) S.Q[k++] = (uint32_t)(tid * N + b3) | (live << 16) | place;
+            }
+        };
+        if constexpr (!ADJ) enqueue();
+        // ---- K3: T1 in place (a thread owns a column) ----
         if (tid < N2) {
             const int bc = tid;
             C acc[N];
@@ -377,169 +492,146 @@ __global__ void __launch_bounds__(threads_for(N), min_blocks_for(N, sizeof(R) ==
                 for (int b1 = 0; b1 < N; ++b1) cfma(acc[b1], E1[aa * N + b1], p);
             }
 #pragma unroll
-            for (int b1 = 0; b1 < N; ++b1) B[b1 * N2 + bc] = acc[b1];
+            for (int b1 = 0; b1 < N; ++b1) A[b1 * N2 + bc] = acc[b1];
         }
         __syncthreads();
-        if (tid < N2) {
-            const int b1 = tid / N, c = tid % N;
-            C acc[N];
+        for (int pass = 0; pass < PASSES; ++pass) {
+            // T2[place][c] of the pass's pairs into B
+            const int p0 = pstart[pass], np = pstart[pass + 1] - p0;
+            for (int i = tid; i < np * N; i += bd) {
+                const int k = i / N, c = i - k * N, pr = pairs[p0 + k], b1 = pr / N, b2 = pr - b1 * N;
+                const C *t1 = A + b1 * N2 + c, *e = E2 + b2;
+                C acc = czero<C>();
 #pragma unroll
-            for (int b2 = 0; b2 < N; ++b2) acc[b2] = czero<C>();
-#pragma unroll 3
-            for (int b = 0; b < N; ++b) {
-                const C tv = B[(b1 * N + b) * N + c];
-#pragma unroll
-                for (int b2 = 0; b2 < N; ++b2) cfma(acc[b2], E2[b * N + b2], tv);
-            }
-#pragma unroll
-            for (int b2 = 0; b2 < N; ++b2) A[(b1 * N + b2) * N + c] = acc[b2];
-        }
-        __syncthreads();
-        // ---- Psi into B; FP32 screen of the Gaussians, survivors counted per thread ----
-        uint32_t live_lo = 0u, live_hi = 0u;  // 4-bit live masks of b3 = 0..7 and 8..15
-        uint32_t live_x = 0u;                 // b3 = 16, 17
-        int nsurv = 0;
-        if (tid < N2) {
-            const int b1 = tid / N, b2 = tid % N;
-            C acc[N];
-#pragma unroll
-            for (int b3 = 0; b3 < N; ++b3) acc[b3] = czero<C>();
-#pragma unroll 3
-            for (int c = 0; c < N; ++c) {
-                const C tv = A[(b1 * N + b2) * N + c];
-#pragma unroll
-                for (int b3 = 0; b3 < N; ++b3) cfma(acc[b3], E3[c * N + b3], tv);
-            }
-#pragma unroll
-            for (int b3 = 0; b3 < N; ++b3) B[(b1 * N + b2) * N + b3] = acc[b3];
-            nsurv = k3_screen<N>(S, it, sigfix32, b1, b2, live_lo, live_hi, live_x);
-        }
-        int nq = 0;
-        const int off = block_exclusive_scan(nsurv, wsum, nq);  // contains __syncthreads
-        // E1..E3 and the phases are dead: the queue overwrites them.
-        if (tid < N2 && nsurv) k3_enqueue<N>(S, tid, off, live_lo, live_hi, live_x);
-        // dense F (doubles) in A; the forward pass reads it only where the row/column bits
-        // are set (entries its survivors wrote), the adjoint all of it (zero where no survivor)
-        double *F = (double *)A;
-        if constexpr (ADJ)
-            for (int i = tid; i < N3; i += bd) F[i] = 0.0;
-        __syncthreads();
-        // ---- delta weights and occupations for the survivors, full warps: FP64 for FP64
-        // runs, FP32 (from FP64 centre differences) in mixed precision, as the tensor-core
-        // kernel; the adjoint keeps d F / d|Psi|^2, i.e. F without |Psi|^2 ----
-        if constexpr (sizeof(R) == 8) {
-            k3_survivors<N>(S, P, nq, perm, [&](int idx) -> double {
-                if constexpr (ADJ) {
-                    return 1.0;
-                } else {
-                    const C psi = B[idx];
-                    return (double)psi.x * (double)psi.x + (double)psi.y * (double)psi.y;
-                }
-            });
-        } else {
-            k3_survivors_f32<N>(S, P, nq, (float)perm, [&](int idx) -> float {
-                if constexpr (ADJ) {
-                    return 1.0f;
-                } else {
-                    const C psi = B[idx];
-                    return (float)psi.x * (float)psi.x + (float)psi.y * (float)psi.y;
-                }
-            });
-        }
-        __syncthreads();
-        if constexpr (ADJ) {
-            // d L / d|Psi_b|^2 = lam[row(b1)] * nred * dF_b/d|Psi_b|^2 (Gamma += nred * sum F);
-            // d|Psi|^2 / d P[abc] = 2 Re(conj(Psi) E1[a][b1] E2[b][b2] E3[c][b3]), so with
-            // W = G conj(Psi):  Q[abc] = sum_b W_b E1[a][b1] E2[b][b2] E3[c][b3] and
-            // d L / d mwm_t(i,j,k) = 2 Re(phase_t Q[3a1+i][3a2+j][3a3+k]).
-            // with a scattering-matrix cotangent xi_bar (the BTE adjoint): the Xi row terms
-            // 2 F om2/om1 at (q2', b2) and 2 F om3/om1 at (q3', b3) of every equivalent
-            // triplet add xi_bar(row, .) times those factors to the cotangent of F;
-            // R2[b1][b2] and XB[b1][b3] hold xi_bar summed over the equivalent triplets
-            double *XB = (double *)(smem + L.xb);
-            if (a.xi_bar) {
-                for (int e = tid; e < 2 * N2; e += bd) {
-                    const int x = e % N2, b1 = x / N, bb = x % N, row = rowid[b1];
-                    double sum = 0.0;
-                    if (row >= 0) {
-                        const double *wr = a.xi_bar + (int64_t)row * ld;
-                        for (int k = 0; k < nred; ++k) {
-                            const int2 pr = red[k];
-                            sum += wr[(int64_t)(e < N2 ? pr.x : pr.y) * N + bb];
-                        }
-                    }
-                    if (e < N2) R2[x] = sum;
-                    else XB[x] = sum;
-                }
-                __syncthreads();
-            }
-            for (int i = tid; i < N3; i += bd) {
-                const int row = rowid[i / N2];
-                double cot = row >= 0 ? a.lam[row] * (double)nred : 0.0;
-                if (a.xi_bar && row >= 0) {
-                    const int b1 = i / N2, b2 = (i / N) % N, b3 = i % N;
-                    cot += 2.0 * (om2[b2] * R2[b1 * N + b2] + om3[b3] * XB[b1 * N + b3]) * inv1[b1];
-                }
-                const double g = cot * F[i];
-                const C psi = B[i];
-                C w;
-                w.x = (R)(g * (double)psi.x);
-                w.y = (R)(-g * (double)psi.y);
-                B[i] = w;
-            }
-            __syncthreads();  // XB shares the eigenvectors' region
-            // the survivor queue overwrote the eigenvectors: load them again
-            for (int i = tid; i < 3 * N2; i += bd) {
-                const int which = i / N2, e = i % N2;
-                const int r = e / N, b = e % N;
-                const int q = which == 0 ? f1 : (which == 1 ? q2 : q3);
-                C *E = which == 0 ? E1 : (which == 1 ? E2 : E3);
-                E[r * N + b] = egvs[((size_t)q * N + b) * N + r];
+                for (int b = 0; b < N; ++b) cfma(acc, e[b * N], t1[b * N]);
+                B[i] = acc;
             }
             __syncthreads();
-            if (tid < N2) {  // A[a][b2b3] = sum_b1 E1[a][b1] W[b1][b2b3]
+            // Psi, delta weights and occupations of the pass's survivors; the forward pass writes F
+            // over T1 of its b1 (dense, read only where the row/column bits are set)
+            C psi;
+            const auto contract = [&](uint32_t qv) {
+                const C *t2 = B + (qv >> 20) * N, *e = E3 + (qv & 0xffffu) % N;
+                psi = czero<C>();
+#pragma unroll
+                for (int c = 0; c < N; ++c) cfma(psi, e[c * N], t2[c]);
+            };
+            if constexpr (!ADJ) {
+                const auto put = [&](uint32_t qv, R f) {
+                    const int idx = (int)(qv & 0xffffu), b1 = idx / N2;
+                    F[b1 * FS + (idx - b1 * N2)] = (double)f;
+                    if (f != (R)0) k3_mark<N>(S, idx);
+                };
+                const auto psisq = [&](uint32_t qv) -> R {
+                    contract(qv);
+                    return psi.x * psi.x + psi.y * psi.y;
+                };
+                if constexpr (sizeof(R) == 8)
+                    k3_survivors<N>(S, P, qstart[pass], qstart[pass + 1], perm, width6, psisq, put);
+                else
+                    k3_survivors_f32<N>(S, P, qstart[pass], qstart[pass + 1], (float)perm, width6, psisq, put);
+                if (pass + 1 < PASSES) __syncthreads();  // B and the next T1 slabs
+            } else {
+                // d L / d|Psi_b|^2 = lam[row(b1)] * nred * dF_b/d|Psi_b|^2 (Gamma += nred * sum F);
+                // d|Psi|^2 / d P[abc] = 2 Re(conj(Psi) E1[a][b1] E2[b][b2] E3[c][b3]), so with
+                // W = G conj(Psi):  Q[abc] = sum_b W_b E1[a][b1] E2[b][b2] E3[c][b3] and
+                // d L / d mwm_t(i,j,k) = 2 Re(phase_t Q[3a1+i][3a2+j][3a3+k]).
+                // with a scattering-matrix cotangent xi_bar (the BTE adjoint): the Xi row terms
+                // 2 F om2/om1 at (q2', b2) and 2 F om3/om1 at (q3', b3) of every equivalent
+                // triplet add xi_bar(row, .) times those factors to the cotangent of F;
+                // R2[b1][b2] and XB[b1][b3] hold xi_bar summed over the equivalent triplets
+                double *XB = (double *)(smem + L.xb);
+                if (a.xi_bar)
+                    for (int e = tid; e < 2 * N2; e += bd) {
+                        const int x = e % N2, b1 = x / N, bb = x % N, row = S.rowid[b1];
+                        double sum = 0.0;
+                        if (row >= 0) {
+                            const double *wr = a.xi_bar + (int64_t)row * ld;
+                            for (int k = 0; k < nred; ++k) {
+                                const int2 pr = S.red[k];
+                                sum += wr[(int64_t)(e < N2 ? pr.x : pr.y) * N + bb];
+                            }
+                        }
+                        if (e < N2) S.R2[x] = sum;
+                        else XB[x] = sum;
+                    }
+                for (int i = tid; i < N3; i += bd) A[i] = czero<C>();
+                enqueue();
+                __syncthreads();
+                const auto psisq = [&](uint32_t qv) -> R {  // F without |Psi|^2, and Psi
+                    contract(qv);
+                    return (R)1;
+                };
+                const auto put = [&](uint32_t qv, R f) {
+                    const int idx = (int)(qv & 0xffffu), b1 = idx / N2, row = S.rowid[b1];
+                    double cot = a.lam[row] * (double)nred;
+                    if (a.xi_bar) {
+                        const int b2 = (idx / N) % N, b3 = idx % N;
+                        cot += 2.0 * (S.om2[b2] * S.R2[b1 * N + b2] + S.om3[b3] * XB[b1 * N + b3]) * S.inv1[b1];
+                    }
+                    const double g = cot * (double)f;
+                    C w;
+                    w.x = (R)(g * (double)psi.x);
+                    w.y = (R)(-g * (double)psi.y);
+                    A[idx] = w;
+                };
+                if constexpr (sizeof(R) == 8)
+                    k3_survivors<N>(S, P, qstart[pass], qstart[pass + 1], perm, width6_again, psisq, put);
+                else
+                    k3_survivors_f32<N>(S, P, qstart[pass], qstart[pass + 1], (float)perm, width6_again, psisq, put);
+            }
+        }
+        if constexpr (ADJ) {
+            __syncthreads();
+            // the queue took the place of two of the eigenvector matrices: load them again
+            for (int i = tid; i < 2 * N2; i += bd) {
+                const int e = i % N2;
+                (i < N2 ? E1 : E2)[e] = egvs[((size_t)(i < N2 ? f1 : q2) * N + e % N) * N + e / N];
+            }
+            __syncthreads();
+            if (tid < N2) {  // B[a][b2b3] = sum_b1 E1[a][b1] W[b1][b2b3]
                 const int bc = tid;
                 C acc[N];
 #pragma unroll
                 for (int x = 0; x < N; ++x) acc[x] = czero<C>();
 #pragma unroll 3
                 for (int b1 = 0; b1 < N; ++b1) {
-                    const C w = B[b1 * N2 + bc];
+                    const C w = A[b1 * N2 + bc];
 #pragma unroll
                     for (int x = 0; x < N; ++x) cfma(acc[x], E1[x * N + b1], w);
                 }
 #pragma unroll
-                for (int x = 0; x < N; ++x) A[x * N2 + bc] = acc[x];
+                for (int x = 0; x < N; ++x) B[x * N2 + bc] = acc[x];
             }
             __syncthreads();
-            if (tid < N2) {  // B[a][b][b3] = sum_b2 E2[b][b2] A[a][b2][b3]
+            if (tid < N2) {  // A[a][b][b3] = sum_b2 E2[b][b2] B[a][b2][b3]
                 const int aa = tid / N, b3 = tid % N;
                 C acc[N];
 #pragma unroll
                 for (int x = 0; x < N; ++x) acc[x] = czero<C>();
 #pragma unroll 3
                 for (int b2 = 0; b2 < N; ++b2) {
-                    const C tv = A[(aa * N + b2) * N + b3];
+                    const C tv = B[(aa * N + b2) * N + b3];
 #pragma unroll
                     for (int x = 0; x < N; ++x) cfma(acc[x], E2[x * N + b2], tv);
                 }
 #pragma unroll
-                for (int x = 0; x < N; ++x) B[(aa * N + x) * N + b3] = acc[x];
+                for (int x = 0; x < N; ++x) A[(aa * N + x) * N + b3] = acc[x];
             }
             __syncthreads();
-            if (tid < N2) {  // A[a][b][c] = sum_b3 E3[c][b3] B[a][b][b3]
+            if (tid < N2) {  // B[a][b][c] = sum_b3 E3[c][b3] A[a][b][b3]
                 const int ab = tid;
                 C acc[N];
 #pragma unroll
                 for (int x = 0; x < N; ++x) acc[x] = czero<C>();
 #pragma unroll 3
                 for (int b3 = 0; b3 < N; ++b3) {
-                    const C tv = B[ab * N + b3];
+                    const C tv = A[ab * N + b3];
 #pragma unroll
                     for (int x = 0; x < N; ++x) cfma(acc[x], E3[x * N + b3], tv);
                 }
 #pragma unroll
-                for (int x = 0; x < N; ++x) A[ab * N + x] = acc[x];
+                for (int x = 0; x < N; ++x) B[ab * N + x] = acc[x];
             }
             // the CTA's slice: doubles on the FP64 path, floats on the mixed path (contiguous
             // slices of n_fc3 * 27 entries of either type)
@@ -549,8 +641,8 @@ __global__ void __launch_bounds__(threads_for(N), min_blocks_for(N, sizeof(R) ==
             // q-triplet exactly one thread touches each entry, and q-triplets are separated by
             // barriers
             const int groups = bd / 27, grp = tid / 27, ijk = tid % 27;
-            const int off = (ijk % 3) * N2 + ((ijk / 3) % 3) * N + ijk / 9;
-            constexpr int PCA = phase_chunk(N, sizeof(C));
+            const int off3 = (ijk % 3) * N2 + ((ijk / 3) % 3) * N + ijk / 9;
+            constexpr int PCA = phase_chunk(N, sizeof(C), ADJ);
             for (int c0 = 0; c0 < fc.n; c0 += PCA) {
                 const int cn = min(PCA, fc.n - c0);
                 __syncthreads();
@@ -559,7 +651,7 @@ __global__ void __launch_bounds__(threads_for(N), min_blocks_for(N, sizeof(R) ==
                 if (grp < groups) {
                     for (int tl = grp; tl < cn; tl += groups) {
                         const int tt = c0 + tl;
-                        const C q = A[fc.abase[tt] + off];
+                        const C q = B[fc.abase[tt] + off3];
                         const C p = ph[tl];
                         const R v = (R)2 * (p.x * q.x - p.y * q.y);
                         if (a.acc_in_smem) {
@@ -587,7 +679,7 @@ __global__ void __launch_bounds__(threads_for(N), min_blocks_for(N, sizeof(R) ==
             continue;
         }
         // ---- R2 = sum over b3, R3 = sum over b2 (into B as doubles), Gamma and Xi ----
-        k3_sums_scatter<N>(S, a, nred);
+        k3_sums_scatter<N, false, FS>(S, a, nred);
     }
     if constexpr (ADJ) {
         if (a.acc_in_smem) {
@@ -706,7 +798,7 @@ int threephonon_threads(int n) { return threads_for(n); }
 
 bool threephonon_plan_fits(int n, int n_fc) {
     // the plan path holds all phase factors (and 4 zero ones after them) in the phase region
-    return n >= 3 && n <= 16 && n_fc + 4 <= phase_chunk(n, (int)sizeof(float2));
+    return n >= 3 && n <= 16 && n_fc + 4 <= phase_chunk(n, (int)sizeof(float2), true);
 }
 
 size_t threephonon_smem_bytes(int n, int precision, int) {

@@ -438,8 +438,15 @@ __global__ void __launch_bounds__(kTcThreads, ADJ ? 3 : 4) k_threephonon_tc(Thre
         if constexpr (ADJ)
             for (int i = tid; i < N3; i += kTcThreads) S.F[i] = 0.0;
         __syncthreads();
+        const auto width6 = [&](int x1, int x2, int x3) { return k3_width6(S, P, x1, x2, x3); };
         if constexpr (!ADJ) {
-            k3_survivors_f32<N, true>(S, P, nq, (float)perm, [&](int idx) -> float { return psq[idx]; });
+            k3_survivors_f32<N>(
+                S, P, 0, nq, (float)perm, width6, [&](uint32_t qv) -> float { return psq[qv & 0xffffu]; },
+                [&](uint32_t qv, float f) {
+                    const int idx = (int)(qv & 0xffffu);
+                    S.Ff[idx] = f;
+                    if (f != 0.f) k3_mark<N>(S, idx);
+                });
             k3_sums_scatter<N, true>(S, a, nred);
         } else {
             // ---- adjoint tail (the SIMT adjoint's algebra, k_threephonon.cu): F without |Psi|^2
@@ -448,7 +455,12 @@ __global__ void __launch_bounds__(kTcThreads, ADJ ? 3 : 4) k_threephonon_tc(Thre
             // equivalent triplets); W = G conj(Psi); Q[abc] = sum_b W_b E1[a,b1] E2[b,b2] E3[c,b3]
             // by three GEMMs against the real-split E^T images (W E3^T over b3, then E2^T over
             // b2, then E1^T over b1); d L / d mwm_t(i,j,k) = 2 Re(phase_t Q[3a1+i][3a2+j][3a3+k]).
-            k3_survivors_f32<N>(S, P, nq, (float)perm, [](int) -> float { return 1.0f; });
+            k3_survivors_f32<N>(S, P, 0, nq, (float)perm, width6, [](uint32_t) -> float { return 1.0f; },
+                                [&](uint32_t qv, float f) {
+                                    const int idx = (int)(qv & 0xffffu);
+                                    S.F[idx] = (double)f;
+                                    if (f != 0.f) k3_mark<N>(S, idx);
+                                });
             __syncthreads();
             double *R2 = S.R2, *XB = S.R3;  // in the |Psi|^2 region, which the adjoint does not use
             if (a.xi_bar) {

@@ -210,6 +210,7 @@ struct tdg_ctx {
     DevBuf<float2> tw32;
     DevBuf<double> d_exp2tab, d_invom;
     DevBuf<float> d_om32, d_sigsq32;
+    DevBuf<float2> d_omhl;
     // isotope scattering: magnitudes of the eigenvector components (first use), screen columns
     DevBuf<double> d_iso_mag;
     DevBuf<float2> d_iso_col;
@@ -679,12 +680,15 @@ extern "C" int tdg_create(tdg_ctx **out, const tdg_problem *p, int device) {
     {
         // per-mode tables of the kernels' screens: omega in FP32 and 1/omega
         std::vector<float> om32(c->omega.size());
+        std::vector<float2> omhl(c->omega.size());
         std::vector<double> invom(c->omega.size());
         for (size_t i = 0; i < c->omega.size(); ++i) {
             om32[i] = (float)c->omega[i];
+            omhl[i] = make_float2(c->omega[i] < kFreqTol ? std::nanf("") : om32[i], (float)(c->omega[i] - (double)om32[i]));
             invom[i] = c->omega[i] > 0.0 ? 1.0 / c->omega[i] : 0.0;
         }
         chk(c->d_om32.upload(om32.data(), om32.size(), s));
+        chk(c->d_omhl.upload(omhl.data(), omhl.size(), s));
         chk(c->d_invom.upload(invom.data(), invom.size(), s));
     }
     chk(c->d_status.alloc(1));
@@ -1003,6 +1007,7 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
     ph.exp2tab = c->d_exp2tab.p;
     ph.inv_omega = c->d_invom.p;
     ph.omega32 = c->d_om32.p;
+    ph.omega_hl = c->d_omhl.p;
 
     std::vector<int32_t> rowidx((size_t)nirr * n, -1), rq1(nr), rb1(nr);
     std::vector<double> w3(nr, 0.0), w4(nr, 0.0), w3q((size_t)nirr * n, 0.0);

@@ -79,6 +79,8 @@ struct PhononDev {
     const double *exp2tab;   // [64] 2^(-j/64), the table of exp_neg
     const double *inv_omega; // [n_full*n] 1/omega, 0 where omega <= 0
     const float *omega32;    // [n_full*n] omega in FP32 (screens)
+    const float2 *omega_hl;  // [n_full*n] the same and the rest in FP32 (omega = h + l to about
+                             // 2^-48); h is NaN where omega < lo_freqtol
     const float *sigsq32;    // [n_irr*n] sigsq in FP32 (screens)
 };
 
