@@ -13,12 +13,21 @@
 // (n^5 complex MACs); for each row b1 the n^3 slice of T1 is contracted with E2, E3, E4 in
 // shared memory (3 n^4 complex MACs per b1): 4 n^5 complex MACs per q-quartet in all.
 // Phases are exact roots of unity from integer lattice vectors, as in the three-phonon
-// kernel. An FP32 pre-screen with a safety margin skips Gaussians that are exactly zero in
-// the reference. Precision R: double (FP64 path: delta weights, occupations and
-// accumulation in FP64 with the reference's window test) or float (mixed path: FP32
-// pretransform and contraction, FP32 delta weights and occupations from FP64 centre
-// differences, FP64 accumulation).
+// kernel.
+//   The delta weights. 13 to 40 % of the mode quadruplets have a Gaussian inside its 8-sigma
+// window with adaptive widths, so an FP32 screen with a safety margin (a Gaussian it drops is
+// exactly zero in the reference) queues them, and full warps contract the last index (E4) for
+// the queued ones alone and form their weights. Precision R: double (FP64 path: weights,
+// occupations and accumulation in FP64 with the reference's window test) or float (mixed
+// path: FP32 pretransform, contraction, weights and occupations; the centre differences from
+// FP32 frequency pairs and the sums over modes in double-float, so that nothing per
+// quadruplet touches the FP64 pipe, which at 2 lanes per clock and SM was 83 % of this
+// kernel's time with FP64 centre differences and conversions).
+//   Measured: perovskite 8^3, 27 x 27 pairs, mixed 4.18 -> 1.75 ms (issue and shared-memory bound); rocksalt 8^3 FP64 1.13 ->
+// 0.79 ms (91 % of the FP64 pipe).
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "dev_common.cuh"
 #include "tdg_internal.cuh"
@@ -28,7 +37,16 @@ namespace tdg {
 namespace {
 
 constexpr double kFourPhononPrefactor = 3.141592653589793 / 96.0;
-constexpr int kPhaseChunk4 = 512;
+// Phase factors at a time: those of one leading atom at once where that costs no CTA (519 of
+// the five-atom perovskite; a second pass reads and writes every output again).
+__host__ __device__ constexpr int phase_chunk4(int n) { return n >= 12 ? 1024 : 512; }
+
+// Modes b1 that go through the second to fourth stage together: few modes leave most of a
+// CTA idle between barriers.
+__host__ __device__ constexpr int b1_batch(int n) { return n <= 6 ? n : (n <= 9 ? 3 : 1); }
+// From 12 modes on a thread owns a column of the second and third stage (n outputs from n
+// inputs in registers), in place; below, n^2 columns are too few and a thread takes one output.
+__host__ __device__ constexpr bool by_column(int n) { return n >= 12; }
 
 template <typename R>
 __device__ __forceinline__ const R *mwm4_ptr(const Fc4Dev &fc);
@@ -64,77 +82,103 @@ __device__ __forceinline__ const float2 *egvs4_ptr<float2>(const PhononDev &ph) 
 }
 
 struct Layout4 {
-    size_t om, be, sg, vel, fo, inv1, wrow, rowid, red, R, occ, E, ph, A, B, total;
+    size_t om, be, sg, fo, inv1, wrow, rowid, red, R, occ, E, ph, Q, w6, A, B, F, total;
 };
 __host__ __device__ inline size_t al16(size_t x) { return (x + 15) & ~size_t(15); }
-__host__ __device__ inline Layout4 make_layout4(int n, int cs) {
+// it6: with the width tables of -it 6.
+__host__ __device__ inline Layout4 make_layout4(int n, int cs, bool it6) {
     Layout4 L;
     size_t o = 0;
-    const size_t n2 = (size_t)n * n, n3 = n2 * n;
+    const size_t n2 = (size_t)n * n, n3 = n2 * n, nb = b1_batch(n), rs = cs / 2;
     L.om = o; o += al16(sizeof(double) * 4 * n);     // omega of q1..q4
     L.be = o; o += al16(sizeof(double) * 4 * n);     // Bose factors of q2..q4 (slot 0 unused)
     L.sg = o; o += al16(sizeof(double) * 4 * n);     // sigsq of q1..q4
-    L.vel = o; o += al16(sizeof(double) * 12 * n);   // velocities of q1..q4
-    L.fo = o; o += al16(sizeof(float) * 8 * n);      // omega and sigsq in FP32
+    L.fo = o; o += al16(sizeof(float) * 12 * n);     // omega, sigsq and omega's rest in FP32
     L.inv1 = o; o += al16(sizeof(double) * n);
     L.wrow = o; o += al16(sizeof(double) * n);
-    L.rowid = o; o += al16(sizeof(int) * n);
+    L.rowid = o; o += al16(sizeof(int) * (n + 4));   // and the queue's length
     L.red = o; o += al16(sizeof(int4) * kMaxRed);
-    L.R = o; o += al16(sizeof(double) * 3 * n);
-    L.occ = o; o += al16(sizeof(double) * (2 * n * n + 4 * n));  // occupation products (see below)
+    L.R = o; o += al16(sizeof(double) * 4 * n * nb);
+    L.occ = o; o += al16(rs * (2 * n2 + 6 * n));     // occupation products (see below)
     L.E = o; o += al16((size_t)cs * 4 * n2);
-    L.ph = o; o += al16((size_t)cs * kPhaseChunk4);
-    const size_t csz = (size_t)cs > sizeof(double) ? (size_t)cs : sizeof(double);
-    L.A = o; o += al16(csz * n3);
-    L.B = o; o += al16(csz * n3);
+    // the phases, then the survivor queue, then the sums over one mode (2 n^2 per b1)
+    const size_t phz = (size_t)cs * phase_chunk4(n), qz = sizeof(uint32_t) * nb * n3, xz = sizeof(double) * 2 * nb * n2;
+    L.ph = L.Q = o;
+    o += al16(phz > qz ? (phz > xz ? phz : xz) : (qz > xz ? qz : xz));
+    L.w6 = o; o += it6 ? al16(sizeof(double) * 6 * n2) : 0;
+    L.A = o; o += al16(cs * nb * n3);
+    L.B = o; o += by_column(n) ? 0 : al16(cs * nb * n3);
+    L.F = o; o += al16(rs * nb * n3);
     L.total = o;
     return L;
 }
 
-__host__ __device__ constexpr int threads4_for(int n) {
-    return n * n * n >= 256 ? 256 : ((n * n * n + 31) / 32) * 32;
+__host__ __device__ constexpr int threads4_for(int n) { return n >= 9 ? 256 : ((n * n * n + 31) / 32) * 32; }
+
+// Resident CTAs the register budget is sized for: what shared memory admits (1 at 15 modes in
+// FP64, 2 at 9 and 12).
+__host__ __device__ constexpr int min_blocks4(int n, bool dbl) {
+    return n <= 3 ? 16 : (n <= 6 ? 3 : (dbl ? (n <= 12 ? 2 : 1) : 3));
 }
 
-// Resident CTAs the register budget is sized for: at n = 15 in FP32 shared memory admits
-// three per SM, which the in-place E1 contraction's registers would otherwise reduce to two.
-__host__ __device__ constexpr int min_blocks4(int n, bool dbl) { return (n == 15 && !dbl) ? 3 : 1; }
+// om1 - (m2 + m3 + m4) from FP32 pairs omega = h + l, as centre_diff_f32 for three.
+__device__ __forceinline__ float centre_diff4_f32(float h1, float l1, float h2, float l2, float h3, float l3, float h4,
+                                                  float l4) {
+    const float s = h2 + h3, bs = s - h2;
+    const float es = (h2 - (s - bs)) + (h3 - bs);
+    const float u = s + h4, bu = u - s;
+    const float eu = (s - (u - bu)) + (h4 - bu);
+    const float d = h1 - u, bd = d - h1;
+    const float ed = (h1 - (d - bd)) + (-u - bd);
+    return d + (ed + ((l1 - l2 - l3 - l4) - (es + eu)));
+}
+
+// The eight Gaussians of get_dirac (scattering_fourphonon.f90:267-327), centred at +-om2 +-om3
+// +-om4: bit j of these is set where the sign is plus. d[j / 2] = g(even j) - g(odd j).
+constexpr uint32_t kPlus2 = 0x59u, kPlus3 = 0x65u, kPlus4 = 0x95u;
 
 template <int N, typename R>
 __global__ void __launch_bounds__(threads4_for(N), min_blocks4(N, sizeof(R) == 8)) k_fourphonon(FourPhArgs a) {
     using C = typename CT<R>::C;
-    constexpr int N2 = N * N, N3 = N2 * N;
+    constexpr int N2 = N * N, N3 = N2 * N, NB = b1_batch(N);
     constexpr int NA = N / 3;
+    constexpr bool DBL = sizeof(R) == 8, COLS = by_column(N);
+    static_assert(N % NB == 0 && (!COLS || NB == 1), "batches of b1");
     extern __shared__ __align__(16) unsigned char smem[];
-    const Layout4 L = make_layout4(N, sizeof(C));
+    const PhononDev &P = a.ph;
+    const int it = P.integrationtype;
+    const Layout4 L = make_layout4(N, sizeof(C), it == 6);
     double *om = (double *)(smem + L.om);   // om[k*N + b], k = 0..3 for q1..q4
     double *be = (double *)(smem + L.be);
     double *sg = (double *)(smem + L.sg);
-    double *vel = (double *)(smem + L.vel); // vel[(k*N + b)*3 + d]
-    float *fo = (float *)(smem + L.fo);     // fo[k*N + b] omega, fo[(4+k)*N + b] sigsq
+    float *fo = (float *)(smem + L.fo);     // fo[k*N + b] omega, fo[(4+k)*N + b] sigsq, fo[(8+k)*N + b] omega's rest
     double *inv1 = (double *)(smem + L.inv1);
     double *wrow = (double *)(smem + L.wrow);
-    int *rowid = (int *)(smem + L.rowid);
+    int *rowid = (int *)(smem + L.rowid), *qlen = rowid + N;
     int4 *red = (int4 *)(smem + L.red);
-    double *Rs = (double *)(smem + L.R);    // R2, R3, R4 of the current b1
+    // the row terms 2 R om / om1 of R2, R3, R4 (sums over the other two modes) for each b1 of
+    // the batch, then R2 itself
+    double *Rs = (double *)(smem + L.R), *R2 = Rs + 3 * N * NB;
     // Occupation products of the quartet, so that the four polynomials of the weights
-    // (scattering_fourphonon.f90:161-186) cost 10 FP64 operations per mode quadruplet
-    // instead of 26: per (b3, b4) P00 = n3 n4 and P11 = (n3+1)(n4+1), with n3 (n4+1) =
-    // P00 + n3 and (n3+1) n4 = P00 + n4; per b2 n2, n2+1, 3 n2, 3 (n2+1). Two tables of n^2
-    // keep three CTAs per SM at n = 15.
-    double *P00 = (double *)(smem + L.occ), *P11 = P00 + N * N;
-    double *N2v = P11 + N * N, *N2p = N2v + N, *N2x3 = N2p + N, *N2px3 = N2x3 + N;
+    // (scattering_fourphonon.f90:161-186) cost 10 operations per mode quadruplet instead of
+    // 26: per (b3, b4) P00 = n3 n4 and P11 = (n3+1)(n4+1), with n3 (n4+1) = P00 + n3 and
+    // (n3+1) n4 = P00 + n4; per b2 n2, n2+1, 3 n2, 3 (n2+1). Formed in FP64, kept in R.
+    R *P00 = (R *)(smem + L.occ), *P11 = P00 + N2;
+    R *N2v = P11 + N2, *N2p = N2v + N, *N2x3 = N2p + N, *N2px3 = N2x3 + N, *N3v = N2px3 + N, *N4v = N3v + N;
     C *E = (C *)(smem + L.E);               // E[k*N2 + r*N + b], k = 0..3
     C *ph = (C *)(smem + L.ph);
+    uint32_t *Q = (uint32_t *)(smem + L.Q); // (b1 b2 b3 b4) within the batch | live Gaussians << 16
+    double *W6d = (double *)(smem + L.w6);  // -it 6: a sixth of the widths of (1,2) (1,3) (1,4) (2,3) (2,4) (3,4)
+    float2 *W6f = (float2 *)(smem + L.w6);  // the same as FP32 pairs (mixed path)
     C *A = (C *)(smem + L.A);
     C *B = (C *)(smem + L.B);
+    R *F = (R *)(smem + L.F);
     const int tid = threadIdx.x, bd = blockDim.x;
     const MeshDev &m = a.mesh;
-    const PhononDev &P = a.ph;
     const Fc4Dev &fc = a.fc;
     const R *mwm = mwm4_ptr<R>(fc);
     const C *egvs = egvs4_ptr<C>(P);
     const int64_t ld = (int64_t)m.n_full * N;
-    const int it = P.integrationtype;
     const float sigfix32 = (float)P.sigma_fixed;
     C *T1 = reinterpret_cast<C *>(a.scratch) + (size_t)blockIdx.x * N3 * N;
 
@@ -161,20 +205,21 @@ __global__ void __launch_bounds__(threads4_for(N), min_blocks4(N, sizeof(R) == 8
         // ---- per-mode scalars, eigenvectors, equivalent quartets ----
         for (int i = tid; i < 4 * N; i += bd) {
             const int k = i / N, b = i % N;
-            const double w = P.omega[(size_t)qf[k] * N + b];
+            const size_t j = (size_t)qf[k] * N + b;
+            const double w = P.omega[j];
+            const float2 hl = P.omega_hl[j];  // NaN below 1e-9 Ha: no window holds it
             om[i] = w;
             sg[i] = P.sigsq[(size_t)qi[k] * N + b];
             be[i] = k > 0 ? P.be[(size_t)qi[k] * N + b] : 0.0;
-            // NaN marks omega < 1e-9 Ha: the skip test then runs in FP32 (double compares and
-            // conversions per mode quadruplet would occupy GB300's narrow FP64 pipe)
-            fo[i] = w < kFreqTolD ? __int_as_float(0x7fc00000) : (float)w;
-            fo[4 * N + i] = (float)sg[i];
-            for (int d = 0; d < 3; ++d) vel[i * 3 + d] = P.vel[((size_t)qf[k] * N + b) * 3 + d];
+            fo[i] = hl.x;
+            fo[4 * N + i] = P.sigsq32[(size_t)qi[k] * N + b];
+            fo[8 * N + i] = hl.y;
             if (k == 0) {
                 inv1[b] = w > 0.0 ? 1.0 / w : 0.0;
                 const int r = a.rows.rowidx[(size_t)rec.q1 * N + b];
                 const bool on = (mask[b >> 5] >> (b & 31)) & 1u;
                 rowid[b] = on ? r : -1;
+                if (!on || r < 0) fo[b] = __int_as_float(0x7fc00000);
                 wrow[b] = r >= 0 ? a.rows.weight4[r] : 0.0;
             }
         }
@@ -184,18 +229,30 @@ __global__ void __launch_bounds__(threads4_for(N), min_blocks4(N, sizeof(R) == 8
             const int r = e / N, b = e % N;
             E[i] = egvs[((size_t)qf[k] * N + b) * N + r];
         }
+        if (it == 6)
+            for (int i = tid; i < 6 * N2; i += bd) {
+                const int which = i / N2, x = (i - which * N2) / N, y = i % N;
+                const int k = which < 3 ? 0 : (which < 5 ? 1 : 2), l = which < 3 ? which + 1 : (which < 5 ? which - 1 : 3);
+                const double w = adaptive_pair(P.vel + ((size_t)qf[k] * N + x) * 3, P.vel + ((size_t)qf[l] * N + y) * 3,
+                                               P.reclat_g) / 6.0;
+                if constexpr (DBL) W6d[i] = w;
+                else W6f[i] = split_df(w);
+            }
+        if (tid == 0) *qlen = 0;
         __syncthreads();  // be[] of q2..q4 is in shared memory
-        for (int i = tid; i < N * N; i += bd) {
+        for (int i = tid; i < N2; i += bd) {
             const double n3 = be[2 * N + i / N], n4 = be[3 * N + i % N];
-            P00[i] = n3 * n4;
-            P11[i] = (n3 + 1.0) * (n4 + 1.0);
+            P00[i] = (R)(n3 * n4);
+            P11[i] = (R)((n3 + 1.0) * (n4 + 1.0));
         }
         for (int b = tid; b < N; b += bd) {
             const double n2 = be[N + b];
-            N2v[b] = n2;
-            N2p[b] = n2 + 1.0;
-            N2x3[b] = 3.0 * n2;
-            N2px3[b] = 3.0 * (n2 + 1.0);
+            N2v[b] = (R)n2;
+            N2p[b] = (R)(n2 + 1.0);
+            N2x3[b] = (R)(3.0 * n2);
+            N2px3[b] = (R)(3.0 * (n2 + 1.0));
+            N3v[b] = (R)be[2 * N + b];
+            N4v[b] = (R)be[3 * N + b];
         }
         int g[3][3];
         {
@@ -213,14 +270,14 @@ __global__ void __launch_bounds__(threads4_for(N), min_blocks4(N, sizeof(R) == 8
         // complex multiply-adds per q-quartet) ----
         constexpr int NA3 = NA * NA * NA;
         for (int a1 = 0; a1 < NA; ++a1) {
-            C *P = T1 + (size_t)(3 * a1) * N3;
+            C *ptf = T1 + (size_t)(3 * a1) * N3;
             const int t0 = fc.blk_ptr[a1 * NA3], t1 = fc.blk_ptr[(a1 + 1) * NA3];
             if (t0 >= t1) {
-                for (int o = tid; o < 3 * N3; o += bd) P[o] = czero<C>();
+                for (int o = tid; o < 3 * N3; o += bd) ptf[o] = czero<C>();
                 continue;
             }
-            for (int c0 = t0; c0 < t1; c0 += kPhaseChunk4) {
-                const int cn = min(kPhaseChunk4, t1 - c0);
+            for (int c0 = t0; c0 < t1; c0 += phase_chunk4(N)) {
+                const int cn = min(phase_chunk4(N), t1 - c0);
                 __syncthreads();
                 // K = sum_d ((g2 lv2 + g3 lv3 + g4 lv4)_d mod N_d) L/N_d mod L, evaluated as
                 // (sum_d (g2 L/N_d) lv2 + ...) mod L: the same integer with one division
@@ -239,7 +296,7 @@ __global__ void __launch_bounds__(threads4_for(N), min_blocks4(N, sizeof(R) == 8
                     const int b = bcd / N2, c = (bcd / N) % N, d = bcd % N;
                     const int blk = ((a1 * NA + b / 3) * NA + c / 3) * NA + d / 3;
                     const int ijkl = i + (b % 3) * 3 + (c % 3) * 9 + (d % 3) * 27;
-                    C acc = c0 == t0 ? czero<C>() : P[o];
+                    C acc = c0 == t0 ? czero<C>() : ptf[o];
                     const int lo = max(fc.blk_ptr[blk], c0), hi = min(fc.blk_ptr[blk + 1], c0 + cn);
                     for (int tt = lo; tt < hi; ++tt) {
                         const R mv = __ldg(mwm + (size_t)tt * 81 + ijkl);
@@ -247,7 +304,7 @@ __global__ void __launch_bounds__(threads4_for(N), min_blocks4(N, sizeof(R) == 8
                         acc.x = fma(mv, p.x, acc.x);
                         acc.y = fma(mv, p.y, acc.y);
                     }
-                    P[o] = acc;
+                    ptf[o] = acc;
                 }
             }
         }
@@ -269,220 +326,252 @@ __global__ void __launch_bounds__(threads4_for(N), min_blocks4(N, sizeof(R) == 8
         }
         __syncthreads();
         const C *E2 = E + N2, *E3 = E + 2 * N2, *E4 = E + 3 * N2;
-        const double *om1 = om, *om2 = om + N, *om3 = om + 2 * N, *om4 = om + 3 * N;
-        const float *fo1 = fo, *fo2 = fo + N, *fo3 = fo + 2 * N, *fo4 = fo + 3 * N;
-        const float *fs1 = fo + 4 * N, *fs2 = fo + 5 * N, *fs3 = fo + 6 * N, *fs4 = fo + 7 * N;
-        for (int b1 = 0; b1 < N; ++b1) {
-            const int row = rowid[b1];
-            if (row < 0) continue;
-            for (int i = tid; i < N3; i += bd) A[i] = T1[(size_t)b1 * N3 + i];
-            __syncthreads();
-            // B[b2][c][d] = sum_b E2[b][b2] A[b][c][d]
-            for (int o = tid; o < N3; o += bd) {
-                const int b2 = o / N2, cd = o % N2;
-                C acc = czero<C>();
-#pragma unroll
-                for (int b = 0; b < N; ++b) cfma(acc, E2[b * N + b2], A[b * N2 + cd]);
-                B[o] = acc;
-            }
-            __syncthreads();
-            // A[b2][b3][d] = sum_c E3[c][b3] B[b2][c][d]
-            for (int o = tid; o < N3; o += bd) {
-                const int b2 = o / N2, b3 = (o / N) % N, d = o % N;
-                C acc = czero<C>();
-#pragma unroll
-                for (int c = 0; c < N; ++c) cfma(acc, E3[c * N + b3], B[(b2 * N + c) * N + d]);
-                A[o] = acc;
-            }
-            __syncthreads();
-            // B[b2][b3][b4] = sum_d E4[d][b4] A[b2][b3][d] = Psi
-            for (int o = tid; o < N3; o += bd) {
-                const int b4 = o % N, b23 = o / N;
-                C acc = czero<C>();
-#pragma unroll
-                for (int d = 0; d < N; ++d) cfma(acc, E4[d * N + b4], A[b23 * N + d]);
-                B[o] = acc;
-            }
-            __syncthreads();
-            // ---- delta weights, occupations (FP64, or FP32 on the mixed path); F in A as doubles ----
-            double *F = (double *)A;
-            const double o1 = om1[b1], w1 = wrow[b1];
-            const double pw4 = kFourPhononPrefactor * w1 * w1;
-            const float f_o1 = fo1[b1];
-            // FP32 F of one live mode quadruplet (mixed precision), the FP64 branch's algebra
-            auto weights_f32 = [&](uint32_t live, int b1x, int b2, int b3, int b4) -> float {
-                float sigma;
-                if (it == 1) {
-                    sigma = sigfix32;
-                } else if (it == 2) {
-                    sigma = sqrtf(fs1[b1x] + fs2[b2] + fs3[b3] + fs4[b4]);
-                } else {
-                    const double *v1 = vel + 3 * b1x, *v2 = vel + 3 * (N + b2), *v3 = vel + 3 * (2 * N + b3),
-                                 *v4 = vel + 3 * (3 * N + b4);
-                    sigma = (float)(adaptive_pair(v1, v2, P.reclat_g) / 6.0 + adaptive_pair(v1, v3, P.reclat_g) / 6.0 +
-                                    adaptive_pair(v1, v4, P.reclat_g) / 6.0 + adaptive_pair(v2, v3, P.reclat_g) / 6.0 +
-                                    adaptive_pair(v2, v4, P.reclat_g) / 6.0 + adaptive_pair(v3, v4, P.reclat_g) / 6.0 +
-                                    P.thresh_sigma);
-                }
-                const float invsig = 1.0f / sigma;
-                const float win8 = 8.0f * sigma, h = 0.5f * invsig * invsig, cg = 0.3989422804014327f * invsig;
-                const double o2 = om2[b2], o3 = om3[b3], o4 = om4[b4];
-                auto gf = [&](double centre) -> float {
-                    const float dx = (float)(o1 - centre);
-                    return fabsf(dx) > win8 ? 0.f : expf(-dx * dx * h) * cg;
-                };
-                const float d0 = ((live & 1u) ? gf(o2 + o3 + o4) : 0.f) - ((live & 2u) ? gf(-o2 - o3 - o4) : 0.f);
-                const float d1 = ((live & 4u) ? gf(-o2 + o3 + o4) : 0.f) - ((live & 8u) ? gf(o2 - o3 - o4) : 0.f);
-                const float d2 = ((live & 16u) ? gf(o2 - o3 + o4) : 0.f) - ((live & 32u) ? gf(-o2 + o3 - o4) : 0.f);
-                const float d3 = ((live & 64u) ? gf(o2 + o3 - o4) : 0.f) - ((live & 128u) ? gf(-o2 - o3 + o4) : 0.f);
-                if (d0 == 0.f && d1 == 0.f && d2 == 0.f && d3 == 0.f) return 0.f;
-                const C psi = B[b2 * N2 + b3 * N + b4];
-                const float ps = fmaf((float)psi.x, (float)psi.x, (float)psi.y * (float)psi.y);
-                const int k34 = b3 * N + b4;
-                const float n2 = (float)N2v[b2], n2p = (float)N2p[b2], p00 = (float)P00[k34], p11 = (float)P11[k34];
-                float acc = 0.f, a1 = 0.f;
-                if (d0 != 0.f) acc = (float)mult0 * fmaf(n2p, p11, -n2 * p00) * d0;
-                if (d1 != 0.f) a1 = fmaf((float)N2x3[b2], p11, -n2p * p00) * d1;
-                if (d2 != 0.f || d3 != 0.f) {
-                    const float q1 = p00 + (float)be[2 * N + b3], q2 = p00 + (float)be[3 * N + b4];
-                    const float n2px3 = (float)N2px3[b2];
-                    if (d2 != 0.f) a1 = fmaf(n2px3, q1, -n2 * q2) * d2 + a1;
-                    if (d3 != 0.f) a1 = fmaf(n2px3, q2, -n2 * q1) * d3 + a1;
-                }
-                return (float)pw4 * ps * fmaf((float)mult1, a1, acc);
-            };
-            for (int o = tid; o < N3; o += bd) {
-                const int b2 = o / N2, b3 = (o / N) % N, b4 = o % N;
-                double fall = 0.0;
-                const float f2 = fo2[b2], f3 = fo3[b3], f4 = fo4[b4];
-                if (f2 == f2 && f3 == f3 && f4 == f4) {  // no omega below 1e-9 Ha
-                    const double o2 = om2[b2], o3 = om3[b3], o4 = om4[b4];
-                    uint32_t live = 0xffu;  // the -it 6 width can cancel in FP32: not screened
-                    if (it != 6) {
-                        float sgf = sigfix32;
-                        if (it == 2) sgf = sqrtf(fs1[b1] + fs2[b2] + fs3[b3] + fs4[b4]);
-                        const float win = 8.0f * sgf * 1.001f + 1e-6f * (f_o1 + f2 + f3 + f4);
-                        const float s234 = f2 + f3 + f4;
-                        live = (fabsf(f_o1 - s234) <= win ? 1u : 0u) | (f_o1 + s234 <= win ? 2u : 0u) |
-                               (fabsf(f_o1 - (-f2 + f3 + f4)) <= win ? 4u : 0u) |
-                               (fabsf(f_o1 - (f2 - f3 - f4)) <= win ? 8u : 0u) |
-                               (fabsf(f_o1 - (f2 - f3 + f4)) <= win ? 16u : 0u) |
-                               (fabsf(f_o1 - (-f2 + f3 - f4)) <= win ? 32u : 0u) |
-                               (fabsf(f_o1 - (f2 + f3 - f4)) <= win ? 64u : 0u) |
-                               (fabsf(f_o1 - (-f2 - f3 + f4)) <= win ? 128u : 0u);
-                    }
-                    if constexpr (sizeof(R) == 4) {
-                        // mixed precision: the weights in FP32 from FP64 centre differences
-                        // rounded to FP32 (as the three-phonon kernels), F in FP32; GB300 issues
-                        // FP64 at 1/64 of the FP32 rate and the FP64 weights held this kernel's
-                        // FP64 pipe at 76 %
-                        if (live) fall = (double)weights_f32(live, b1, b2, b3, b4);
-                        live = 0u;
-                    }
+        for (int b0 = 0; b0 < N; b0 += NB) {
+            if (NB == 1 && rowid[b0] < 0) continue;
+            // ---- screen: a thread per (b1, b2, b3) of the batch; survivors queued (in no fixed
+            // order: each writes its own F) ----
+            for (int i = tid; i < NB * N2; i += bd) {
+                const int b1 = b0 + i / N2, b23 = i % N2, b2 = b23 / N, b3 = b23 - b2 * N;
+                const float f1 = fo[b1], f2 = fo[N + b2], f3 = fo[2 * N + b3];
+                if (!(f1 == f1 && f2 == f2 && f3 == f3)) continue;
+                const float s123 = fo[4 * N + b1] + fo[5 * N + b2] + fo[6 * N + b3];
+                float w123 = 0.f;
+                if (it == 6)
+                    w123 = (float)P.thresh_sigma +
+                           (DBL ? (float)(W6d[b1 * N + b2] + W6d[N2 + b1 * N + b3] + W6d[3 * N2 + b23])
+                                : W6f[b1 * N + b2].x + W6f[N2 + b1 * N + b3].x + W6f[3 * N2 + b23].x);
+                // om1 -+ om2 -+ om3, and the window's absolute margin
+                const float pp = f1 - f2 - f3, mm = f1 + f2 + f3, pm = f1 - f2 + f3, mp = f1 + f2 - f3;
+                for (int b4 = 0; b4 < N; ++b4) {
+                    const float f4 = fo[3 * N + b4];
+                    float s = sigfix32;
+                    if (it == 2) s = sqrt_screen(s123 + fo[7 * N + b4]);
+                    else if (it == 6)
+                        s = w123 + (DBL ? (float)(W6d[2 * N2 + b1 * N + b4] + W6d[4 * N2 + b2 * N + b4] +
+                                                  W6d[5 * N2 + b3 * N + b4])
+                                        : W6f[2 * N2 + b1 * N + b4].x + W6f[4 * N2 + b2 * N + b4].x +
+                                              W6f[5 * N2 + b3 * N + b4].x);
+                    const float win = 8.0f * s * 1.001f + 1e-6f * (mm + f4);
+                    const uint32_t live =
+                        (fabsf(pp - f4) <= win ? 1u : 0u) | (mm + f4 <= win ? 2u : 0u) | (fabsf(mp - f4) <= win ? 4u : 0u) |
+                        (fabsf(pm + f4) <= win ? 8u : 0u) | (fabsf(pm - f4) <= win ? 16u : 0u) |
+                        (fabsf(mp + f4) <= win ? 32u : 0u) | (fabsf(pp + f4) <= win ? 64u : 0u) |
+                        (fabsf(mm - f4) <= win ? 128u : 0u);
                     if (live) {
-                        double sigma, invsig;
-                        if (it == 1) {
-                            sigma = P.sigma_fixed;
-                            invsig = 1.0 / sigma;
-                        } else if (it == 2) {
-                            const double sq = sg[b1] + sg[N + b2] + sg[2 * N + b3] + sg[3 * N + b4];
-                            invsig = rsqrt(sq);
-                            sigma = sq * invsig;
-                        } else {
-                            const double *v1 = vel + 3 * b1, *v2 = vel + 3 * (N + b2), *v3 = vel + 3 * (2 * N + b3),
-                                         *v4 = vel + 3 * (3 * N + b4);
-                            sigma = 0.0;
-                            sigma += adaptive_pair(v1, v2, P.reclat_g) / 6.0;
-                            sigma += adaptive_pair(v1, v3, P.reclat_g) / 6.0;
-                            sigma += adaptive_pair(v1, v4, P.reclat_g) / 6.0;
-                            sigma += adaptive_pair(v2, v3, P.reclat_g) / 6.0;
-                            sigma += adaptive_pair(v2, v4, P.reclat_g) / 6.0;
-                            sigma += adaptive_pair(v3, v4, P.reclat_g) / 6.0;
-                            sigma += P.thresh_sigma;
-                            invsig = 1.0 / sigma;
-                        }
-                        const double win8 = 8.0 * sigma, h = 0.5 * invsig * invsig, cg = kSqrt2PiInv * invsig;
-                        const double *tab = P.exp2tab;
-                        // a centre is formed only for a Gaussian that the screen left live
-                        const double d0 = ((live & 1u) ? gauss(o1 - (o2 + o3 + o4), win8, h, cg, tab) : 0.0) -
-                                          ((live & 2u) ? gauss(o1 - (-o2 - o3 - o4), win8, h, cg, tab) : 0.0);
-                        const double d1 = ((live & 4u) ? gauss(o1 - (-o2 + o3 + o4), win8, h, cg, tab) : 0.0) -
-                                          ((live & 8u) ? gauss(o1 - (o2 - o3 - o4), win8, h, cg, tab) : 0.0);
-                        const double d2 = ((live & 16u) ? gauss(o1 - (o2 - o3 + o4), win8, h, cg, tab) : 0.0) -
-                                          ((live & 32u) ? gauss(o1 - (-o2 + o3 - o4), win8, h, cg, tab) : 0.0);
-                        const double d3 = ((live & 64u) ? gauss(o1 - (o2 + o3 - o4), win8, h, cg, tab) : 0.0) -
-                                          ((live & 128u) ? gauss(o1 - (-o2 - o3 + o4), win8, h, cg, tab) : 0.0);
-                        if (nonzero(d0) || nonzero(d1) || nonzero(d2) || nonzero(d3)) {
-                            const C psi = B[o];
-                            double ps;
-                            if constexpr (sizeof(R) == 4) {
-                                ps = (double)fmaf(psi.x, psi.x, psi.y * psi.y);  // |Psi|^2 of an FP32 Psi
-                            } else {
-                                ps = psi.x * psi.x + psi.y * psi.y;
-                            }
-                            // plf0 = (n2+1)(n3+1)(n4+1) - n2 n3 n4, plf1 = 3 n2 (n3+1)(n4+1) - (n2+1) n3 n4,
-                            // plf2 = 3 n3 (n2+1)(n4+1) - (n3+1) n2 n4, plf3 = 3 n4 (n2+1)(n3+1) - (n4+1) n2 n3
-                            const int k34 = b3 * N + b4;
-                            const double n2 = N2v[b2], n2p = N2p[b2], p00 = P00[k34], p11 = P11[k34];
-                            double acc = 0.0;
-                            if (nonzero(d0)) acc = mult0 * fma(n2p, p11, -n2 * p00) * d0;
-                            double a1 = 0.0;
-                            if (nonzero(d1)) a1 = fma(N2x3[b2], p11, -n2p * p00) * d1;
-                            if (nonzero(d2) || nonzero(d3)) {
-                                const double q1 = p00 + be[2 * N + b3], q2 = p00 + be[3 * N + b4];
-                                if (nonzero(d2)) a1 = fma(N2px3[b2], q1, -n2 * q2) * d2 + a1;
-                                if (nonzero(d3)) a1 = fma(N2px3[b2], q2, -n2 * q1) * d3 + a1;
-                            }
-                            fall = pw4 * ps * fma(mult1, a1, acc);
-                        }
+                        const unsigned on = __activemask();
+                        const int lane = tid & 31, lead = __ffs(on) - 1;
+                        int at = 0;
+                        if (lane == lead) at = atomicAdd(qlen, __popc(on));
+                        at = __shfl_sync(on, at, lead) + __popc(on & ((1u << lane) - 1u));
+                        Q[at] = (uint32_t)(i * N + b4) | (live << 16);
                     }
                 }
-                F[o] = fall;
             }
-            __syncthreads();
-            // R2[b2] = sum_{b3,b4} F, R3[b3] = sum_{b2,b4} F, R4[b4] = sum_{b2,b3} F
-            for (int e = tid; e < 3 * N; e += bd) {
-                const int which = e / N, b = e % N;
-                double sum = 0.0;
-                for (int x = 0; x < N; ++x)
-                    for (int y = 0; y < N; ++y) {
-                        const int idx = which == 0 ? (b * N + x) * N + y : (which == 1 ? (x * N + b) * N + y : (x * N + y) * N + b);
-                        const double f = F[idx];
-                        if (nonzero(f)) sum += f;
+            for (int i = tid; i < NB * N3; i += bd) F[i] = (R)0;
+            // ---- second stage [b2][c][d] = sum_b E2[b][b2] T1[b1][b][c][d], third
+            // [b2][b3][d] = sum_c E3[c][b3] [b2][c][d]; the fourth is the survivors' ----
+            const C *T3;
+            if constexpr (COLS) {
+                for (int cd = tid; cd < N2; cd += bd) {
+                    const C *t1 = T1 + (size_t)b0 * N3 + cd;
+                    C acc[N];
+#pragma unroll
+                    for (int x = 0; x < N; ++x) acc[x] = czero<C>();
+#pragma unroll 3
+                    for (int b = 0; b < N; ++b) {
+                        const C v = t1[b * N2];
+#pragma unroll
+                        for (int x = 0; x < N; ++x) cfma(acc[x], E2[b * N + x], v);
                     }
-                Rs[e] = sum;
+#pragma unroll
+                    for (int x = 0; x < N; ++x) A[x * N2 + cd] = acc[x];
+                }
+                __syncthreads();
+                for (int i = tid; i < N2; i += bd) {
+                    const int b2 = i / N, d = i - b2 * N;
+                    C *col = A + b2 * N2 + d;
+                    C acc[N];
+#pragma unroll
+                    for (int x = 0; x < N; ++x) acc[x] = czero<C>();
+#pragma unroll 3
+                    for (int c = 0; c < N; ++c) {
+                        const C v = col[c * N];
+#pragma unroll
+                        for (int x = 0; x < N; ++x) cfma(acc[x], E3[c * N + x], v);
+                    }
+#pragma unroll
+                    for (int x = 0; x < N; ++x) col[x * N] = acc[x];
+                }
+                T3 = A;
+            } else {
+                for (int i = tid; i < NB * N3; i += bd) B[i] = T1[(size_t)b0 * N3 + i];
+                __syncthreads();
+                for (int i = tid; i < NB * N3; i += bd) {
+                    const int b1 = i / N3, o = i - b1 * N3, b2 = o / N2, cd = o - b2 * N2;
+                    C acc = czero<C>();
+#pragma unroll
+                    for (int b = 0; b < N; ++b) cfma(acc, E2[b * N + b2], B[b1 * N3 + b * N2 + cd]);
+                    A[i] = acc;
+                }
+                __syncthreads();
+                for (int i = tid; i < NB * N3; i += bd) {
+                    const int k = i / N2, b3 = (i - k * N2) / N, d = i % N;  // k = (b1, b2)
+                    C acc = czero<C>();
+#pragma unroll
+                    for (int c = 0; c < N; ++c) cfma(acc, E3[c * N + b3], A[k * N2 + c * N + d]);
+                    B[i] = acc;
+                }
+                T3 = B;
             }
             __syncthreads();
-            if (tid == 0) {
+            // ---- survivors: weights, Psi, F ----
+            const int nq = *qlen;
+            for (int s = tid; s < nq; s += bd) {
+                const uint32_t qv = Q[s];
+                const int o = (int)(qv & 0xffffu);
+                uint32_t live = qv >> 16;
+                const int b1 = b0 + o / N3, b2 = (o / N2) % N, b3 = (o / N) % N, b4 = o % N;
+                R sigma, invsig, dd[4] = {(R)0, (R)0, (R)0, (R)0};
+                if constexpr (DBL) {
+                    if (it == 1) {
+                        sigma = P.sigma_fixed;
+                        invsig = 1.0 / sigma;
+                    } else if (it == 2) {
+                        const double sq = sg[b1] + sg[N + b2] + sg[2 * N + b3] + sg[3 * N + b4];
+                        invsig = rsqrt(sq);
+                        sigma = sq * invsig;
+                    } else {
+                        sigma = W6d[b1 * N + b2];
+                        sigma += W6d[N2 + b1 * N + b3];
+                        sigma += W6d[2 * N2 + b1 * N + b4];
+                        sigma += W6d[3 * N2 + b2 * N + b3];
+                        sigma += W6d[4 * N2 + b2 * N + b4];
+                        sigma += W6d[5 * N2 + b3 * N + b4];
+                        sigma += P.thresh_sigma;
+                        invsig = 1.0 / sigma;
+                    }
+                } else {
+                    if (it == 1) {
+                        sigma = sigfix32;
+                    } else if (it == 2) {
+                        sigma = sqrtf(fo[4 * N + b1] + fo[5 * N + b2] + fo[6 * N + b3] + fo[7 * N + b4]);
+                    } else {
+                        float2 w = df_merge(W6f[b1 * N + b2], W6f[N2 + b1 * N + b3]);
+                        w = df_merge(w, W6f[2 * N2 + b1 * N + b4]);
+                        w = df_merge(w, W6f[3 * N2 + b2 * N + b3]);
+                        w = df_merge(w, W6f[4 * N2 + b2 * N + b4]);
+                        w = df_merge(w, W6f[5 * N2 + b3 * N + b4]);
+                        sigma = w.x + (w.y + (float)P.thresh_sigma);
+                    }
+                    invsig = 1.0f / sigma;
+                }
+                const R win8 = (R)8 * sigma, h = (R)0.5 * invsig * invsig, cg = (R)kSqrt2PiInv * invsig;
+                for (; live; live &= live - 1) {
+                    const int j = __ffs(live) - 1;
+                    const bool p2 = (kPlus2 >> j) & 1u, p3 = (kPlus3 >> j) & 1u, p4 = (kPlus4 >> j) & 1u;
+                    R gj;
+                    if constexpr (DBL) {
+                        const double m2 = p2 ? om[N + b2] : -om[N + b2], m3 = p3 ? om[2 * N + b3] : -om[2 * N + b3],
+                                     m4 = p4 ? om[3 * N + b4] : -om[3 * N + b4];
+                        gj = gauss(om[b1] - (m2 + m3 + m4), win8, h, cg, P.exp2tab);
+                    } else {
+                        const float s2 = p2 ? 1.f : -1.f, s3 = p3 ? 1.f : -1.f, s4 = p4 ? 1.f : -1.f;
+                        const float dx =
+                            centre_diff4_f32(fo[b1], fo[8 * N + b1], s2 * fo[N + b2], s2 * fo[9 * N + b2], s3 * fo[2 * N + b3],
+                                             s3 * fo[10 * N + b3], s4 * fo[3 * N + b4], s4 * fo[11 * N + b4]);
+                        gj = fabsf(dx) > win8 ? 0.f : expf(-dx * dx * h) * cg;
+                    }
+                    const R sj = (j & 1) ? -gj : gj;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) dd[k] += (j >> 1) == k ? sj : (R)0;
+                }
+                if (dd[0] != (R)0 || dd[1] != (R)0 || dd[2] != (R)0 || dd[3] != (R)0) {
+                    C psi = czero<C>();
+                    const C *t3 = T3 + (o - b4);
+#pragma unroll
+                    for (int d = 0; d < N; ++d) cfma(psi, E4[d * N + b4], t3[d]);
+                    const R ps = DBL ? psi.x * psi.x + psi.y * psi.y : fma(psi.x, psi.x, psi.y * psi.y);
+                    // plf0 = (n2+1)(n3+1)(n4+1) - n2 n3 n4, plf1 = 3 n2 (n3+1)(n4+1) - (n2+1) n3 n4,
+                    // plf2 = 3 n3 (n2+1)(n4+1) - (n3+1) n2 n4, plf3 = 3 n4 (n2+1)(n3+1) - (n4+1) n2 n3
+                    const int k34 = b3 * N + b4;
+                    const R n2 = N2v[b2], n2p = N2p[b2], p00 = P00[k34], p11 = P11[k34];
+                    const R q1 = p00 + N3v[b3], q2x = p00 + N4v[b4];
+                    const R acc = (R)mult0 * fma(n2p, p11, -n2 * p00) * dd[0];
+                    R a1 = fma(N2x3[b2], p11, -n2p * p00) * dd[1];
+                    a1 = fma(fma(N2px3[b2], q1, -n2 * q2x), dd[2], a1);
+                    a1 = fma(fma(N2px3[b2], q2x, -n2 * q1), dd[3], a1);
+                    const double w1 = wrow[b1];
+                    F[o] = (R)(kFourPhononPrefactor * w1 * w1) * ps * fma((R)mult1, a1, acc);
+                }
+            }
+            __syncthreads();
+            // ---- sums over b4 (X) and over b3 (Y), in the queue's place, then R2, R3, R4, Gamma and
+            // the row terms; the mixed path in double-float ----
+            using Sum = typename std::conditional<DBL, double, float2>::type;
+            Sum *X = (Sum *)Q, *Y = X + NB * N2;
+            const auto clear = [](Sum &v) {
+                if constexpr (DBL) v = 0.0;
+                else v = make_float2(0.f, 0.f);
+            };
+            const auto add = [](Sum &v, R f) {
+                if constexpr (DBL) v += f;
+                else df_acc(v, f);
+            };
+            const auto merge = [](Sum &v, Sum w) {
+                if constexpr (DBL) v += w;
+                else v = df_merge(v, w);
+            };
+            if (tid == 0) *qlen = 0;
+            for (int i = tid; i < 2 * NB * N2; i += bd) {
+                const int e = i < NB * N2 ? i : i - NB * N2, k = e / N, x = e - k * N;  // k = (b1, b2); x = b3 or b4
+                const R *f = i < NB * N2 ? F + e * N : F + k * N2 + x;
+                const int step = i < NB * N2 ? 1 : N;
+                Sum v;
+                clear(v);
+#pragma unroll
+                for (int y = 0; y < N; ++y) add(v, f[y * step]);
+                (i < NB * N2 ? X : Y)[e] = v;
+            }
+            __syncthreads();
+            // R2[b2] = sum_b3 X, R3[b3] = sum_b2 X, R4[b4] = sum_b2 Y
+            for (int i = tid; i < 3 * N * NB; i += bd) {
+                const int b1 = i / (3 * N), e = i - b1 * 3 * N, which = e / N, b = e - which * N;
+                const Sum *x = (which == 2 ? Y : X) + b1 * N2;
+                Sum v;
+                clear(v);
+#pragma unroll
+                for (int k = 0; k < N; ++k) merge(v, which == 0 ? x[b * N + k] : x[k * N + b]);
+                double r;
+                if constexpr (DBL) r = v;
+                else r = (double)v.x + (double)v.y;
+                if (which == 0) R2[b1 * N + b] = r;
+                Rs[i] = nonzero(r) && rowid[b0 + b1] >= 0 ? 2.0 * r * om[(which + 1) * N + b] * inv1[b0 + b1] : 0.0;
+            }
+            __syncthreads();
+            for (int b1 = tid; b1 < NB; b1 += bd) {
+                const int row = rowid[b0 + b1];
                 double gsum = 0.0;
-                for (int b2 = 0; b2 < N; ++b2) gsum += Rs[b2];
-                if (nonzero(gsum)) atomicAdd(a.gamma + row, (double)nred * gsum);
+                for (int b2 = 0; b2 < N; ++b2) gsum += R2[b1 * N + b2];
+                if (row >= 0 && nonzero(gsum)) atomicAdd(a.gamma + row, (double)nred * gsum);
             }
-            // the row terms 2 R om / om1, formed once for all equivalent quartets (after Gamma
-            // has read R2)
-            __syncthreads();
-            for (int e = tid; e < 3 * N; e += bd) {
-                const double v = Rs[e];
-                Rs[e] = nonzero(v) ? 2.0 * v * om[(e / N + 1) * N + e % N] * inv1[b1] : 0.0;
-            }
-            __syncthreads();
-            for (int i = tid; i < 3 * N * nred; i += bd) {
-                const int r = i / (3 * N), e = i % (3 * N);
-                const int which = e / N, b = e % N;
-                const double v = Rs[e];
+            for (int i = tid; i < 3 * N * NB * nred; i += bd) {
+                const int r = i / (3 * N * NB), k = i - r * 3 * N * NB, b1 = k / (3 * N), e = k - b1 * 3 * N;
+                const int which = e / N, b = e - which * N, row = rowid[b0 + b1];
+                const double v = Rs[k];
                 if (!nonzero(v)) continue;
                 const int4 pr = red[r];
                 const int qp = which == 0 ? pr.x : (which == 1 ? pr.y : pr.z);
                 atomicAdd(a.od + row * ld + (int64_t)qp * N + b, v);
             }
-            __syncthreads();
+            // (the next batch's barriers separate its X and Rs from these reads; its queue does
+            // not start before X is read: the barrier above)
         }
     }
 }
 
 template <int N, typename R>
-int grid_n(int n_sm, int n_quart) {
-    const Layout4 L = make_layout4(N, sizeof(typename CT<R>::C));
+int grid_n(int n_sm, int n_quart, bool it6) {
+    const Layout4 L = make_layout4(N, sizeof(typename CT<R>::C), it6);
     const int per_sm = resident_ctas((const void *)k_fourphonon<N, R>, threads4_for(N), L.total, nullptr, nullptr);
     if (per_sm < 1) return 0;
     int grid = n_sm * per_sm;
@@ -492,19 +581,19 @@ int grid_n(int n_sm, int n_quart) {
 
 template <int N, typename R>
 cudaError_t launch_n4(const FourPhArgs &a, int grid, cudaStream_t s) {
-    const Layout4 L = make_layout4(N, sizeof(typename CT<R>::C));
+    const Layout4 L = make_layout4(N, sizeof(typename CT<R>::C), a.ph.integrationtype == 6);
     k_fourphonon<N, R><<<grid, threads4_for(N), L.total, s>>>(a);
     return cudaGetLastError();
 }
 
 template <typename R>
-int grid_prec(int n, int n_sm, int n_quart) {
+int grid_prec(int n, int n_sm, int n_quart, bool it6) {
     switch (n) {
-        case 3: return grid_n<3, R>(n_sm, n_quart);
-        case 6: return grid_n<6, R>(n_sm, n_quart);
-        case 9: return grid_n<9, R>(n_sm, n_quart);
-        case 12: return grid_n<12, R>(n_sm, n_quart);
-        case 15: return grid_n<15, R>(n_sm, n_quart);
+        case 3: return grid_n<3, R>(n_sm, n_quart, it6);
+        case 6: return grid_n<6, R>(n_sm, n_quart, it6);
+        case 9: return grid_n<9, R>(n_sm, n_quart, it6);
+        case 12: return grid_n<12, R>(n_sm, n_quart, it6);
+        case 15: return grid_n<15, R>(n_sm, n_quart, it6);
         default: return 0;
     }
 }
@@ -523,9 +612,10 @@ cudaError_t launch_prec4(const FourPhArgs &a, int grid, cudaStream_t s) {
 
 }  // namespace
 
-int fourphonon_grid(int n, int precision, int n_sm, int n_quart) {
+int fourphonon_grid(int n, int precision, int integrationtype, int n_sm, int n_quart) {
+    const bool it6 = integrationtype == 6;
     if (n_quart <= 0) return 0;
-    return precision == 0 ? grid_prec<double>(n, n_sm, n_quart) : grid_prec<float>(n, n_sm, n_quart);
+    return precision == 0 ? grid_prec<double>(n, n_sm, n_quart, it6) : grid_prec<float>(n, n_sm, n_quart, it6);
 }
 
 size_t fourphonon_scratch_bytes(int n, int precision, int grid) {

@@ -1544,7 +1544,7 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
         if (st) return st;
         nquart = tot[0];
         nred4 = tot[1];
-        const int grid4 = fourphonon_grid(n, o->precision, c->n_sm, nquart);
+        const int grid4 = fourphonon_grid(n, o->precision, o->integrationtype, c->n_sm, nquart);
         if (nquart > 0 && grid4 < 1) return set_error(kErrDevice, "four-phonon kernel configuration failed");
         chk(c->d_quart.alloc(nquart));
         chk(c->d_red4.alloc(nred4));

@@ -240,7 +240,7 @@ struct FourPhArgs {
 };
 // Grid of the four-phonon kernel and the device scratch it needs (bytes); 0 when the mode
 // count is not supported.
-int fourphonon_grid(int n, int precision, int n_sm, int n_quart);
+int fourphonon_grid(int n, int precision, int integrationtype, int n_sm, int n_quart);
 size_t fourphonon_scratch_bytes(int n, int precision, int grid);
 cudaError_t launch_fourphonon(const FourPhArgs &a, int precision, int grid, cudaStream_t s);
 
