@@ -266,9 +266,9 @@ class QLists:
         rb1 = np.zeros(cap, np.int32)
         p3 = np.zeros(cap + 1, np.int64)
         p4 = np.zeros(cap + 1, np.int64)
-        l3 = np.zeros(cap * np3 if opts.thirdorder else 1, np.int32)
-        l4a = np.zeros(cap * np4 if opts.fourthorder else 1, np.int32)
-        l4b = np.zeros(cap * np4 if opts.fourthorder else 1, np.int32)
+        l3 = np.empty(cap * np3 if opts.thirdorder else 1, np.int32)
+        l4a = np.empty(cap * np4 if opts.fourthorder else 1, np.int32)
+        l4b = np.empty(cap * np4 if opts.fourthorder else 1, np.int32)
         nr = C.c_int32(0)
         ps = prob.struct()
         os_ = opts.struct(prob.grid)
@@ -278,10 +278,10 @@ class QLists:
         n = nr.value
         return cls(rq1[:n].copy(), rb1[:n].copy(),
                    p3[: n + 1].copy() if opts.thirdorder else None,
-                   l3[: n * np3].copy() if opts.thirdorder else None,
+                   l3[: n * np3] if opts.thirdorder else None,
                    p4[: n + 1].copy() if opts.fourthorder else None,
-                   l4a[: n * np4].copy() if opts.fourthorder else None,
-                   l4b[: n * np4].copy() if opts.fourthorder else None)
+                   l4a[: n * np4] if opts.fourthorder else None,
+                   l4b[: n * np4] if opts.fourthorder else None)
 
     @classmethod
     def per_irreducible(cls, prob: Problem, samples3: dict | None = None, samples4: dict | None = None) -> "QLists":
