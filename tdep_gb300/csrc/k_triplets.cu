@@ -52,45 +52,95 @@ __device__ __forceinline__ int fourth_index(const MeshDev &m, int f1, int q2, in
     return (i4 * m.grid[1] + j4) * m.grid[2] + k4;
 }
 
-// Returns -1 when the triplet is reducible, else the number of distinct equivalent
-// triplets; when out != nullptr they are written in operation order (unsorted pairs).
-__device__ int triplet_images(const MeshDev &m, int q1, int q2, int q3, int2 *out) {
+// Images (x, y) of (q2, q3) under operation j of q1's little group; false where one of them
+// is off the mesh.
+__device__ __forceinline__ bool triplet_image(const MeshDev &m, const int32_t *ops, int j, int q2, int q3, int &x,
+                                              int &y) {
+    const int32_t *rot = m.rot + (size_t)ops[j] * m.n_full;
+    x = rot[q2];
+    y = rot[q3];
+    return x >= 0 && y >= 0;
+}
+
+// triplet_is_irreducible's first test: no image has its smaller point above q2.
+__device__ __forceinline__ bool triplet_accepted(const MeshDev &m, int q1, int q2, int q3) {
     const int nop = m.irr_nop[q1];
     const int32_t *ops = m.irr_ops + (size_t)q1 * m.n_op;
-    int a[kMaxOps], b[kMaxOps];
-    bool isred = false;
     for (int j = 0; j < nop; ++j) {
-        const int o = ops[j];
-        const int x = m.rot[(size_t)o * m.n_full + q2];
-        const int y = m.rot[(size_t)o * m.n_full + q3];
-        if (x < 0 || y < 0) {
-            a[j] = -1;
-            b[j] = -1;
-            continue;
-        }
-        a[j] = x;
-        b[j] = y;
-        if (min(x, y) > q2) isred = true;
+        int x, y;
+        if (triplet_image(m, ops, j, q2, q3, x, y) && min(x, y) > q2) return false;
     }
-    if (isred) return -1;
-    for (int j = 0; j < nop; ++j)
-        if (a[j] < 0) {
-            a[j] = q2;
-            b[j] = q3;
+    return true;
+}
+
+// The distinct equivalent triplets of an accepted one: an operation counts unless a later one
+// gives the same pair (in either order); operations off the mesh give (q2, q3). Returns their
+// number; when out != nullptr they are written in operation order (unsorted pairs).
+// Up to kLaneOps operations one thread compares all pairs of them (triplet_images); larger
+// little groups take a warp, 32 operations at a time (triplet_images_warp): at the zone
+// centre of a cubic mesh one thread with 48 operations in local memory held the kernel for
+// 50 us whatever the mesh.
+constexpr int kLaneOps = 4;
+
+__device__ __forceinline__ int triplet_images(const MeshDev &m, int q1, int q2, int q3, int2 *out) {
+    const int nop = m.irr_nop[q1];
+    const int32_t *ops = m.irr_ops + (size_t)q1 * m.n_op;
+    int x[kLaneOps], y[kLaneOps], cnt = 0;
+#pragma unroll
+    for (int j = 0; j < kLaneOps; ++j)
+        if (j >= nop || !triplet_image(m, ops, j, q2, q3, x[j], y[j])) {
+            x[j] = q2;
+            y[j] = q3;
         }
-    int cnt = 0;
-    for (int j = 0; j < nop; ++j) {
-        const int lo = min(a[j], b[j]), hi = max(a[j], b[j]);
-        bool uniq = true;
-        for (int k = j + 1; k < nop; ++k)
-            if (min(a[k], b[k]) == lo && max(a[k], b[k]) == hi) {
-                uniq = false;
-                break;
-            }
+#pragma unroll
+    for (int j = 0; j < kLaneOps; ++j) {
+        bool uniq = j < nop;
+#pragma unroll
+        for (int k = j + 1; k < kLaneOps; ++k)
+            if (k < nop && ((x[k] == x[j] && y[k] == y[j]) || (x[k] == y[j] && y[k] == x[j]))) uniq = false;
         if (uniq) {
-            if (out) out[cnt] = make_int2(a[j], b[j]);
+            if (out) out[cnt] = make_int2(x[j], y[j]);
             ++cnt;
         }
+    }
+    return cnt;
+}
+
+// All lanes of a full warp with the same arguments.
+__device__ int triplet_images_warp(const MeshDev &m, int q1, int q2, int q3, int2 *out) {
+    constexpr int kChunks = kMaxOps / 32;
+    const int nop = m.irr_nop[q1], lane = threadIdx.x & 31, nch = (nop + 31) / 32;
+    const int32_t *ops = m.irr_ops + (size_t)q1 * m.n_op;
+    unsigned long long key[kChunks];
+    int2 img[kChunks];
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c) {
+        const int j = c * 32 + lane;
+        int x = q2, y = q3;
+        if (j < nop && !triplet_image(m, ops, j, q2, q3, x, y)) {
+            x = q2;
+            y = q3;
+        }
+        img[c] = make_int2(x, y);
+        // no pair has this key: lanes past the last operation match one another only
+        key[c] = j < nop ? ((unsigned long long)(unsigned)min(x, y) << 32) | (unsigned)max(x, y) : ~0ULL;
+    }
+    int cnt = 0;
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c) {
+        if (c >= nch) break;
+        const unsigned same = __match_any_sync(0xffffffffu, key[c]);
+        bool uniq = c * 32 + lane < nop && (same >> lane) == 1u;  // the last of them in this chunk
+#pragma unroll
+        for (int d = c + 1; d < kChunks; ++d) {
+            if (d >= nch) break;
+            const int left = min(32, nop - d * 32);
+            for (int l = 0; l < left; ++l)
+                if (__shfl_sync(0xffffffffu, key[d], l) == key[c]) uniq = false;
+        }
+        const unsigned in = __ballot_sync(0xffffffffu, uniq);
+        if (out && uniq) out[cnt + __popc(in & ((1u << lane) - 1u))] = img[c];
+        cnt += __popc(in);
     }
     return cnt;
 }
@@ -157,42 +207,58 @@ __device__ int quartet_images(const MeshDev &m, int q1, int q2, int q3, int q4, 
 
 __global__ void k_triplet_count(MeshDev m, const int4 *cand, int32_t n_cand, int32_t *n_trip, int32_t *n_red,
                                 int32_t *status) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n_cand) return;
-    const int q1 = cand[c].x, q2 = cand[c].y;
-    int nt = 0, nr = 0;
-    if (q1 < 0 || q1 >= m.n_irr || q2 < 0 || q2 >= m.n_full || m.irr_nop[q1] > kMaxOps) {
-        atomicCAS(status, kDevOk, kDevBadIndex);
-    } else {
-        const int q3 = third_index(m, m.irr_full[q1], q2);
-        if (q3 >= q2) {
-            const int k = triplet_images(m, q1, q2, q3, nullptr);
-            if (k >= 0) {
-                nt = 1;
-                nr = k;
-            }
+    const int c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    int q1 = 0, q2 = 0, q3 = 0, nr = 0;
+    bool on = false, warp = false;
+    if (c < n_cand) {
+        q1 = cand[c].x;
+        q2 = cand[c].y;
+        if (q1 < 0 || q1 >= m.n_irr || q2 < 0 || q2 >= m.n_full || m.irr_nop[q1] > kMaxOps) {
+            atomicCAS(status, kDevOk, kDevBadIndex);
+        } else {
+            q3 = third_index(m, m.irr_full[q1], q2);
+            on = q3 >= q2 && triplet_accepted(m, q1, q2, q3);
+            warp = on && m.irr_nop[q1] > kLaneOps;
+            if (on && !warp) nr = triplet_images(m, q1, q2, q3, nullptr);
         }
     }
-    n_trip[c] = nt;
+    for (unsigned left = __ballot_sync(0xffffffffu, warp); left; left &= left - 1) {
+        const int l = __ffs(left) - 1;
+        const int k = triplet_images_warp(m, __shfl_sync(0xffffffffu, q1, l), __shfl_sync(0xffffffffu, q2, l),
+                                          __shfl_sync(0xffffffffu, q3, l), nullptr);
+        if (lane == l) nr = k;
+    }
+    if (c >= n_cand) return;
+    n_trip[c] = on ? 1 : 0;
     n_red[c] = nr;
 }
 
 __global__ void k_triplet_fill(MeshDev m, const int4 *cand, int32_t n_cand, const int32_t *trip_off,
                                const int32_t *red_off, TripletRec *trip, int2 *red) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n_cand) return;
-    if (trip_off[c + 1] == trip_off[c]) return;
-    const int q1 = cand[c].x, q2 = cand[c].y;
-    const int q3 = third_index(m, m.irr_full[q1], q2);
-    const int k = triplet_images(m, q1, q2, q3, red + red_off[c]);
-    TripletRec r;
-    r.q1 = q1;
-    r.q2 = q2;
-    r.q3 = q3;
-    r.cand = cand[c].z;
-    r.red_off = red_off[c];
-    r.red_cnt = k;
-    trip[trip_off[c]] = r;
+    int q1 = 0, q2 = 0, q3 = 0, at = 0;
+    bool warp = false;
+    if (c < n_cand && trip_off[c + 1] != trip_off[c]) {
+        q1 = cand[c].x;
+        q2 = cand[c].y;
+        q3 = third_index(m, m.irr_full[q1], q2);
+        at = red_off[c];
+        TripletRec r;
+        r.q1 = q1;
+        r.q2 = q2;
+        r.q3 = q3;
+        r.cand = cand[c].z;
+        r.red_off = at;
+        r.red_cnt = red_off[c + 1] - at;
+        trip[trip_off[c]] = r;
+        warp = m.irr_nop[q1] > kLaneOps;
+        if (!warp) triplet_images(m, q1, q2, q3, red + at);
+    }
+    for (unsigned left = __ballot_sync(0xffffffffu, warp); left; left &= left - 1) {
+        const int l = __ffs(left) - 1;
+        triplet_images_warp(m, __shfl_sync(0xffffffffu, q1, l), __shfl_sync(0xffffffffu, q2, l),
+                            __shfl_sync(0xffffffffu, q3, l), red + __shfl_sync(0xffffffffu, at, l));
+    }
 }
 
 __global__ void k_quartet_count(MeshDev m, const int4 *cand, int32_t n_cand, int32_t *n_q, int32_t *n_red,
@@ -238,60 +304,96 @@ __global__ void k_quartet_fill(MeshDev m, const int4 *cand, int32_t n_cand, cons
     quart[q_off[c]] = r;
 }
 
-// ---- exclusive scan: per-block scan of 2048 elements, scan of block sums, add ----
+// ---- exclusive scan: per-block scan of 2048 elements, scan of block sums, add; up to two
+// arrays at once (grid.y), and a single kernel when one block covers them ----
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 2 * kScanThreads;
 
+// in[n] to out[n + 1] (the total last); total (may be null) receives it as well.
+struct Scan {
+    const int32_t *in[2];
+    int32_t *out[2], *total[2], *sums[2];
+    int32_t n, nb;
+};
+
+// Exclusive scan over the block's threads by warp shuffles; sh holds a warp's sum each.
 __device__ int32_t block_exclusive_scan(int32_t v, int32_t *sh, int32_t &total) {
-    // Hillis-Steele inclusive scan in shared memory, converted to exclusive.
-    const int t = threadIdx.x;
-    sh[t] = v;
-    __syncthreads();
-    for (int off = 1; off < blockDim.x; off <<= 1) {
-        const int32_t x = (t >= off) ? sh[t - off] : 0;
-        __syncthreads();
-        sh[t] += x;
-        __syncthreads();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    int32_t x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
     }
-    total = sh[blockDim.x - 1];
-    const int32_t incl = sh[t];
+    if (lane == 31) sh[w] = x;
     __syncthreads();
-    return incl - v;
+    if (w == 0) {
+        int32_t t = lane < nw ? sh[lane] : 0;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t y = __shfl_up_sync(0xffffffffu, t, o);
+            if (lane >= o) t += y;
+        }
+        if (lane < nw) sh[lane] = t;
+    }
+    __syncthreads();
+    total = sh[nw - 1];
+    const int32_t before = w ? sh[w - 1] : 0;
+    __syncthreads();
+    return before + x - v;
 }
 
-__global__ void k_scan_blocks(const int32_t *in, int32_t *out, int32_t n, int32_t *block_sums) {
-    __shared__ int32_t sh[kScanThreads];
-    const int64_t base = (int64_t)blockIdx.x * kScanItems;
-    const int64_t i0 = base + 2 * threadIdx.x;
-    const int32_t a = i0 < n ? in[i0] : 0;
-    const int32_t b = i0 + 1 < n ? in[i0 + 1] : 0;
+__device__ __forceinline__ void scan_total(const Scan &a, int y, int32_t total) {
+    a.out[y][a.n] = total;
+    if (a.total[y]) *a.total[y] = total;
+}
+
+__global__ void k_scan_blocks(Scan a) {
+    __shared__ int32_t sh[32];
+    const int y = blockIdx.y;
+    const int64_t i0 = (int64_t)blockIdx.x * kScanItems + 2 * threadIdx.x;
+    const int32_t v = i0 < a.n ? a.in[y][i0] : 0;
+    const int32_t w = i0 + 1 < a.n ? a.in[y][i0 + 1] : 0;
     int32_t total;
-    const int32_t ex = block_exclusive_scan(a + b, sh, total);
-    if (i0 < n) out[i0] = ex;
-    if (i0 + 1 < n) out[i0 + 1] = ex + a;
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
+    const int32_t ex = block_exclusive_scan(v + w, sh, total);
+    if (i0 < a.n) a.out[y][i0] = ex;
+    if (i0 + 1 < a.n) a.out[y][i0 + 1] = ex + v;
+    if (threadIdx.x != 0) return;
+    if (a.nb == 1)
+        scan_total(a, y, total);
+    else
+        a.sums[y][blockIdx.x] = total;
 }
 
-__global__ void k_scan_sums(int32_t *sums, int32_t nb, int32_t *grand_total) {
-    __shared__ int32_t sh[kScanThreads];
+__global__ void k_scan_sums(Scan a) {
+    __shared__ int32_t sh[32];
+    const int y = blockIdx.y;
     int32_t carry = 0;
-    for (int32_t c = 0; c < nb; c += kScanThreads) {
+    for (int32_t c = 0; c < a.nb; c += kScanThreads) {
         const int32_t i = c + threadIdx.x;
-        const int32_t v = i < nb ? sums[i] : 0;
+        const int32_t v = i < a.nb ? a.sums[y][i] : 0;
         int32_t total;
         const int32_t ex = block_exclusive_scan(v, sh, total);
-        if (i < nb) sums[i] = ex + carry;
+        if (i < a.nb) a.sums[y][i] = ex + carry;
         carry += total;
-        __syncthreads();
     }
-    if (threadIdx.x == 0) *grand_total = carry;
+    if (threadIdx.x == 0) scan_total(a, y, carry);
 }
 
-__global__ void k_scan_add(int32_t *out, int32_t n, const int32_t *sums) {
+__global__ void k_scan_add(Scan a) {
+    const int y = blockIdx.y;
     const int64_t i = (int64_t)blockIdx.x * kScanItems + threadIdx.x;
-    const int32_t add = sums[blockIdx.x];
-    if (i < n) out[i] += add;
-    if (i + kScanThreads < n) out[i + kScanThreads] += add;
+    const int32_t add = a.sums[y][blockIdx.x];
+    if (i < a.n) a.out[y][i] += add;
+    if (i + kScanThreads < a.n) a.out[y][i + kScanThreads] += add;
+}
+
+cudaError_t launch_scan(const Scan &a, int arrays, cudaStream_t s) {
+    const dim3 grid((unsigned)a.nb, (unsigned)arrays);
+    k_scan_blocks<<<grid, kScanThreads, 0, s>>>(a);
+    if (a.nb > 1) {
+        k_scan_sums<<<dim3(1, (unsigned)arrays), kScanThreads, 0, s>>>(a);
+        k_scan_add<<<grid, kScanThreads, 0, s>>>(a);
+    }
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -317,13 +419,21 @@ size_t exclusive_scan_tmp_elems(int32_t n) { return (size_t)(n + kScanItems - 1)
 
 cudaError_t exclusive_scan_i32(const int32_t *in, int32_t *out, int32_t n, int32_t *tmp, cudaStream_t s) {
     const int32_t nb = (n + kScanItems - 1) / kScanItems;
+    if (nb == 0) return cudaMemsetAsync(out, 0, sizeof(int32_t), s);
+    return launch_scan(Scan{{in, nullptr}, {out, nullptr}, {nullptr, nullptr}, {tmp, nullptr}, n, nb}, 1, s);
+}
+
+cudaError_t exclusive_scan_pair_i32(const int32_t *in0, int32_t *out0, const int32_t *in1, int32_t *out1, int32_t n,
+                                    int32_t *tmp, int32_t *totals, cudaStream_t s) {
+    const int32_t nb = (n + kScanItems - 1) / kScanItems;
     if (nb == 0) {
-        return cudaMemsetAsync(out, 0, sizeof(int32_t), s);
+        cudaError_t e = cudaMemsetAsync(out0, 0, sizeof(int32_t), s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(out1, 0, sizeof(int32_t), s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(totals, 0, 2 * sizeof(int32_t), s);
+        return e;
     }
-    k_scan_blocks<<<nb, kScanThreads, 0, s>>>(in, out, n, tmp);
-    k_scan_sums<<<1, kScanThreads, 0, s>>>(tmp, nb, out + n);
-    k_scan_add<<<nb, kScanThreads, 0, s>>>(out, n, tmp);
-    return cudaGetLastError();
+    int32_t *tmp1 = tmp + exclusive_scan_tmp_elems(n);
+    return launch_scan(Scan{{in0, in1}, {out0, out1}, {totals, totals + 1}, {tmp, tmp1}, n, nb}, 2, s);
 }
 
 cudaError_t launch_triplet_count(const MeshDev &m, const int4 *cand, int32_t n_cand, int32_t *n_trip,

@@ -172,7 +172,6 @@ struct tdg_ctx {
     int n_sm = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[10] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    int32_t h_tot[2] = {0, 0};  // enumeration totals (a pinned allocation costs more than it saves)
     DevBuf<int32_t> d_full_op;
     DevBuf<double> d_op_cart, d_fn;
     // host copy of the problem
@@ -691,7 +690,7 @@ extern "C" int tdg_create(tdg_ctx **out, const tdg_problem *p, int device) {
         chk(c->d_omhl.upload(omhl.data(), omhl.size(), s));
         chk(c->d_invom.upload(invom.data(), invom.size(), s));
     }
-    chk(c->d_status.alloc(1));
+    chk(c->d_status.alloc(4));  // the status word, then the totals of an enumeration
     chk(cudaStreamSynchronize(s));
     pt.mark("force constants, tables, uploads");
     if (e != cudaSuccess) return fail(set_error(kErrDevice, std::string("upload failed: ") + cudaGetErrorString(e)));
@@ -787,6 +786,18 @@ int read_status(tdg_ctx *c) {
     CUDA_TRY(copy_async(&st, c->d_status.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     if (st != kDevOk) return set_error(kErrDevice, "device-side index check failed (status " + std::to_string(st) + ")");
+    return kOk;
+}
+
+// The same with the two totals of the enumeration that just ran, in one copy.
+int read_status_totals(tdg_ctx *c, int32_t *total0, int32_t *total1) {
+    int32_t w[3] = {0, 0, 0};
+    CUDA_TRY(copy_async(w, c->d_status.p, sizeof w, cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(cudaStreamSynchronize(c->stream));
+    if (w[0] != kDevOk)
+        return set_error(kErrDevice, "device-side index check failed (status " + std::to_string(w[0]) + ")");
+    *total0 = w[1];
+    *total1 = w[2];
     return kOk;
 }
 
@@ -1307,7 +1318,7 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
         chk(c->d_nrd.alloc(nc + 1));
         chk(c->d_toff.alloc(nc + 1));
         chk(c->d_roff.alloc(nc + 1));
-        chk(c->d_tmp.alloc(exclusive_scan_tmp_elems(nc)));
+        chk(c->d_tmp.alloc(2 * exclusive_scan_tmp_elems(nc)));
         chk(c->d_rbeg.upload(rbeg.data(), rbeg.size(), s));
         chk(c->d_rlen.upload(rlen.data(), rlen.size(), s));
         if (shared) {
@@ -1336,7 +1347,7 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
         chk(c->d_nrd4.alloc(nc4 + 1));
         chk(c->d_qoff.alloc(nc4 + 1));
         chk(c->d_roff4.alloc(nc4 + 1));
-        chk(c->d_tmp4.alloc(exclusive_scan_tmp_elems(nc4)));
+        chk(c->d_tmp4.alloc(2 * exclusive_scan_tmp_elems(nc4)));
         chk(c->d_rbeg4.upload(rbeg4.data(), rbeg4.size(), s));
         chk(c->d_rlen4.upload(rlen4.data(), rlen4.size(), s));
         chk(c->d_list4a.upload(ql->list4a, ql->ptr4[nr], s));
@@ -1372,16 +1383,11 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
     int32_t ntrip = 0, nred = 0;
     if (o->thirdorder) {
         CUDA_TRY(launch_triplet_count(mesh, c->d_cand.p, nc, c->d_nt.p, c->d_nrd.p, c->d_status.p, s));
-        CUDA_TRY(exclusive_scan_i32(c->d_nt.p, c->d_toff.p, nc, c->d_tmp.p, s));
-        CUDA_TRY(exclusive_scan_i32(c->d_nrd.p, c->d_roff.p, nc, c->d_tmp.p, s));
-        launches += 1 + 2 * 3;
-        int32_t *tot = c->h_tot;
-        CUDA_TRY(copy_async(&tot[0], c->d_toff.p + nc, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-        CUDA_TRY(copy_async(&tot[1], c->d_roff.p + nc, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-        st = read_status(c);
+        CUDA_TRY(exclusive_scan_pair_i32(c->d_nt.p, c->d_toff.p, c->d_nrd.p, c->d_roff.p, nc, c->d_tmp.p,
+                                         c->d_status.p + 1, s));
+        launches += 1 + 3;
+        st = read_status_totals(c, &ntrip, &nred);
         if (st) return st;
-        ntrip = tot[0];
-        nred = tot[1];
         chk(c->d_trip.alloc(ntrip));
         chk(c->d_red.alloc(nred));
         if (e != cudaSuccess) return set_error(kErrDevice, std::string("allocation failed: ") + cudaGetErrorString(e));
@@ -1534,16 +1540,11 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
     if (o->fourthorder) {
         CUDA_TRY(cudaMemsetAsync(c->d_od.p, 0, sizeof(double) * (size_t)nr * ld, s));
         CUDA_TRY(launch_quartet_count(mesh, c->d_cand4.p, nc4, c->d_nq.p, c->d_nrd4.p, c->d_status.p, s));
-        CUDA_TRY(exclusive_scan_i32(c->d_nq.p, c->d_qoff.p, nc4, c->d_tmp4.p, s));
-        CUDA_TRY(exclusive_scan_i32(c->d_nrd4.p, c->d_roff4.p, nc4, c->d_tmp4.p, s));
-        launches += 1 + 2 * 3;
-        int32_t *tot = c->h_tot;
-        CUDA_TRY(copy_async(&tot[0], c->d_qoff.p + nc4, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-        CUDA_TRY(copy_async(&tot[1], c->d_roff4.p + nc4, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-        st = read_status(c);
+        CUDA_TRY(exclusive_scan_pair_i32(c->d_nq.p, c->d_qoff.p, c->d_nrd4.p, c->d_roff4.p, nc4, c->d_tmp4.p,
+                                         c->d_status.p + 1, s));
+        launches += 1 + 3;
+        st = read_status_totals(c, &nquart, &nred4);
         if (st) return st;
-        nquart = tot[0];
-        nred4 = tot[1];
         const int grid4 = fourphonon_grid(n, o->precision, o->integrationtype, c->n_sm, nquart);
         if (nquart > 0 && grid4 < 1) return set_error(kErrDevice, "four-phonon kernel configuration failed");
         chk(c->d_quart.alloc(nquart));

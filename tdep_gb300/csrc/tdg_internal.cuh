@@ -134,6 +134,9 @@ cudaError_t launch_quartet_fill(const MeshDev &m, const int4 *cand, int32_t n_ca
 // Exclusive scan of int32 (n <= 2^31), result in out; total in out[n].
 cudaError_t exclusive_scan_i32(const int32_t *in, int32_t *out, int32_t n, int32_t *tmp, cudaStream_t s);
 size_t exclusive_scan_tmp_elems(int32_t n);
+// Two of them at once; totals[2] receives both totals; tmp holds 2 exclusive_scan_tmp_elems(n).
+cudaError_t exclusive_scan_pair_i32(const int32_t *in0, int32_t *out0, const int32_t *in1, int32_t *out1, int32_t n,
+                                    int32_t *tmp, int32_t *totals, cudaStream_t s);
 
 // K2+K3+K4: fused pretransform, contraction and delta/Bose accumulation.
 struct ThreePhArgs {
