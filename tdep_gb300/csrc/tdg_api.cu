@@ -232,6 +232,8 @@ struct tdg_ctx {
     DevBuf<uint32_t> d_mask;
     DevBuf<int32_t> d_nt, d_nrd, d_toff, d_roff, d_tmp, d_list3, d_rlen;
     DevBuf<int64_t> d_rbeg;
+    DevBuf<int32_t> d_row_of, d_copies, d_ucnt, d_uoff;  // union_candidates
+    DevBuf<unsigned long long> d_utotal;
     DevBuf<int4> d_qdesc;
     DevBuf<TripletRec> d_trip;
     DevBuf<int2> d_red;
@@ -925,6 +927,78 @@ cudaError_t rezero_outputs(tdg_ctx *c, int64_t nr, int64_t ld, cudaStream_t s) {
     return e;
 }
 
+namespace {
+// Total length of the three-phonon lists up to which they go to the device as they are.
+constexpr int64_t kShortLists = 1 << 16;
+// Copies counted at a time (rows x points) by union_candidates.
+constexpr int64_t kUnionCounts = (int64_t)1 << 28;
+
+// Three-phonon candidates and their row masks (d_cand, d_mask) from samples that differ
+// between the rows of a q1. row_of: first row of every q1. Nothing of the context's last
+// scattering is touched before the lists have been found good.
+int union_candidates(tdg_ctx *c, const tdg_qlists *ql, const std::vector<int> &row_of, const std::vector<int64_t> &rbeg,
+                     const std::vector<int32_t> &rlen, const std::vector<int32_t> &row_b1, int64_t &nc) {
+    cudaStream_t s = c->stream;
+    const int N = c->N, nirr = c->nirr, nr = ql->n_row;
+    const int64_t all = (int64_t)nirr * N;
+    cudaError_t e = cudaSuccess;
+    auto chk = [&](cudaError_t x) {
+        if (e == cudaSuccess) e = x;
+    };
+    // whole q1 at a time, as many as kUnionCounts holds
+    std::vector<int> part{0};
+    int64_t most = 0;
+    for (int q1 = 0; q1 < nirr; ++q1) {
+        const int64_t rows = row_of[q1 + 1] - row_of[part.back()];
+        if (rows * N > kUnionCounts && q1 > part.back()) part.push_back(q1);
+        most = std::max<int64_t>(most, row_of[q1 + 1] - row_of[part.back()]);
+    }
+    part.push_back(nirr);
+    chk(c->d_list3.upload(ql->list3, ql->ptr3[nr], s));
+    chk(c->d_rbeg.upload(rbeg.data(), rbeg.size(), s));
+    chk(c->d_rlen.upload(rlen.data(), rlen.size(), s));
+    chk(c->d_row_b1.upload(row_b1.data(), row_b1.size(), s));
+    chk(c->d_row_of.upload(row_of.data(), row_of.size(), s));
+    chk(c->d_copies.alloc((size_t)most * N));
+    chk(c->d_ucnt.alloc((size_t)all + 1));
+    chk(c->d_uoff.alloc((size_t)all + 1));
+    chk(c->d_tmp.alloc(exclusive_scan_tmp_elems((int32_t)all)));
+    chk(c->d_utotal.alloc(1));
+    if (e != cudaSuccess) return set_error(kErrDevice, std::string("allocation/upload failed: ") + cudaGetErrorString(e));
+    CUDA_TRY(cudaMemsetAsync(c->d_status.p, 0, sizeof(int32_t), s));
+    CUDA_TRY(cudaMemsetAsync(c->d_utotal.p, 0, sizeof(unsigned long long), s));
+    auto count = [&](size_t k) {
+        const int r0 = row_of[part[k]];
+        return launch_union_count(N, r0, row_of[part[k + 1]] - r0, c->d_rbeg.p, c->d_rlen.p, c->d_list3.p, c->d_copies.p,
+                                  c->d_status.p, s);
+    };
+    for (size_t k = 0; k + 1 < part.size(); ++k) {
+        CUDA_TRY(count(k));
+        CUDA_TRY(launch_union_copies(N, part[k], part[k + 1] - part[k], row_of[part[k]], c->d_row_of.p, c->d_copies.p,
+                                     c->d_ucnt.p, c->d_utotal.p, s));
+    }
+    CUDA_TRY(exclusive_scan_i32(c->d_ucnt.p, c->d_uoff.p, (int32_t)all, c->d_tmp.p, s));
+    int32_t bad = 0;
+    unsigned long long total = 0;
+    CUDA_TRY(copy_async(&bad, c->d_status.p, sizeof bad, cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(copy_async(&total, c->d_utotal.p, sizeof total, cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(cudaStreamSynchronize(s));
+    if (bad) return set_error(kErrParam, "three-phonon sample: q' index out of range");
+    if (total >= ((unsigned long long)1 << 31) - 1)
+        return set_error(kErrBadDim, "too many three-phonon candidates for one call");
+    nc = (int64_t)total;
+    chk(c->d_cand.alloc((size_t)nc));
+    chk(c->d_mask.alloc(4 * (size_t)nc));
+    if (e != cudaSuccess) return set_error(kErrDevice, std::string("allocation failed: ") + cudaGetErrorString(e));
+    for (size_t k = 0; k + 1 < part.size(); ++k) {
+        if (part.size() > 2) CUDA_TRY(count(k));  // one part: still counted
+        CUDA_TRY(launch_union_write(N, part[k], part[k + 1] - part[k], row_of[part[k]], c->d_row_of.p, c->d_row_b1.p,
+                                    c->d_copies.p, c->d_uoff.p, c->d_cand.p, c->d_mask.p, s));
+    }
+    return kOk;
+}
+}  // namespace
+
 extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *ql, double *linewidth, double *qs_out,
                               double *stats) {
     XferScope xs(c ? c->xfer : nullptr);
@@ -1035,12 +1109,11 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
     // When all rows of a q1 share one sample (the full grid, or samples given per q1) it is
     // uploaded once per q1 and the candidates (q1, q2, mask of every row of q1) are formed
     // on the device, in sample order. Otherwise the candidates are, per q1, the union of
-    // its rows' samples, with the set of rows that sampled q2 as a bit mask. Masks are
-    // stored once in a table of distinct masks. A q-point that a row samples k times (the
+    // its rows' samples, with the set of rows that sampled q2 as a bit mask, formed on the
+    // device from the uploaded lists (union_candidates). A q-point that a row samples k times (the
     // reference's sampler only avoids repeating the previous point, so this happens when the
     // Monte-Carlo grid does not divide the mesh) is counted k times, as the reference does:
     // the j-th copy of a candidate carries the rows that sampled the point at least j times.
-    std::vector<int4> cand;                 // union path
     std::vector<uint32_t> masks;            // distinct row masks (4 words each)
     std::vector<int64_t> rbeg(nr, 0);       // per row: start of its sample in the uploaded list
     std::vector<int32_t> rlen(nr, 0);
@@ -1062,8 +1135,11 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
         };
         // rows of a q1 share one sample when every row's list equals the first row's
         // (compared on all host threads)
+        // short lists go up as they are instead: merging them on the device costs less than
+        // waking the host threads for the comparison (fcc 4^3, 1344 entries: 91 us on the host)
+        shared = ql->ptr3[nr] > kShortLists;
         std::vector<char> same(nirr, 1);
-        parallel_for(nirr, [&](int64_t q1) {
+        if (shared) parallel_for(nirr, [&](int64_t q1) {
             int r0, r1;
             rows_of((int)q1, r0, r1);
             for (int r = r0 + 1; r < r1; ++r) {
@@ -1084,7 +1160,6 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
             table.push_back(key);
             return (int)table.size() - 1;
         };
-        std::vector<int32_t> stamp(N, -1);
         if (shared) {
             // one list per q1: offsets first, then range checks and the copy in parallel (the
             // other rows' lists are byte-equal to it); a repeated entry becomes a repeated
@@ -1131,57 +1206,12 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
             nc64 = start[nirr];
             pt.mark("three-phonon shared samples (host)");
         } else {
-            std::atomic<int> bad{0};
-            parallel_for(nr, [&](int64_t r) {
-                for (int64_t i = ql->ptr3[r]; i < ql->ptr3[r + 1]; ++i)
-                    if (ql->list3[i] < 1 || ql->list3[i] > N) bad.store(1);
-            });
-            if (bad.load()) return set_error(kErrParam, "three-phonon sample: q' index out of range");
-            std::vector<uint32_t> mark((size_t)N * 4, 0u);
-            std::vector<int32_t> touched, occ(N, 0), row_touched;
-            std::vector<std::array<int, 3>> extra;  // (q2, copy index >= 2, b1)
-            for (int q1 = 0; q1 < nirr; ++q1) {
-                int r0, r1;
-                rows_of(q1, r0, r1);
-                touched.clear();
-                extra.clear();
-                for (int r = r0; r < r1; ++r) {
-                    const int b1 = rb1[r];
-                    rbeg[r] = ql->ptr3[r];
-                    rlen[r] = (int32_t)(ql->ptr3[r + 1] - ql->ptr3[r]);
-                    row_touched.clear();
-                    for (int64_t i = ql->ptr3[r]; i < ql->ptr3[r + 1]; ++i) {
-                        const int q2 = ql->list3[i] - 1;
-                        if (stamp[q2] == r) {
-                            extra.push_back({q2, ++occ[q2], b1});
-                            continue;
-                        }
-                        stamp[q2] = r;
-                        occ[q2] = 1;
-                        row_touched.push_back(q2);
-                        uint32_t *mk = &mark[(size_t)q2 * 4];
-                        if (!(mk[0] | mk[1] | mk[2] | mk[3])) touched.push_back(q2);
-                        mk[b1 >> 5] |= 1u << (b1 & 31);
-                    }
-                    for (int q2 : row_touched) occ[q2] = 0;
-                }
-                std::sort(touched.begin(), touched.end());
-                for (int q2 : touched) {
-                    uint32_t *mk = &mark[(size_t)q2 * 4];
-                    cand.push_back(make_int4(q1, q2, mask_id({mk[0], mk[1], mk[2], mk[3]}), 0));
-                    mk[0] = mk[1] = mk[2] = mk[3] = 0u;
-                }
-                std::sort(extra.begin(), extra.end());
-                for (size_t i = 0; i < extra.size();) {
-                    std::array<uint32_t, 4> key = {0u, 0u, 0u, 0u};
-                    size_t j = i;
-                    for (; j < extra.size() && extra[j][0] == extra[i][0] && extra[j][1] == extra[i][1]; ++j)
-                        key[extra[j][2] >> 5] |= 1u << (extra[j][2] & 31);
-                    cand.push_back(make_int4(q1, extra[i][0], mask_id(key), 0));
-                    i = j;
-                }
+            for (int r = 0; r < nr; ++r) {
+                rbeg[r] = ql->ptr3[r];
+                rlen[r] = (int32_t)(ql->ptr3[r + 1] - ql->ptr3[r]);
             }
-            nc64 = (int64_t)cand.size();
+            st = union_candidates(c, ql, qr0, rbeg, rlen, rb1, nc64);
+            if (st) return st;
         }
         for (const auto &t : table) masks.insert(masks.end(), t.begin(), t.end());
         if (nc64 >= ((int64_t)1 << 31) - 1 || (int64_t)slist_n >= ((int64_t)1 << 31))
@@ -1313,24 +1343,21 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
     chk(c->d_xi.alloc((size_t)nr * ld));
     chk(c->d_gamma.alloc(nr));
     if (o->thirdorder) {
-        chk(c->d_mask.upload(masks.data(), masks.size(), s));
+        if (shared) chk(c->d_mask.upload(masks.data(), masks.size(), s));
         chk(c->d_nt.alloc(nc + 1));
         chk(c->d_nrd.alloc(nc + 1));
         chk(c->d_toff.alloc(nc + 1));
         chk(c->d_roff.alloc(nc + 1));
         chk(c->d_tmp.alloc(2 * exclusive_scan_tmp_elems(nc)));
-        chk(c->d_rbeg.upload(rbeg.data(), rbeg.size(), s));
-        chk(c->d_rlen.upload(rlen.data(), rlen.size(), s));
         if (shared) {
+            chk(c->d_rbeg.upload(rbeg.data(), rbeg.size(), s));
+            chk(c->d_rlen.upload(rlen.data(), rlen.size(), s));
             chk(c->d_list3.upload(tl_slist.get(), slist_n, s));
             chk(c->d_qdesc.upload(qdesc.data(), qdesc.size(), s));
             chk(c->d_cand.alloc(nc));
             int maxL = 0;
             for (const auto &d : qdesc) maxL = std::max(maxL, d.y);
             chk(launch_build_candidates(c->d_qdesc.p, nirr, maxL, c->d_list3.p, c->d_cand.p, s));
-        } else {
-            chk(c->d_cand.upload(cand.data(), cand.size(), s));
-            chk(c->d_list3.upload(ql->list3, ql->ptr3[nr], s));
         }
     }
     if (o->isotope) {
@@ -1353,7 +1380,6 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
         chk(c->d_list4a.upload(ql->list4a, ql->ptr4[nr], s));
         chk(c->d_od.alloc((size_t)nr * ld));
     }
-    chk(cudaStreamSynchronize(s));
     pt.mark("allocations and uploads");
     if (e != cudaSuccess) return set_error(kErrDevice, std::string("allocation/upload failed: ") + cudaGetErrorString(e));
     ph.be = c->d_be.p;

@@ -330,6 +330,16 @@ cudaError_t launch_sym_distribute(const MeshDev &m, const OrbitDev &o, int32_t n
 // first candidate, mask id); cand[desc.z + i] = (q1, list[desc.x + i] - 1, desc.w, 0).
 cudaError_t launch_build_candidates(const int4 *desc, int32_t n_irr, int32_t max_len, const int32_t *list, int4 *cand,
                                     cudaStream_t s);
+// Candidates of rows with samples of their own: copies of every point in each of the rows
+// [r0, r0 + n_row) (cnt, [n_row * n_full]; a list entry off the mesh sets the status word);
+// candidates per (q1, q2) of the q1 those rows are all of, and their sum; the candidates and
+// a mask for each from the exclusive scan off of all copies. row_of[n_irr + 1]: first row.
+cudaError_t launch_union_count(int n_full, int r0, int n_row, const int64_t *rbeg, const int32_t *rlen,
+                               const int32_t *list, int32_t *cnt, int32_t *status, cudaStream_t s);
+cudaError_t launch_union_copies(int n_full, int q0, int n_q1, int r0, const int32_t *row_of, const int32_t *cnt,
+                                int32_t *copies, unsigned long long *total, cudaStream_t s);
+cudaError_t launch_union_write(int n_full, int q0, int n_q1, int r0, const int32_t *row_of, const int32_t *row_b1,
+                               const int32_t *cnt, const int32_t *off, int4 *cand, uint32_t *mask, cudaStream_t s);
 // K5b: symmetrize_and_distribute of the three-phonon terms in place on xi (dist, orbits
 // whose representative the row sampled per sbits, launch_sample_bits) and/or
 // symmetrize_scatmat (scat, scattering.f90:296-357), on tiles of whole orbits.
