@@ -425,14 +425,22 @@ __global__ void __launch_bounds__(kLnGemmThreads, 1) k_ln_gemm(LnGemmArgs g) {
     }
 }
 
-// ---- delta weights and accumulation: one CTA per (slot, b1) ----
-// GB300's FP64 pipe is 1/64 of FP32, and only a fraction of the n^2 mode pairs (b2, b3) has a
-// Gaussian inside its 8-sigma window. In blocks of BB rows b2 (16 or 32, autotuned): (A) every pair is screened
-// in FP32 (window with a margin far above FP32 rounding, degeneracy skips pre-checked in
-// FP32), the survivors are compacted into a queue with a block scan; (B) full warps evaluate
-// the queue's Gaussians (the reference's 8-sigma window) and occupations in FP32 into a
-// dense FP64 F; (C) R2[b2] = sum_b3 F and R3[b3] += sum_b2 F in FP64.
-
+// ---- delta weights and accumulation: four warps per (slot, b1), two b1 per CTA ----
+// Bound by instruction issue: n^2 mode pairs (b2, b3) a row mode, of which the 8-sigma windows
+// keep a quarter or so. A warp takes four rows b2 at a time with the columns b3 spread over
+// its lanes (their screen values stay in registers for the whole pass): (A) the FP32 screen of
+// the four rows, without square root or division and with a margin far above FP32 rounding,
+// queues the survivors; (B) full warps evaluate the queue's Gaussians (the reference's 8-sigma
+// window) and occupations in FP32, the centre differences from FP32 (hi, rest) frequency
+// pairs, into the warp's dense rows F; (C) the rows and columns of F are summed in
+// double-float (TwoSum; exact to ~2^-44 for these few hundred FP32 terms): the columns in
+// registers to the end, the four rows by one transposing reduction. No barrier but the one
+// before and the one after the rows. GB300 issues FP64 at 1/64 of the FP32 rate, so FP64 is
+// left to the FP32 copy of the occupations and to the final sums.
+// 120 modes, 1184 q-triplets (2e9 pairs): about 3.8 ms of
+// the call, against 15.9 ms for a CTA per row mode that screened with a square root and two
+// integer divisions a pair, queued by block scans and summed F between barriers (call 44.4 ->
+// 32.3 ms).
 struct LnDeltaArgs {
     MeshDev mesh;
     PhononDev ph;
@@ -448,227 +456,223 @@ struct LnDeltaArgs {
     float2 *w;
 };
 
-__host__ __device__ inline size_t ln_delta_smem(int n, int bb) {
-    return sizeof(double) * (size_t)14 * n + sizeof(float) * (size_t)bb * n + sizeof(uint32_t) * (size_t)bb * n +
-           sizeof(int) * 33 + sizeof(float) * 8 * (size_t)n + 16;
+constexpr int kLnDeltaThreads = 256;
+constexpr int kLnDeltaB1 = 2;                                        // row modes per CTA
+constexpr int kLnDeltaWarps = kLnDeltaThreads / 32 / kLnDeltaB1;     // warps per row mode
+constexpr int kLnDeltaRows = 4;                                      // rows b2 a warp takes at a time
+constexpr float kLnNoMode = 1e18f;                                   // a frequency no window holds
+
+__host__ __device__ inline size_t ln_delta_smem(int n, int nc) {
+    return sizeof(float4) * (size_t)2 * n +                                    // T2, T3
+           sizeof(float2) * (size_t)kLnDeltaB1 * (1 + kLnDeltaWarps) * n +     // row and column sums
+           (size_t)(kLnDeltaThreads / 32) * kLnDeltaRows * 32 * nc * (sizeof(float) + sizeof(uint16_t));
+}
+
+__device__ __forceinline__ float2 df_shfl_xor(float2 v, int o) {
+    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
 }
 
 // ADJ: the adjoint's weights. F holds G_b = lam(row) * nred * dF_b/d|Psi_b|^2 of the
 // survivors (F without |Psi|^2), and W_b = G_b conj(Psi_b) replaces Psi_b for every (b2, b3)
 // of the row mode b1, zero where nothing survives or the row is not sampled.
-template <bool ADJ, int BB>
-__global__ void __launch_bounds__(256) k_ln_delta(LnDeltaArgs a) {
+// NC = ceil(n / 32), the columns of a lane. W6: integrationtype 6, whose FP64 widths take more
+// registers (apart, the other types need no spill at four CTAs per SM).
+template <bool ADJ, int NC, bool W6>
+__global__ void __launch_bounds__(kLnDeltaThreads, W6 ? 2 : 4) k_ln_delta(LnDeltaArgs a) {
     extern __shared__ __align__(16) unsigned char sm[];
+    constexpr int W = 32 * NC;
     const int n = a.n;
-    const int s = blockIdx.y, b1 = blockIdx.x;
-    const int tid = threadIdx.x, bd = blockDim.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int sub = warp % kLnDeltaWarps, slot1 = warp / kLnDeltaWarps;
+    const int s = blockIdx.y, b1 = blockIdx.x * kLnDeltaB1 + slot1;
     const TripletRec rec = a.trip[s];
     const MeshDev &m = a.mesh;
     const PhononDev &P = a.ph;
     const uint32_t *mask = a.cand_mask + (size_t)rec.cand * 4;
-    const int row = a.rows.rowidx[(size_t)rec.q1 * n + b1];
-    if (!((mask[b1 >> 5] >> (b1 & 31)) & 1u) || row < 0) {
-        if (ADJ) {
-            float2 *wr = a.w + ((int64_t)s * n + b1) * n * n;
-            for (int e = tid; e < n * n; e += bd) wr[e] = make_float2(0.f, 0.f);
-        }
-        return;
-    }
+    const int row = b1 < n ? a.rows.rowidx[(size_t)rec.q1 * n + b1] : -1;
+    const bool active = row >= 0 && ((mask[b1 >> 5] >> (b1 & 31)) & 1u);
     const int f1 = m.irr_full[rec.q1], q2 = rec.q2, q3 = rec.q3;
     const int i2 = m.full_irr[q2], i3 = m.full_irr[q3];
-    double *om2 = (double *)sm, *om3 = om2 + n, *be2 = om3 + n, *be3 = be2 + n, *s2 = be3 + n, *s3 = s2 + n;
-    double *v2 = s3 + n, *v3 = v2 + 3 * n, *R2 = v3 + 3 * n, *R3 = R2 + n;
-    float *F = (float *)(R3 + n);  // the block's F in FP32 (its values are FP32 products)
-    uint32_t *Q = (uint32_t *)(F + (size_t)BB * n);
-    int *wsum = (int *)(Q + (size_t)BB * n);
-    // FP32 copies for the screen (double -> float conversions run on the FP64 pipe, so they
-    // are made once per mode here instead of once per pair); NaN marks omega < 1e-9 Ha.
-    float *g2 = (float *)(wsum + 33), *g3 = g2 + n, *t2 = g3 + n, *t3 = t2 + n, *c2 = t3 + n, *c3 = c2 + n;
-    float *l2 = c3 + n, *l3 = l2 + n;  // om - (double)g, the FP32 rest of each frequency
-    for (int b = tid; b < n; b += bd) {
-        om2[b] = P.omega[(size_t)q2 * n + b];
-        om3[b] = P.omega[(size_t)q3 * n + b];
-        be2[b] = P.be[(size_t)i2 * n + b];
-        be3[b] = P.be[(size_t)i3 * n + b];
-        s2[b] = P.sigsq[(size_t)i2 * n + b];
-        s3[b] = P.sigsq[(size_t)i3 * n + b];
-        g2[b] = om2[b] < kFreqTolD ? __int_as_float(0x7fc00000) : (float)om2[b];
-        g3[b] = om3[b] < kFreqTolD ? __int_as_float(0x7fc00000) : (float)om3[b];
-        t2[b] = (float)s2[b];
-        t3[b] = (float)s3[b];
-        c2[b] = (float)be2[b];
-        c3[b] = (float)be3[b];
-        l2[b] = om2[b] < kFreqTolD ? 0.f : (float)(om2[b] - (double)g2[b]);
-        l3[b] = om3[b] < kFreqTolD ? 0.f : (float)(om3[b] - (double)g3[b]);
-        for (int d = 0; d < 3; ++d) {
-            v2[b * 3 + d] = P.vel[((size_t)q2 * n + b) * 3 + d];
-            v3[b * 3 + d] = P.vel[((size_t)q3 * n + b) * 3 + d];
-        }
-        R3[b] = 0.0;
-    }
-    __syncthreads();
-    const double o1 = P.omega[(size_t)f1 * n + b1];
-    const double s1 = P.sigsq[(size_t)rec.q1 * n + b1];
-    double v1[3];
-    for (int d = 0; d < 3; ++d) v1[d] = P.vel[((size_t)f1 * n + b1) * 3 + d];
-    const double w = a.rows.weight3[row];
-    const double perm = q2 == q3 ? 1.0 : 2.0;
-    // F = perm * (pi/16) |Psi|^2 w * ((n2 - n3) d0 + (n2 + n3 + 1) d1), constants folded;
-    // the adjoint's G = lambda(row) * k * dF/d|Psi|^2
-    const double pw = perm * kLnPrefactor * w;
-    const double fadj = ADJ ? a.lam[row] * (double)rec.red_cnt * pw : 0.0;
-    const float pwf = (float)pw, fadjf = (float)fadj;
     const int it = P.integrationtype;
-    const float fo1 = (float)o1, fs1 = (float)s1, fsig = (float)P.sigma_fixed;
-    const float fl1 = (float)(o1 - (double)fo1);
-    const float2 *psi = a.psi + ((int64_t)s * n + b1) * n * n;
-    // 4-bit live mask of the Gaussians of pair (b2, b3), 0 when a skip rule applies
-    // (scattering_threephonon.f90:90-101) or no Gaussian can reach its window. FP64 work
-    // only for the rare pairs whose FP32 frequencies nearly coincide.
-    auto screen = [&](int b2, int b3) -> uint32_t {
-        const float f2 = g2[b2], f3 = g3[b3];
-        if (f2 != f2 || f3 != f3) return 0u;  // omega2 or omega3 below 1e-9 Ha
-        // |x - y| < 1e-9 from the FP32 (hi, rest) pairs: the hi difference is exact where it
-        // matters (Sterbenz), so the test is the FP64 one to ~1e-17; no FP64 instruction (a
-        // short-circuit FP64 test is evaluated for every pair once the compiler if-converts it)
-        if (close_f32(fo1, fl1, f2, l2[b2])) return 0u;
-        if (close_f32(fo1, fl1, f3, l3[b3])) return 0u;
-        if (close_f32(f2, l2[b2], f3, l3[b3])) return 0u;
-        if (it == 6) return 15u;  // the velocity-difference width can cancel in FP32: not screened
-        const float sg = it == 1 ? fsig : sqrt_screen(fs1 + t2[b2] + t3[b3]);
-        const float win = 8.0f * sg * 1.001f + 1e-6f * (fo1 + f2 + f3);
-        return (fabsf(fo1 + f2 - f3) <= win ? 1u : 0u) | (fabsf(fo1 - f2 + f3) <= win ? 2u : 0u) |
-               (fabsf(fo1 - f2 - f3) <= win ? 4u : 0u) | (fo1 + f2 + f3 <= win ? 8u : 0u);
-    };
-    for (int bb = 0; bb < n; bb += BB) {
-        const int nbb = min(BB, n - bb), cnt = nbb * n;
-        // (A) contiguous chunk per thread (at most 16 entries: BB * 128 / 256)
-        const int per = (cnt + bd - 1) / bd;
-        const int e0 = min(cnt, tid * per), e1 = min(cnt, e0 + per);
-        uint64_t lives = 0;
-        int ns = 0;
-        for (int e = e0; e < e1; ++e) {
-            const uint32_t l = screen(bb + e / n, e % n);
-            lives |= (uint64_t)l << (4 * (e - e0));
-            ns += l != 0u;
-        }
-        for (int e = tid; e < cnt; e += bd) F[e] = 0.f;
-        int total = 0;
-        int k = block_exclusive_scan(ns, wsum, total);  // contains __syncthreads
-        for (int e = e0; e < e1; ++e) {
-            const uint32_t l = (uint32_t)(lives >> (4 * (e - e0))) & 15u;
-            if (l) Q[k++] = (uint32_t)e | (l << 16);
-        }
-        __syncthreads();
-        // (B) delta weights and occupations of the survivors, full warps: the Gaussians and
-        // occupation factors in FP32, the centre differences from FP32 (hi, rest) frequency
-        // pairs (the path is mixed precision; GB300 issues FP64 at 1/64 of the FP32 rate, and
-        // an FP64 warp instruction holds its pipe for 16 cycles whatever its active lanes),
-        // the sums in FP64
-        for (int i = tid; i < total; i += bd) {
-            const uint32_t qv = Q[i];
-            const int e = (int)(qv & 0xffffu);
-            uint32_t live = qv >> 16;
-            const int b2 = bb + e / n, b3 = e % n;
-            float sigma;
-            if (it == 1) {
-                sigma = fsig;
-            } else if (it == 2) {
-                sigma = sqrtf(fs1 + t2[b2] + t3[b3]);
-            } else {
-                sigma = (float)(adaptive_pair(v1, v2 + 3 * b2, P.reclat_g) / 3.0 +
-                                adaptive_pair(v1, v3 + 3 * b3, P.reclat_g) / 3.0 +
-                                adaptive_pair(v2 + 3 * b2, v3 + 3 * b3, P.reclat_g) / 3.0 + P.thresh_sigma);
-            }
-            const float invsig = 1.0f / sigma;
-            const float win8 = 8.0f * sigma, h = 0.5f * invsig * invsig, cg = kSqrt2PiInvF * invsig;
-            float gs[4] = {0.f, 0.f, 0.f, 0.f};
-            const float h2 = g2[b2], r2 = l2[b2], h3 = g3[b3], r3 = l3[b3];
-            while (live) {
-                const int j = __ffs(live) - 1;
-                live &= live - 1;
-                // Gaussian j centred at (-om2+om3, om2-om3, om2+om3, -om2-om3), get_dirac's
-                // order; the centre difference from the FP32 (hi, rest) pairs, no FP64
-                const float sg2 = (j == 1 || j == 2) ? 1.f : -1.f;
-                const float sg3 = (j == 0 || j == 2) ? 1.f : -1.f;
-                const float dx = centre_diff_f32(fo1, fl1, sg2 * h2, sg2 * r2, sg3 * h3, sg3 * r3);
-                const float gj = fabsf(dx) > win8 ? 0.f : expf(-dx * dx * h) * cg;
-                gs[0] = j == 0 ? gj : gs[0];
-                gs[1] = j == 1 ? gj : gs[1];
-                gs[2] = j == 2 ? gj : gs[2];
-                gs[3] = j == 3 ? gj : gs[3];
-            }
-            const float d0 = gs[0] - gs[1], d1 = gs[2] - gs[3];
-            if (d0 == 0.f && d1 == 0.f) continue;
-            const float n2 = c2[b2], n3 = c3[b3];
-            const float occ = (n2 - n3) * d0 + (n2 + n3 + 1.0f) * d1;
-            if (ADJ) {
-                F[e] = fadjf * occ;
-                continue;
-            }
-            const float2 ps = psi[b2 * n + b3];
-            F[e] = pwf * fmaf(ps.x, ps.x, ps.y * ps.y) * occ;
-        }
-        __syncthreads();
-        if (ADJ) {
-            float2 *wr = a.w + ((int64_t)s * n + b1) * n * n + (int64_t)bb * n;
-            for (int e = tid; e < cnt; e += bd) {
-                const float g = F[e];
-                const float2 ps = wr[e];
-                wr[e] = make_float2(g * ps.x, -g * ps.y);
-            }
-            __syncthreads();
-            continue;
-        }
-        // (C) row sums of the block and running column sums, spread over the whole block: a
-        // warp per row with the columns split over its lanes, two threads per column; the
-        // block sums in double-float on the FP32 pipe (TwoSum; exact to ~2^-44 for these
-        // few hundred FP32 terms), turned into FP64 once per row and column: an FP64 warp
-        // instruction holds GB300's FP64 pipe 16 cycles whatever its active lanes, and the
-        // FP64 adds over the dense block had been about 40 % of the kernel
-        {
-            const int lane = tid & 31, wid = tid >> 5, nw = bd >> 5;
-            for (int r = wid; r < nbb; r += nw) {
-                float2 sum = make_float2(0.f, 0.f);
-                for (int b3 = lane; b3 < n; b3 += 32) df_acc(sum, F[r * n + b3]);
+    float4 *T2 = (float4 *)sm, *T3 = T2 + n;  // (frequency, its rest, width^2, occupation) of every mode
+    float2 *R2 = (float2 *)(T3 + n) + (size_t)slot1 * n;
+    float2 *R3 = (float2 *)(T3 + n) + (size_t)(kLnDeltaB1 + slot1 * kLnDeltaWarps) * n;
+    float *F = (float *)((float2 *)(T3 + n) + (size_t)kLnDeltaB1 * (1 + kLnDeltaWarps) * n) +
+               (size_t)warp * kLnDeltaRows * W;
+    uint16_t *Q = (uint16_t *)(F + (size_t)(kLnDeltaThreads / 32 - warp) * kLnDeltaRows * W) +
+                  (size_t)warp * kLnDeltaRows * W;
+    for (int e = tid; e < 2 * n; e += kLnDeltaThreads) {
+        const int b = e < n ? e : e - n;
+        const float2 hl = P.omega_hl[(size_t)(e < n ? q2 : q3) * n + b];
+        const size_t ib = (size_t)(e < n ? i2 : i3) * n + b;
+        // NaN marks omega < 1e-9 Ha; with one width for all, every width^2 comes from s1 below
+        T2[e] = make_float4(hl.x != hl.x ? kLnNoMode : hl.x, hl.x != hl.x ? 0.f : hl.y, it == 1 ? 0.f : P.sigsq32[ib],
+                            (float)P.be[ib]);
+    }
+    for (int b = sub * 32 + lane; b < n; b += 32 * kLnDeltaWarps) R2[b] = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1)
-                    sum = df_merge(sum, make_float2(__shfl_xor_sync(0xffffffffu, sum.x, o),
-                                                    __shfl_xor_sync(0xffffffffu, sum.y, o)));
-                if (lane == 0) R2[bb + r] = (double)sum.x + (double)sum.y;
+    for (int r = 0; r < kLnDeltaRows; ++r)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) F[r * W + c * 32 + lane] = 0.f;
+    __syncthreads();
+
+    if (ADJ && !active && b1 < n) {
+        float2 *wr = a.w + ((int64_t)s * n + b1) * n * n;
+        for (int e = sub * 32 + lane; e < n * n; e += 32 * kLnDeltaWarps) wr[e] = make_float2(0.f, 0.f);
+    }
+    if (active) {
+        const float2 o1 = P.omega_hl[(size_t)f1 * n + b1];
+        const float fo1 = o1.x, fl1 = o1.y;
+        const float fsig = (float)P.sigma_fixed;
+        const float fs1 = it == 1 ? fsig * fsig : P.sigsq32[(size_t)rec.q1 * n + b1];
+        // F = perm * (pi/16) |Psi|^2 w * ((n2 - n3) d0 + (n2 + n3 + 1) d1), constants folded;
+        // the adjoint's G = lambda(row) * k * dF/d|Psi|^2
+        const double pw = (q2 == q3 ? 1.0 : 2.0) * kLnPrefactor * a.rows.weight3[row];
+        const float pwf = ADJ ? (float)(a.lam[row] * (double)rec.red_cnt * pw) : (float)pw;
+        // The columns of this lane for the screen: kLnNoMode where a skip rule applies to the
+        // column whatever the row (scattering_threephonon.f90:90-101). |d| - 2e-6 (sum of the
+        // frequencies) <= 8.016 sigma is tested by its square; 64.26 = 8.016^2.
+        float f3[NC], w3[NC], f3max = 0.f;
+        [[maybe_unused]] float2 col[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const int b3 = c * 32 + lane;
+            const float4 t = b3 < n ? T3[b3] : make_float4(kLnNoMode, 0.f, 0.f, 0.f);
+            const bool no = t.x >= kLnNoMode || close_f32(fo1, fl1, t.x, t.y);
+            f3[c] = no ? kLnNoMode : t.x;
+            w3[c] = 64.26f * t.z;
+            f3max = fmaxf(f3max, no ? 0.f : t.x);
+            col[c] = make_float2(0.f, 0.f);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) f3max = fmaxf(f3max, __shfl_xor_sync(0xffffffffu, f3max, o));
+        const uint32_t below = (1u << lane) - 1u;
+        for (int base = sub * kLnDeltaRows; base < n; base += kLnDeltaWarps * kLnDeltaRows) {
+            // (A) the screen
+            int cnt = 0;
+#pragma unroll
+            for (int r = 0; r < kLnDeltaRows; ++r) {
+                const int b2 = base + r;
+                if (b2 >= n) break;
+                const float4 t = T2[b2];
+                if (t.x >= kLnNoMode || close_f32(fo1, fl1, t.x, t.y)) continue;
+                const float fp = fo1 + t.x, fm = fo1 - t.x, w12 = 64.26f * (fs1 + t.z), eps = 2e-6f * (fp + f3max);
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const float d = fmaxf(
+                        fminf(fminf(fabsf(fp - f3[c]), fabsf(fm + f3[c])), fabsf(fm - f3[c])) - eps, 0.f);
+                    // it 6: the velocity-difference width can cancel in FP32: not screened
+                    const bool live = W6 ? f3[c] < kLnNoMode : d * d <= w12 + w3[c];
+                    const uint32_t bal = __ballot_sync(0xffffffffu, live);
+                    if (live) Q[cnt + __popc(bal & below)] = (uint16_t)((r << 7) | (c * 32 + lane));
+                    cnt += __popc(bal);
+                }
             }
-            const int n2c = ((2 * n + 31) / 32) * 32;
-            for (int t = tid; t < n2c; t += bd) {  // warp-uniform trip count
-                const int b3 = t >> 1, h = t & 1;
-                float2 sum = make_float2(0.f, 0.f);
-                if (b3 < n)
-                    for (int r = h; r < nbb; r += 2) df_acc(sum, F[r * n + b3]);
-                sum = df_merge(sum, make_float2(__shfl_xor_sync(0xffffffffu, sum.x, 1),
-                                                __shfl_xor_sync(0xffffffffu, sum.y, 1)));
-                if (h == 0 && b3 < n) R3[b3] += (double)sum.x + (double)sum.y;
+            if (cnt == 0 && !ADJ) continue;
+            __syncwarp();
+            // (B) the survivors
+            for (int i = lane; i < cnt; i += 32) {
+                const int qv = Q[i], r = qv >> 7, b2 = base + r, b3 = qv & 127;
+                const float4 u = T2[b2], v = T3[b3];
+                float2 ps = make_float2(0.f, 0.f);
+                if (!ADJ) ps = a.psi[(((int64_t)s * n + b1) * n + b2) * n + b3];
+                float sigma;
+                if (!W6) {
+                    sigma = it == 1 ? fsig : sqrtf(fs1 + u.z + v.z);
+                } else {
+                    const double *v1 = P.vel + ((size_t)f1 * n + b1) * 3;
+                    const double *v2 = P.vel + ((size_t)q2 * n + b2) * 3, *v3 = P.vel + ((size_t)q3 * n + b3) * 3;
+                    sigma = (float)(adaptive_pair(v1, v2, P.reclat_g) / 3.0 + adaptive_pair(v1, v3, P.reclat_g) / 3.0 +
+                                    adaptive_pair(v2, v3, P.reclat_g) / 3.0 + P.thresh_sigma);
+                }
+                const float invsig = 1.0f / sigma;
+                const float win8 = 8.0f * sigma, h = 0.5f * invsig * invsig, cg = kSqrt2PiInvF * invsig;
+                // Gaussians centred at (-om2+om3, om2-om3, om2+om3, -om2-om3), get_dirac's order
+                auto gauss = [&](float s2, float s3) -> float {
+                    const float dx = centre_diff_f32(fo1, fl1, s2 * u.x, s2 * u.y, s3 * v.x, s3 * v.y);
+                    return fabsf(dx) > win8 ? 0.f : expf(-dx * dx * h) * cg;
+                };
+                const float d0 = gauss(-1.f, 1.f) - gauss(1.f, -1.f);
+                float d1 = gauss(1.f, 1.f);
+                if (fo1 + u.x + v.x <= win8 * 1.001f) d1 -= gauss(-1.f, -1.f);
+                if (close_f32(u.x, u.y, v.x, v.y)) continue;
+                const float occ = (u.w - v.w) * d0 + (u.w + v.w + 1.0f) * d1;
+                F[r * W + b3] = ADJ ? pwf * occ : pwf * fmaf(ps.x, ps.x, ps.y * ps.y) * occ;
+            }
+            __syncwarp();
+            if constexpr (ADJ) {
+                float2 *wr = a.w + ((int64_t)s * n + b1) * n * n;
+#pragma unroll
+                for (int r = 0; r < kLnDeltaRows; ++r)
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        const int b2 = base + r, b3 = c * 32 + lane;
+                        const float g = F[r * W + b3];
+                        F[r * W + b3] = 0.f;
+                        if (b2 < n && b3 < n) {
+                            const float2 ps = wr[b2 * n + b3];
+                            wr[b2 * n + b3] = make_float2(g * ps.x, -g * ps.y);
+                        }
+                    }
+                __syncwarp();
+            } else {
+                // (C) sums; F is left zero for the next rows
+                float2 rs[kLnDeltaRows];
+#pragma unroll
+                for (int r = 0; r < kLnDeltaRows; ++r) {
+                    rs[r] = make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        const float v = F[r * W + c * 32 + lane];
+                        F[r * W + c * 32 + lane] = 0.f;
+                        df_acc(col[c], v);
+                        df_acc(rs[r], v);
+                    }
+                }
+                // lanes of half h (lane / 16) go on with rows 2 h and 2 h + 1, quarters with one row
+                static_assert(kLnDeltaRows == 4, "the reduction halves four rows twice");
+                const bool up = lane & 16, up2 = lane & 8;
+                const float2 k0 = df_merge(up ? rs[2] : rs[0], df_shfl_xor(up ? rs[0] : rs[2], 16));
+                const float2 k1 = df_merge(up ? rs[3] : rs[1], df_shfl_xor(up ? rs[1] : rs[3], 16));
+                float2 k = df_merge(up2 ? k1 : k0, df_shfl_xor(up2 ? k0 : k1, 8));
+                k = df_merge(k, df_shfl_xor(k, 4));
+                k = df_merge(k, df_shfl_xor(k, 2));
+                k = df_merge(k, df_shfl_xor(k, 1));
+                const int b2 = base + (lane >> 3);
+                if ((lane & 7) == 0 && b2 < n) R2[b2] = k;
+                __syncwarp();
             }
         }
-        __syncthreads();
+        if (!ADJ)
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+                if (c * 32 + lane < n) R3[sub * n + c * 32 + lane] = col[c];
     }
     if (ADJ) return;
+    __syncthreads();
+    if (!active) return;
     const int nred = rec.red_cnt;
-    if (tid == 0) {
-        double gsum = 0.0;
-        for (int b2 = 0; b2 < n; ++b2) gsum += R2[b2];
-        if (nonzero(gsum)) atomicAdd(a.gamma + row, (double)nred * gsum);
+    if (sub == 0) {
+        float2 g = make_float2(0.f, 0.f);
+        for (int b2 = lane; b2 < n; b2 += 32) g = df_merge(g, R2[b2]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) g = df_merge(g, df_shfl_xor(g, o));
+        if (lane == 0 && (g.x != 0.f || g.y != 0.f))
+            atomicAdd(a.gamma + row, (double)nred * ((double)g.x + (double)g.y));
     }
-    const double inv1 = 1.0 / o1;
-    const int64_t ldx = (int64_t)m.n_full * n;
-    for (int i = tid; i < 2 * n * nred; i += bd) {
-        const int r = i / (2 * n), e = i % (2 * n);
-        const int2 pr = a.red[rec.red_off + r];
-        if (e < n) {
-            const double v = R2[e];
-            if (nonzero(v)) atomicAdd(a.od + row * ldx + (int64_t)pr.x * n + e, 2.0 * v * om2[e] * inv1);
-        } else {
-            const int b3 = e - n;
-            const double v = R3[b3];
-            if (nonzero(v)) atomicAdd(a.od + row * ldx + (int64_t)pr.y * n + b3, 2.0 * v * om3[b3] * inv1);
+    const double inv1 = P.inv_omega[(size_t)f1 * n + b1];
+    double *od = a.od + row * ((int64_t)m.n_full * n);
+    for (int e = sub * 32 + lane; e < 2 * n; e += 32 * kLnDeltaWarps) {
+        const bool second = e >= n;
+        const int b = second ? e - n : e;
+        float2 v = second ? R3[b] : R2[b];
+        if (second)
+            for (int j = 1; j < kLnDeltaWarps; ++j) v = df_merge(v, R3[j * n + b]);
+        if (v.x == 0.f && v.y == 0.f) continue;
+        const double x = 2.0 * ((double)v.x + (double)v.y) * P.omega[(size_t)(second ? q3 : q2) * n + b] * inv1;
+        for (int r = 0; r < nred; ++r) {
+            const int2 pr = a.red[rec.red_off + r];
+            atomicAdd(od + (int64_t)(second ? pr.y : pr.x) * n + b, x);
         }
     }
 }
@@ -810,25 +814,31 @@ LnDeltaArgs delta_args(const LnBatch &b) {
     return d;
 }
 
+template <bool ADJ, int NC, bool W6>
+cudaError_t launch_ln_delta_nc(const LnBatch &b, cudaStream_t s) {
+    const size_t dsm = ln_delta_smem(b.n, NC);
+    const dim3 grid((unsigned)((b.n + kLnDeltaB1 - 1) / kLnDeltaB1), (unsigned)b.nb);
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_ln_delta<ADJ, NC, W6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
+    if (e != cudaSuccess) return e;
+    k_ln_delta<ADJ, NC, W6><<<grid, kLnDeltaThreads, dsm, s>>>(delta_args(b));
+    return cudaGetLastError();
+}
+
+template <bool ADJ, bool W6>
+cudaError_t launch_ln_delta_w(const LnBatch &b, cudaStream_t s) {
+    switch ((b.n + 31) / 32) {
+        case 1: return launch_ln_delta_nc<ADJ, 1, W6>(b, s);
+        case 2: return launch_ln_delta_nc<ADJ, 2, W6>(b, s);
+        case 3: return launch_ln_delta_nc<ADJ, 3, W6>(b, s);
+        case 4: return launch_ln_delta_nc<ADJ, 4, W6>(b, s);
+        default: return cudaErrorNotSupported;
+    }
+}
+
 template <bool ADJ>
 cudaError_t launch_ln_delta(const LnBatch &b, cudaStream_t s) {
-    const LnDeltaArgs d = delta_args(b);
-    const int bb = b.delta_bb == 16 ? 16 : 32;
-    const size_t dsm = ln_delta_smem(b.n, bb);
-    const dim3 grid((unsigned)b.n, (unsigned)b.nb);
-    cudaError_t e;
-    if (bb == 16) {
-        if ((e = cudaFuncSetAttribute(k_ln_delta<ADJ, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm)) !=
-            cudaSuccess)
-            return e;
-        k_ln_delta<ADJ, 16><<<grid, 256, dsm, s>>>(d);
-    } else {
-        if ((e = cudaFuncSetAttribute(k_ln_delta<ADJ, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm)) !=
-            cudaSuccess)
-            return e;
-        k_ln_delta<ADJ, 32><<<grid, 256, dsm, s>>>(d);
-    }
-    return cudaGetLastError();
+    return b.ph.integrationtype == 6 ? launch_ln_delta_w<ADJ, true>(b, s) : launch_ln_delta_w<ADJ, false>(b, s);
 }
 }  // namespace
 

@@ -289,7 +289,7 @@ struct tdg_ctx {
     DevBuf<int32_t> d_deg_irr, d_dm_irr, d_chain, d_star_ptr, d_star, d_arrived;
     DevBuf<BteCtl> d_ctl;
     bool last_ln = false;  // the last tdg_scattering took the large-cell (tensor-core) path
-    int last_ln_tune = 324;  // its launch shape (delta row block * 10 + GEMM stages)
+    int last_ln_tune = 324;  // its launch shape (ln_apply_tune)
     DevBuf<__nv_bfloat16> d_bmat_t;  // transposed real-split matrices (adjoint)
     DevBuf<float> d_ghi, d_glo;      // double-float gradient accumulator (large-cell adjoint)
     int xi_fmt = -1;  // d_xi_df holds the current Xi (1) or nothing (-1)
@@ -833,7 +833,6 @@ int ln_batch_setup(tdg_ctx *c, const MeshDev &mesh, const PhononDev &ph, const R
     if (c->d_lnx.p != old) CUDA_TRY(cudaMemsetAsync(c->d_lnx.p, 0, sizeof(__nv_bfloat16) * c->d_lnx.n, s));
     const size_t slots = c->d_lnx.n / (4 * (size_t)plane);
     std::memset(&b, 0, sizeof b);  // kernel-argument bytes are compared as graph keys
-    b.delta_bb = 32;
     b.mesh = mesh;
     b.ph = ph;
     b.rows = rows;
@@ -858,13 +857,11 @@ int ln_batch_setup(tdg_ctx *c, const MeshDev &mesh, const PhononDev &ph, const R
 }
 }  // namespace
 
-// Launch shape of the large-cell path packed as one tuning value: delta row block * 10 +
-// GEMM pipeline stages.
+// Launch shape of the large-cell path as a tuning value: the last digit is the GEMM's
+// pipeline stages; the others are a shape that is no longer chosen and are kept for saved
+// decisions.
 constexpr int kLnTuneDefault = 324;
-void ln_apply_tune(LnBatch &b, int v) {
-    b.delta_bb = v / 10 == 16 ? 16 : 32;
-    b.gemm_stages = v % 10;
-}
+void ln_apply_tune(LnBatch &b, int v) { b.gemm_stages = v % 10; }
 
 bool graphs_enabled() {
     const char *p = std::getenv("TDG_GRAPHS");
@@ -1472,7 +1469,7 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
             // large-cell path: batches of q-triplets through the tcgen05 contraction
             st = ln_batch_setup(c, mesh, ph, rows, a.fc, ntrip, b, nbmax);
             if (st) return st;
-            // launch shape (delta row block, GEMM pipeline depth), timed on the first slots
+            // GEMM pipeline depth, timed on the first slots
             {
                 const std::string key = tune_key("largecell", n, o->precision, c->device);
                 int v = kLnTuneDefault;
@@ -1480,7 +1477,7 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
                 LnBatch tb = b;
                 tb.trip = c->d_trip.p;
                 tb.nb = std::min(std::min(nbmax, ntrip), 16);
-                CUDA_TRY(tune_pick(key, {324, 164, 323, 163}, kLnTuneDefault,
+                CUDA_TRY(tune_pick(key, {324, 323}, kLnTuneDefault,
                                    [&](int cand) {
                                        ln_apply_tune(tb, cand);
                                        return launch_ln_batch(tb, s);

@@ -261,7 +261,6 @@ struct LnBatch {
     int64_t plane;           // elements of one operand plane per slot: ln_kp(n) * mp
     int mp;                  // ln_mp(n): M tiles of 128 rows (8 x by 16 y) times 128
     int n_sm = 0;            // SMs of the device (persistent GEMM grid)
-    int delta_bb = 32;       // rows b2 per block of the delta kernel (16 or 32)
     int gemm_stages = 0;     // shared-memory pipeline stages of the GEMM (0: the most that fit, at most 4)
     __nv_bfloat16 *xa_hi, *xa_lo, *xb_hi, *xb_lo;  // operand planes (hi/lo), zero-initialised
     const __nv_bfloat16 *bmat;                     // launch_ln_bmat
