@@ -192,22 +192,29 @@ struct LnGemmArgs {
 //                        K = 16) into one of two tensor-memory accumulators, committed to
 //                        the stage's `empty` barrier and, after the last chunk, to the
 //                        accumulator's `afull` barrier;
-//   warps 2-9            epilogue: wait on `afull`; copy the accumulator into a padded
+//   warps 2-17           epilogue: wait on `afull`; copy the accumulator into a padded
 //                        shared-memory staging tile (warp w reads the TMEM lanes of its lane
-//                        group w % 4, warps w and w + 4 split the columns) and release it
+//                        group w % 4, the four warps of a group split the columns) and release it
 //                        (`aempty`), so that the MMAs of tile i + 2 can start; then write the
 //                        tile's outputs from the staging tile with coalesced stores: whole
 //                        2 KB runs of the next operand (hi and lo), or whole rows of Psi.
+// A tile at 120 modes takes 13 200 cycles, of which the MMAs need 5 400; shared-memory traffic
+// (MMA operands 527 KB, copies 353 KB, staging 250 KB: 8 800 cycles at 128 bytes a cycle) is
+// what bounds it now. With eight epilogue warps and index divisions for every 16-byte unit the
+// epilogue alone took 14 500 cycles, and the issuing thread's divisions and descriptors 900 a
+// tile more than it waits; 40 atoms, 4x4x4 mesh: call 32.3 -> 29.7 ms.
 // Every wait is bounded; a role that gives up sets a shared abort flag that makes the other
 // roles leave their loops (the epilogue warps decide together, through a barrier reduction,
 // so that none waits at a barrier the others have left), and the CTA drains its copies and
 // MMAs before the tensor memory is freed.
 constexpr int kLnMaxStages = 8;
-constexpr int kLnGemmThreads = 320;
+constexpr int kLnEpiWarps = 16;
+constexpr int kLnGemmThreads = 64 + 32 * kLnEpiWarps;
 constexpr uint32_t kLnTileBytes = 128u * 16u * 2u;  // one plane of one A chunk
 constexpr int kLnSmemLimit = 232448 - 1024;        // dynamic shared memory available to k_ln_gemm
 
 __device__ __forceinline__ bool ln_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
+    if (tc::mbar_try_wait(bar, parity)) return true;
     const long long t0 = clock64();
     while (!tc::mbar_try_wait(bar, parity)) {
         if (*abort_flag) return false;
@@ -219,17 +226,17 @@ __device__ __forceinline__ bool ln_wait(uint64_t *bar, uint32_t parity, volatile
     return true;
 }
 
-// Named barrier 1 over the 256 epilogue threads, with the AND of their predicates.
+// Named barrier 1 over the epilogue threads, with the AND of their predicates.
 __device__ __forceinline__ bool epi_bar_and(bool p) {
     uint32_t r;
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 1, 256, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
         : "=r"(r)
-        : "r"(p ? 1u : 0u)
+        : "r"(p ? 1u : 0u), "n"(32 * kLnEpiWarps)
         : "memory");
     return r != 0;
 }
-__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kLnEpiWarps) : "memory"); }
 
 __global__ void __launch_bounds__(kLnGemmThreads, 1) k_ln_gemm(LnGemmArgs g) {
     extern __shared__ __align__(16) unsigned char sm[];
@@ -246,6 +253,7 @@ __global__ void __launch_bounds__(kLnGemmThreads, 1) k_ln_gemm(LnGemmArgs g) {
     const int64_t bper = (int64_t)kp * kp;
     const int pitch = kp + 4;  // staging row pitch in floats: rows of consecutive lanes hit distinct banks
     float *stg = reinterpret_cast<float *>(sm + (size_t)S * stage_bytes);
+    const uint32_t ring = tc::smem_u32(sm);
 
     if (warp == 0) tc::tmem_alloc(&tbase, 2u * g.acc_cols);
     if (tid == 0) {
@@ -255,7 +263,7 @@ __global__ void __launch_bounds__(kLnGemmThreads, 1) k_ln_gemm(LnGemmArgs g) {
         }
         for (int i = 0; i < 2; ++i) {
             tc::mbar_init(&afull[i], 1);
-            tc::mbar_init(&aempty[i], 8);
+            tc::mbar_init(&aempty[i], kLnEpiWarps);
         }
         tc::mbar_init(&done, 1);
         abort_flag = 0;
@@ -268,7 +276,10 @@ __global__ void __launch_bounds__(kLnGemmThreads, 1) k_ln_gemm(LnGemmArgs g) {
 
     if (warp == 0) {
         if (lane == 0) {  // ---- producer ----
-            int it = 0;
+            // ring position st and the parity of its use; the parity before a first use is that
+            // of a phase already past, so the first round of the ring does not wait
+            int it = 0, st = 0;
+            uint32_t par = 1;
             for (int t = blockIdx.x; t < n_tiles && !abort_flag; t += gridDim.x) {
                 const int s = t / g.n_mt, mt = t % g.n_mt;
                 const TripletRec rec = g.trip[s];
@@ -277,15 +288,16 @@ __global__ void __launch_bounds__(kLnGemmThreads, 1) k_ln_gemm(LnGemmArgs g) {
                 const __nv_bfloat16 *xh = g.xhi + (int64_t)s * g.plane + (int64_t)mt * nch * 2048;
                 const __nv_bfloat16 *xl = g.xlo + (int64_t)s * g.plane + (int64_t)mt * nch * 2048;
                 for (int c = 0; c < nch; ++c, ++it) {
-                    const int st = it % S, use = it / S;
-                    if (use > 0 && !ln_wait(&empty[st], (uint32_t)((use - 1) & 1), &abort_flag)) break;
-                    unsigned char *base = sm + (size_t)st * stage_bytes;
-                    tc::mbar_arrive_expect_tx(&full[st], stage_bytes);
-                    tc::bulk_g2s(tc::smem_u32(base), xh + (int64_t)c * 2048, kLnTileBytes, &full[st]);
-                    tc::bulk_g2s(tc::smem_u32(base + kLnTileBytes), xl + (int64_t)c * 2048, kLnTileBytes, &full[st]);
-                    tc::bulk_g2s(tc::smem_u32(base + 2 * kLnTileBytes), bh + (int64_t)c * 16 * kp, b_bytes, &full[st]);
-                    tc::bulk_g2s(tc::smem_u32(base + 2 * kLnTileBytes + b_bytes), bl + (int64_t)c * 16 * kp, b_bytes,
-                                 &full[st]);
+                    if (!ln_wait(&empty[st], par, &abort_flag)) break;
+                    const uint32_t base = ring + (uint32_t)st * stage_bytes;
+                    uint64_t *bar = &full[st];
+                    tc::mbar_arrive_expect_tx(bar, stage_bytes);
+                    tc::bulk_g2s(base, xh, kLnTileBytes, bar);
+                    tc::bulk_g2s(base + kLnTileBytes, xl, kLnTileBytes, bar);
+                    tc::bulk_g2s(base + 2 * kLnTileBytes, bh, b_bytes, bar);
+                    tc::bulk_g2s(base + 2 * kLnTileBytes + b_bytes, bl, b_bytes, bar);
+                    xh += 2048, xl += 2048, bh += 16 * kp, bl += 16 * kp;
+                    if (++st == S) st = 0, par ^= 1u;
                 }
             }
             // copies still in flight land before the CTA leaves: the last fill of every stage
@@ -298,7 +310,12 @@ __global__ void __launch_bounds__(kLnGemmThreads, 1) k_ln_gemm(LnGemmArgs g) {
     } else if (warp == 1) {
         if (lane == 0) {  // ---- MMA issuer ----
             const uint32_t idesc = tc::idesc_bf16_f32(128, kp, true, true);
-            int it = 0, tl = 0;
+            // operand descriptors of ring position 0; a position further adds its byte offset / 16
+            const uint64_t dah = tc::smem_desc(ring, a_ck, 128), dal = tc::smem_desc(ring + kLnTileBytes, a_ck, 128);
+            const uint64_t dbh = tc::smem_desc(ring + 2 * kLnTileBytes, b_ck, 128);
+            const uint64_t dbl = tc::smem_desc(ring + 2 * kLnTileBytes + b_bytes, b_ck, 128);
+            int st = 0, tl = 0;
+            uint32_t par = 0;
             bool issued = false;
             for (int t = blockIdx.x; t < n_tiles && !abort_flag; t += gridDim.x, ++tl) {
                 const int buf = tl & 1, use = tl >> 1;
@@ -306,22 +323,19 @@ __global__ void __launch_bounds__(kLnGemmThreads, 1) k_ln_gemm(LnGemmArgs g) {
                 tc::fence_after_sync();
                 const uint32_t d = taddr + (uint32_t)buf * g.acc_cols;
                 bool ok = true;
-                for (int c = 0; c < nch; ++c, ++it) {
-                    const int st = it % S;
-                    if (!ln_wait(&full[st], (uint32_t)((it / S) & 1), &abort_flag)) {
+                for (int c = 0; c < nch; ++c) {
+                    if (!ln_wait(&full[st], par, &abort_flag)) {
                         ok = false;
                         break;
                     }
                     tc::fence_after_sync();
-                    const uint32_t a0 = tc::smem_u32(sm + (size_t)st * stage_bytes);
-                    const uint32_t ah = a0, al = a0 + kLnTileBytes, bh = a0 + 2 * kLnTileBytes, bl = bh + b_bytes;
-                    const uint64_t dah = tc::smem_desc(ah, a_ck, 128), dal = tc::smem_desc(al, a_ck, 128);
-                    const uint64_t dbh = tc::smem_desc(bh, b_ck, 128), dbl = tc::smem_desc(bl, b_ck, 128);
-                    tc::mma_bf16(d, dah, dbh, idesc, c > 0 ? 1u : 0u);
-                    tc::mma_bf16(d, dah, dbl, idesc, 1u);
-                    tc::mma_bf16(d, dal, dbh, idesc, 1u);
+                    const uint64_t off = (uint64_t)((uint32_t)st * (stage_bytes >> 4));
+                    tc::mma_bf16(d, dah + off, dbh + off, idesc, c > 0 ? 1u : 0u);
+                    tc::mma_bf16(d, dah + off, dbl + off, idesc, 1u);
+                    tc::mma_bf16(d, dal + off, dbh + off, idesc, 1u);
                     tc::mma_commit(&empty[st]);
                     issued = true;
+                    if (++st == S) st = 0, par ^= 1u;
                 }
                 if (!ok) break;
                 tc::mma_commit(&afull[buf]);
@@ -334,8 +348,8 @@ __global__ void __launch_bounds__(kLnGemmThreads, 1) k_ln_gemm(LnGemmArgs g) {
                 }
             }
         }
-    } else {  // ---- epilogue (warps 2-9) ----
-        const int lg = warp & 3, half = (warp - 2) >> 2, et = tid - 64;
+    } else {  // ---- epilogue (warps 2-17) ----
+        const int lg = warp & 3, part = (warp - 2) >> 2, et = tid - 64;
         const int row = 32 * lg + lane;
         int tl = 0;
         for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++tl) {
@@ -343,13 +357,13 @@ __global__ void __launch_bounds__(kLnGemmThreads, 1) k_ln_gemm(LnGemmArgs g) {
             const bool w = ln_wait(&afull[buf], (uint32_t)(use & 1), &abort_flag);
             if (!epi_bar_and(w)) break;
             tc::fence_after_sync();
-            // (1) accumulator row `row`, this warp's column half, into the staging tile
+            // (1) accumulator row `row`, this warp's quarter of the columns, into the staging tile
             const uint32_t trow = taddr + (uint32_t)buf * g.acc_cols + ((uint32_t)(32 * lg) << 16);
             float *srow = stg + (size_t)row * pitch;
-            const int c_lo = half * (kp / 2), c_hi = c_lo + kp / 2;  // kp / 2 is a multiple of 8
+            const int c_lo = (kp / 8 * part / 4) * 8, c_hi = (kp / 8 * (part + 1) / 4) * 8;
             for (int c0 = c_lo; c0 < c_hi; c0 += 16) {
-                float x[16];
                 if (c0 + 16 <= c_hi) {
+                    float x[16];
                     tc::tmem_ld16(trow + (uint32_t)c0, x);
 #pragma unroll
                     for (int i = 0; i < 16; i += 4)
@@ -373,44 +387,39 @@ __global__ void __launch_bounds__(kLnGemmThreads, 1) k_ln_gemm(LnGemmArgs g) {
             if (g.stage < 3) {
                 // D[(x, y)][ri np + w] -> X'[k' = ri np + x][position of (y, w)]: for every (ri, y half
                 // jy, w block wb) one 2 KB run of 128 units of 16 bytes, unit q = (w % 16) * 8 +
-                // x % 8 holding the 8 y of the half
-                __nv_bfloat16 *hi = g.ohi + (int64_t)s * g.plane, *lo = g.olo + (int64_t)s * g.plane;
-                const int nruns = 2 * 2 * nyb;
-                for (int u = et; u < nruns * 128; u += 256) {
-                    const int R = u >> 7, q = u & 127;
-                    const int ri = R / (2 * nyb), jy = (R / nyb) & 1, wb = R % nyb;
-                    const int xk = q & 7, w = wb * 16 + (q >> 3);
-                    const int x = x0 + xk, ya = y0 + 8 * jy;
-                    if (x >= n || w >= n || ya >= n) continue;
-                    const int kq = ri * np + x;
-                    const int64_t o = (((int64_t)((ya >> 3) * nyb + wb)) * nch + (kq >> 4)) * 2048 + ((kq >> 3) & 1) * 1024 +
-                                      (int64_t)q * 8;
-                    const float *col = stg + (size_t)(8 * 8 * jy + xk) * pitch + ri * np + w;
-                    if (ya + 8 <= n) {
+                // x % 8 holding the 8 y of the half. 128 threads per (ri, jy), over the w blocks.
+                static_assert(kLnEpiWarps == 16, "four groups of 128 threads");
+                const int ri = et >> 8, jy = (et >> 7) & 1, q = et & 127, xk = q & 7;
+                const int x = x0 + xk, ya = y0 + 8 * jy, kq = ri * np + x;
+                const int64_t o0 = (int64_t)s * g.plane + ((int64_t)((ya >> 3) * nyb) * nch + (kq >> 4)) * 2048 +
+                                   ((kq >> 3) & 1) * 1024 + (int64_t)q * 8;
+                const float *col = stg + (size_t)(64 * jy + xk) * pitch + ri * np + (q >> 3);
+                const int nw = x < n && ya < n ? (n - (q >> 3) + 15) / 16 : 0;  // w = 16 wb + q / 8 < n
+                if (ya + 8 <= n) {
+#pragma unroll 2
+                    for (int wb = 0; wb < nw; ++wb) {
                         unsigned short h[8], l[8];
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) tc::split_bf16(col[(size_t)8 * i * pitch], h[i], l[i]);
-                        *reinterpret_cast<uint4 *>(hi + o) = pack8(h);
-                        *reinterpret_cast<uint4 *>(lo + o) = pack8(l);
-                    } else {
-                        for (int i = 0; ya + i < n; ++i) store_split(hi, lo, o + i, col[(size_t)8 * i * pitch]);
+                        for (int i = 0; i < 8; ++i) tc::split_bf16(col[(size_t)8 * i * pitch + 16 * wb], h[i], l[i]);
+                        const int64_t o = o0 + (int64_t)wb * nch * 2048;
+                        *reinterpret_cast<uint4 *>(g.ohi + o) = pack8(h);
+                        *reinterpret_cast<uint4 *>(g.olo + o) = pack8(l);
                     }
+                } else {
+                    for (int wb = 0; wb < nw; ++wb)
+                        for (int i = 0; ya + i < n; ++i)
+                            store_split(g.ohi, g.olo, o0 + (int64_t)wb * nch * 2048 + i,
+                                        col[(size_t)8 * i * pitch + 16 * wb]);
                 }
             } else {
-                // Psi[(x n + y) n + b3] = (D[(x, y)][b3], D[(x, y)][np + b3]): for each x of the
-                // tile the rows y0.. are one contiguous run
-                float2 *out = g.psi + (int64_t)s * n * n * n;
+                // Psi[(x n + y) n + b3] = (D[(x, y)][b3], D[(x, y)][np + b3]): a warp per row
                 const int ny = min(16, n - y0);
-                const int per_x = ny * n;
-                for (int xk = 0; xk < 8; ++xk) {
-                    const int x = x0 + xk;
-                    if (x >= n) break;
-                    float2 *dst = out + ((int64_t)x * n + y0) * n;
-                    for (int e = et; e < per_x; e += 256) {
-                        const int yy = e / n, b3 = e - yy * n;
-                        const float *r = stg + (size_t)(yy * 8 + xk) * pitch;
-                        dst[e] = make_float2(r[b3], r[np + b3]);
-                    }
+                for (int r = warp - 2; r < 8 * ny; r += kLnEpiWarps) {
+                    const int x = x0 + (r & 7);
+                    if (x >= n) continue;
+                    float2 *dst = g.psi + (((int64_t)s * n + x) * n + y0 + (r >> 3)) * n;
+                    const float *src = stg + (size_t)r * pitch;
+                    for (int b3 = lane; b3 < n; b3 += 32) dst[b3] = make_float2(src[b3], src[np + b3]);
                 }
             }
             epi_bar();  // the staging tile is free for the next tile
