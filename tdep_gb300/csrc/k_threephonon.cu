@@ -749,19 +749,37 @@ cudaError_t launch_adj_prec(const ThreePhArgs &a, int grid, size_t extra, cudaSt
     }
 }
 
-__global__ void k_sum_slices(const double *slices, int32_t n_slice, int64_t n, double *out) {
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
-        double acc = 0.0;
-        for (int g = 0; g < n_slice; ++g) acc += slices[(int64_t)g * n + e];
-        out[e] = acc;
+// Sums of n_slice slices of `pitch` entries, 32 entries and 8 groups of slices per block (one
+// thread per entry had left most of the chip idle, and its FP64 additions bound it: 73 us for
+// 456 slices of 30 105 entries). Slices in FP32 are summed in double-float (exact to ~2^-44),
+// the groups in FP64. Quads: entry [ijk][triplet] of the tensor-core adjoint, the triplets padded
+// to a multiple of four, goes to out[27 triplet + ijk].
+template <typename T, bool Quads>
+__global__ void __launch_bounds__(256) k_sum_slices(const T *slices, int32_t n_slice, int64_t pitch, int32_t n_fc,
+                                                    double *out) {
+    __shared__ double part[8][33];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int64_t e = (int64_t)blockIdx.x * 32 + x;
+    double acc = 0.0;
+    if (e < pitch) {
+        if constexpr (sizeof(T) == sizeof(float)) {
+            float2 s = make_float2(0.f, 0.f);
+#pragma unroll 8
+            for (int g = y; g < n_slice; g += 8) df_acc(s, slices[(int64_t)g * pitch + e]);
+            acc = (double)s.x + (double)s.y;
+        } else {
+#pragma unroll 4
+            for (int g = y; g < n_slice; g += 8) acc += slices[(int64_t)g * pitch + e];
+        }
     }
-}
-
-// The same over float slices (mixed-precision adjoint).
-__global__ void k_sum_slices_f(const float *slices, int32_t n_slice, int64_t n, double *out) {
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
-        double acc = 0.0;
-        for (int g = 0; g < n_slice; ++g) acc += (double)slices[(int64_t)g * n + e];
+    part[y][x] = acc;
+    __syncthreads();
+    if (y != 0 || e >= pitch) return;
+    for (int k = 1; k < 8; ++k) acc += part[k][x];
+    if constexpr (Quads) {
+        const int64_t n4 = pitch / 27, t = e % n4;
+        if (t < n_fc) out[t * 27 + e / n4] = acc;
+    } else {
         out[e] = acc;
     }
 }
@@ -831,15 +849,18 @@ cudaError_t launch_threephonon_adjoint(const ThreePhArgs &a, int precision, int 
     return launch_adj_prec<float>(a, grid, extra, s);
 }
 
-cudaError_t launch_sum_slices(const double *slices, int32_t n_slice, int64_t n, int precision, double *out,
-                              cudaStream_t s) {
-    if (n <= 0) return cudaSuccess;
-    const int64_t blocks = (n + 255) / 256;
-    const unsigned g = (unsigned)(blocks < 4096 ? blocks : 4096);
-    if (precision == 0)
-        k_sum_slices<<<g, 256, 0, s>>>(slices, n_slice, n, out);
+cudaError_t launch_sum_slices(const double *slices, int32_t n_slice, int32_t n_fc, bool quads, int precision,
+                              double *out, cudaStream_t s) {
+    const int64_t pitch = adjoint_slice_entries(n_fc, quads);
+    if (pitch <= 0) return cudaSuccess;
+    const unsigned g = (unsigned)((pitch + 31) / 32);
+    const float *f = reinterpret_cast<const float *>(slices);
+    if (quads)
+        k_sum_slices<float, true><<<g, 256, 0, s>>>(f, n_slice, pitch, n_fc, out);
+    else if (precision == 0)
+        k_sum_slices<double, false><<<g, 256, 0, s>>>(slices, n_slice, pitch, n_fc, out);
     else
-        k_sum_slices_f<<<g, 256, 0, s>>>(reinterpret_cast<const float *>(slices), n_slice, n, out);
+        k_sum_slices<float, false><<<g, 256, 0, s>>>(f, n_slice, pitch, n_fc, out);
     return cudaGetLastError();
 }
 

@@ -78,8 +78,8 @@ constexpr long long kTcWait = 2000000000LL;  // about 1 s at 2 GHz
 //           |Psi|^2 (then the row and column sums) all in X: 55.5 KB at 15 modes and 1115
 //           force-constant triplets, 4 CTAs per SM;
 //  adjoint: the three E images at once (the back-contraction reloads them as E^T), the
-//           phase factors kept to the end for 2 Re(phase Q); queue and FP64 F in X, |Psi|^2
-//           after it (74.4 KB, 3 CTAs per SM).
+//           phase factors kept to the end for 2 Re(phase Q); queue and F in X, the Xi row
+//           terms' cotangents after it (64.5 KB, 3 CTAs per SM).
 struct TcLayout {
     size_t A, E, E3, ph, Q, F, psq, om, f32, v, masks, rowid, red, wsum, mbar, tslot, total;
 };
@@ -106,9 +106,9 @@ __host__ __device__ inline TcLayout tc_layout(int n, int nt, bool adj) {
         L.ph = L.E + 3 * kEImgBytes;
         L.E3 = L.E + 2 * kEImgBytes;
         const size_t x_end = L.ph + phb;
-        const size_t y_end = L.F + sizeof(double) * n3;
+        const size_t y_end = L.F + sizeof(float) * n3;
         o = tc_al(x_end > y_end ? x_end : y_end, 128);
-        L.psq = o; o += tc_al(sizeof(float) * n3);  // |Psi|^2, then the row and column sums (2 n^2 doubles)
+        L.psq = o; o += 2 * n2 * sizeof(double);  // the Xi row terms' cotangents
     }
     L.om = o; o += 9 * tc_al(sizeof(double) * n) + tc_al(sizeof(double) * n);  // om1..3 inv1 be2 be3 s1..3, wrow
     L.v = o; o += 3 * tc_al(sizeof(double) * 3 * n);
@@ -243,8 +243,8 @@ __global__ void __launch_bounds__(kTcThreads, ADJ ? 3 : 4) k_threephonon_tc(Thre
         S.R3 = S.R2 + N2;
         S.R2s = S.R3 + N2;
         S.R3s = S.R2s + N2;
-        S.F = ADJ ? (double *)(smem + L.F) : nullptr;
-        S.Ff = ADJ ? nullptr : (float *)(smem + L.F);
+        S.F = nullptr;
+        S.Ff = (float *)(smem + L.F);
         S.Q = (uint32_t *)(smem + L.Q);
         S.rowid = (int *)(smem + L.rowid);
         S.red = (int2 *)(smem + L.red);
@@ -415,8 +415,9 @@ __global__ void __launch_bounds__(kTcThreads, ADJ ? 3 : 4) k_threephonon_tc(Thre
                 }
             } else {
                 // row (b1, b2) of Psi over b3 -> |Psi|^2 of the valid modes
+                // (the adjoint takes Psi itself from tensor memory)
                 const int b1 = mrow >> 4, b2 = mrow & 15;
-                if (b1 < N && b2 < N) {
+                if (!ADJ && b1 < N && b2 < N) {
 #pragma unroll
                     for (int b3 = 0; b3 < N; ++b3) psq[(b1 * N + b2) * N + b3] = v[b3] * v[b3] + v[16 + b3] * v[16 + b3];
                 }
@@ -436,7 +437,7 @@ __global__ void __launch_bounds__(kTcThreads, ADJ ? 3 : 4) k_threephonon_tc(Thre
         // the forward pass reads F only where the row and column bits are set (entries written
         // by this q-triplet's survivors); the adjoint reads all of it
         if constexpr (ADJ)
-            for (int i = tid; i < N3; i += kTcThreads) S.F[i] = 0.0;
+            for (int i = tid; i < N3; i += kTcThreads) S.Ff[i] = 0.f;
         __syncthreads();
         const auto width6 = [&](int x1, int x2, int x3) { return k3_width6(S, P, x1, x2, x3); };
         if constexpr (!ADJ) {
@@ -458,11 +459,12 @@ __global__ void __launch_bounds__(kTcThreads, ADJ ? 3 : 4) k_threephonon_tc(Thre
             k3_survivors_f32<N>(S, P, 0, nq, (float)perm, width6, [](uint32_t) -> float { return 1.0f; },
                                 [&](uint32_t qv, float f) {
                                     const int idx = (int)(qv & 0xffffu);
-                                    S.F[idx] = (double)f;
-                                    if (f != 0.f) k3_mark<N>(S, idx);
+                                    S.Ff[idx] = f;
                                 });
             __syncthreads();
-            double *R2 = S.R2, *XB = S.R3;  // in the |Psi|^2 region, which the adjoint does not use
+            // the cotangents' Xi row terms as FP32 pairs, 2 om2/om1 xi_bar(q2', b2) per (b1, b2)
+            // and 2 om3/om1 xi_bar(q3', b3) per (b1, b3)
+            float2 *XA = (float2 *)(smem + L.psq), *XB = XA + N2;
             if (a.xi_bar) {
                 const int64_t ld = (int64_t)m.n_full * N;
                 for (int e = tid; e < 2 * N2; e += kTcThreads) {
@@ -475,25 +477,26 @@ __global__ void __launch_bounds__(kTcThreads, ADJ ? 3 : 4) k_threephonon_tc(Thre
                             sum += wr[(int64_t)(e < N2 ? pr.x : pr.y) * N + bb];
                         }
                     }
-                    if (e < N2)
-                        R2[x] = sum;
-                    else
-                        XB[x] = sum;
+                    XA[e] = split_df(2.0 * (e < N2 ? S.om2 : S.om3)[bb] * sum * S.inv1[eb1]);
                 }
                 __syncthreads();
             }
+            // G = cot F with cot an FP32 pair, one rounding to FP32: an FP64 product and two
+            // conversions for each of the n^3 entries had taken a 64th-rate pipe 5 000 cycles
+            // of every q-triplet
             float gw[16];
 #pragma unroll
             for (int b3 = 0; b3 < 16; ++b3) gw[b3] = 0.f;
             {
                 const int r = mine ? S.rowid[b1] : -1;
                 if (r >= 0) {
-                    const double lr = a.lam[r] * (double)nred;
+                    float2 c2 = split_df(a.lam[r] * (double)nred);
+                    if (a.xi_bar) c2 = df_merge(c2, XA[b1 * N + b2]);
 #pragma unroll
                     for (int b3 = 0; b3 < N; ++b3) {
-                        double cot = lr;
-                        if (a.xi_bar) cot += 2.0 * (S.om2[b2] * R2[b1 * N + b2] + S.om3[b3] * XB[b1 * N + b3]) * S.inv1[b1];
-                        gw[b3] = (float)(cot * S.F[(b1 * N + b2) * N + b3]);
+                        const float2 cot = a.xi_bar ? df_merge(c2, XB[b1 * N + b3]) : c2;
+                        const float f = S.Ff[(b1 * N + b2) * N + b3];
+                        gw[b3] = fmaf(cot.x, f, cot.y * f);
                     }
                 }
             }
@@ -571,17 +574,44 @@ __global__ void __launch_bounds__(kTcThreads, ADJ ? 3 : 4) k_threephonon_tc(Thre
             }
             if (!ok) break;
             __syncthreads();
+            // The CTA's gradient slice in device memory, [ijk][triplet] with the triplets padded to
+            // a multiple of four: a thread adds four triplets at a time, kBatch such quads in
+            // flight. Reading and writing the slice stays the longest part of a q-triplet, 30 500 of
+            // its 93 000 cycles (15 modes, 1115 triplets, three CTAs per SM); with eight scalar
+            // entries in flight 38 600, with one at a time the kernel took 1.85 ms instead of 1.25
+            // (12 617 q-triplets, with the FP32 pairs above).
             {
                 const float2 *Qs = (const float2 *)Aop;
-                float *slice = reinterpret_cast<float *>(a.mwm_bar) + (size_t)blockIdx.x * fc.n * 27;
-                constexpr int kGroups = kTcThreads / 27;
-                const int grp = tid / 27, ijk = tid % 27;
-                const int qoff = (ijk % 3) * N2 + ((ijk / 3) % 3) * N + ijk / 9;
-                if (grp < kGroups) {
-                    for (int tt = grp; tt < fc.n; tt += kGroups) {
-                        const float2 q = Qs[fc.abase[tt] + qoff];
-                        const float2 p = ph[tt];
-                        slice[(size_t)tt * 27 + ijk] += 2.f * (p.x * q.x - p.y * q.y);
+                const int nq = (fc.n + 3) >> 2, total = 27 * nq;
+                const float inv_nq = 1.0f / (float)nq;
+                float4 *slice = reinterpret_cast<float4 *>(a.mwm_bar) + (size_t)blockIdx.x * total;
+                constexpr int kBatch = 6;
+                for (int e0 = tid; e0 < total; e0 += kBatch * kTcThreads) {
+                    float4 g[kBatch];
+#pragma unroll
+                    for (int u = 0; u < kBatch; ++u) {
+                        const int e = e0 + u * kTcThreads;
+                        g[u] = e < total ? slice[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+#pragma unroll
+                    for (int u = 0; u < kBatch; ++u) {
+                        const int e = e0 + u * kTcThreads;
+                        if (e >= total) break;
+                        // e = ijk nq + t4; the quotient is below 27 and its distance from the next
+                        // integer at least 0.5 / nq, far above the rounding of the product
+                        const int ijk = (int)(((float)e + 0.5f) * inv_nq), t0 = 4 * (e - ijk * nq);
+                        const float2 *Qi = Qs + (ijk % 3) * N2 + ((ijk / 3) % 3) * N + ijk / 9;
+                        // the phases of the padding (t >= fc.n) are zero
+                        const float4 p01 = *(const float4 *)(ph + t0), p23 = *(const float4 *)(ph + t0 + 2);
+                        const int last = fc.n - 1;
+                        const float2 q0 = Qi[__ldg(fc.abase + t0)], q1 = Qi[__ldg(fc.abase + min(t0 + 1, last))],
+                                     q2v = Qi[__ldg(fc.abase + min(t0 + 2, last))],
+                                     q3v = Qi[__ldg(fc.abase + min(t0 + 3, last))];
+                        g[u].x += 2.f * (p01.x * q0.x - p01.y * q0.y);
+                        g[u].y += 2.f * (p01.z * q1.x - p01.w * q1.y);
+                        g[u].z += 2.f * (p23.x * q2v.x - p23.y * q2v.y);
+                        g[u].w += 2.f * (p23.z * q3v.x - p23.w * q3v.y);
+                        slice[e] = g[u];
                     }
                 }
             }

@@ -2446,17 +2446,19 @@ extern "C" int tdg_adjoint_fc3(tdg_ctx *c, const tdg_opts *o, const double *lw_b
                             : threephonon_adjoint_grid(n, o->precision, c->n_sm, ntrip, c->n_fc3, acc_smem);
     if (ntrip > 0 && grid < 1) return set_error(kErrDevice, "adjoint kernel configuration failed");
     const int64_t nm = (int64_t)c->n_fc3 * 27;
+    const size_t slice_bytes = (size_t)std::max(grid, 1) * adjoint_slice_entries(c->n_fc3, use_tc) *
+                               (o->precision == TDG_PREC_FP64 ? sizeof(double) : sizeof(float));
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t x) {
         if (e == cudaSuccess) e = x;
     };
     chk(c->d_lam.upload(lam.data(), lam.size(), s));
-    chk(c->d_slices.alloc((size_t)std::max(grid, 1) * nm));
+    chk(c->d_slices.alloc((slice_bytes + sizeof(double) - 1) / sizeof(double)));
     chk(c->d_mwm_bar.alloc(nm));
     if (e != cudaSuccess) return set_error(kErrDevice, std::string("allocation failed: ") + cudaGetErrorString(e));
     cudaEvent_t *ev = c->ev;
     CUDA_TRY(cudaEventRecord(ev[0], s));
-    CUDA_TRY(cudaMemsetAsync(c->d_slices.p, 0, sizeof(double) * (size_t)std::max(grid, 1) * nm, s));
+    CUDA_TRY(cudaMemsetAsync(c->d_slices.p, 0, slice_bytes, s));
     CUDA_TRY(cudaMemsetAsync(c->d_status.p, 0, sizeof(int32_t), s));
     ThreePhArgs a;
     std::memset(&a, 0, sizeof a);
@@ -2506,7 +2508,8 @@ extern "C" int tdg_adjoint_fc3(tdg_ctx *c, const tdg_opts *o, const double *lw_b
     else
         CUDA_TRY(launch_threephonon_adjoint(a, o->precision, grid, s));
     CUDA_TRY(cudaEventRecord(ev[2], s));
-    CUDA_TRY(launch_sum_slices(c->d_slices.p, std::max(grid, 1), nm, o->precision, c->d_mwm_bar.p, s));
+    CUDA_TRY(launch_sum_slices(c->d_slices.p, std::max(grid, 1), c->n_fc3, use_tc, o->precision, c->d_mwm_bar.p,
+                               s));
     std::vector<double> dev(nm);
     CUDA_TRY(copy_async(dev.data(), c->d_mwm_bar.p, sizeof(double) * nm, cudaMemcpyDeviceToHost, s));
     CUDA_TRY(cudaEventRecord(ev[3], s));
