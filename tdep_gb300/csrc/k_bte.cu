@@ -202,6 +202,131 @@ __global__ void k_bte_compact(int n, int64_t ld, int n_row, const BteRow *rows, 
     }
 }
 
+// ---- the products over the non-zero elements alone ----
+// Energy conservation empties most of a large mesh's Xi: a Gaussian reaches 8 sigma, and sigma
+// shrinks with the mesh (rocksalt: 21 % of the elements are not zero at 12^3, 3.2 % at 24^3;
+// perovskite 20 % at 16^3). Where few are left a row is the list of its non-zero elements, 12
+// bytes each, and the F sums are gathered, 32 bytes per column from L2: rocksalt 24^3, 75
+// iterations, call 22.9 -> 12.0 ms: an iteration takes 51 us where the dense products had
+// alone taken some 195.
+// A CTA takes an item of up to 2048 elements of a row, four gathers in flight per thread; the
+// items' sums are added in order by k_bte_update.
+__global__ void __launch_bounds__(256) k_bte_products_sparse(BteDev d) {
+    __shared__ float2 sh[8][3];
+    if (d.ctl->done) return;
+    const BteSparseItem it = d.sparse[blockIdx.x];
+    const float2 *val = d.sp_val + it.first;
+    const int32_t *col = d.sp_col + it.first;
+    const float4 *fs = d.fsum + it.fsum;
+    const int tid = threadIdx.x;
+    float2 a[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    auto term = [](float2 &s, float2 v, float fh, float fl) {
+        const float p = v.x * fh, pe = fmaf(v.x, fh, -p), cross = fmaf(v.x, fl, v.y * fh);
+        const float t = s.x + p, bb = t - s.x;
+        s.y += ((s.x - (t - bb)) + (p - bb)) + pe + cross;
+        s.x = t;
+    };
+    for (int i0 = tid; i0 < it.count; i0 += 4 * 256) {
+        float2 v[4];
+        float4 f0[4];
+        float2 f1[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = i0 + 256 * u;
+            const bool on = i < it.count;
+            v[u] = on ? __ldcs(val + i) : make_float2(0.f, 0.f);
+            const float4 *f = fs + 2 * (int64_t)(on ? __ldcs(col + i) : 0);
+            f0[u] = f[0];
+            f1[u] = *reinterpret_cast<const float2 *>(f + 1);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (i0 + 256 * u >= it.count) break;
+            term(a[0], v[u], f0[u].x, f0[u].y);
+            term(a[1], v[u], f0[u].z, f0[u].w);
+            term(a[2], v[u], f1[u].x, f1[u].y);
+        }
+    }
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        for (int o = 16; o > 0; o >>= 1)
+            a[x] = df_merge(a[x], make_float2(__shfl_xor_sync(0xffffffffu, a[x].x, o),
+                                              __shfl_xor_sync(0xffffffffu, a[x].y, o)));
+        if ((tid & 31) == 0) sh[tid >> 5][x] = a[x];
+    }
+    __syncthreads();
+    if (tid < 3) {
+        float2 s = sh[0][tid];
+        for (int w = 1; w < 8; ++w) s = df_merge(s, sh[w][tid]);
+        d.part[(int64_t)blockIdx.x * 3 + tid] = (double)s.x + (double)s.y;
+    }
+}
+
+// Element `col` of a row's (representative, mode) list.
+__device__ __forceinline__ double bte_element(const double *xr, const int32_t *rep, const BteRow &q, int n, int col) {
+    const int k = col / n;
+    return __ldcs(xr + (int64_t)rep[q.rep0 + k] * n + (col - k * n));
+}
+
+// A CTA per row; four loads in flight per thread.
+__global__ void __launch_bounds__(256) k_bte_count(int n, int64_t ld, int stride, const BteRow *rows, const int32_t *rep,
+                                                   const double *xi, int32_t *nnz) {
+    __shared__ int32_t total;
+    const int r = blockIdx.x * stride;
+    const BteRow q = rows[r];
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    int c = 0;
+#pragma unroll 4
+    for (int col = threadIdx.x; col < q.n_col; col += 256) c += bte_element(xi + (int64_t)r * ld, rep, q, n, col) != 0.0;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(&total, c);
+    __syncthreads();
+    if (threadIdx.x == 0) nnz[blockIdx.x] = total;
+}
+
+// A CTA per row, 1024 columns at a time: four consecutive blocks of 256, placed in column order.
+__global__ void __launch_bounds__(256) k_bte_sparse(int n, int64_t ld, const BteRow *rows, const int32_t *rep,
+                                                    const double *xi, const int64_t *first, float2 *val, int32_t *out) {
+    __shared__ int cnt[2][4][8];
+    const int r = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const BteRow q = rows[r];
+    int64_t at = first[r];
+    int buf = 0;
+    for (int c0 = 0; c0 < q.n_col; c0 += 1024, buf ^= 1) {
+        double v[4];
+        uint32_t bal[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int col = c0 + 256 * u + (int)threadIdx.x;
+            v[u] = col < q.n_col ? bte_element(xi + (int64_t)r * ld, rep, q, n, col) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            bal[u] = __ballot_sync(0xffffffffu, v[u] != 0.0);
+            if (lane == 0) cnt[buf][u][w] = __popc(bal[u]);
+        }
+        __syncthreads();  // the other buffer's counts were read before it
+        int total = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            int before = 0, all = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                before += j < w ? cnt[buf][u][j] : 0;
+                all += cnt[buf][u][j];
+            }
+            if (v[u] != 0.0) {
+                const int64_t k = at + total + before + __popc(bal[u] & ((1u << lane) - 1u));
+                val[k] = split_df(v[u]);
+                out[k] = c0 + 256 * u + (int)threadIdx.x;
+            }
+            total += all;
+        }
+        at += total;
+    }
+}
+
 // Points of every orbit of the groups, one orbit after another: orbit i of group g starts at
 // img_off[orb0 + i] (off: exclusive scan of the points per orbit over all q1; a q1's orbits
 // cover the mesh once).
@@ -219,7 +344,7 @@ __global__ void k_bte_images(int n_full, int n_op, const BteGroup *grp, const in
 }
 
 // F summed over the orbits of every group, as the products read it: [direction][column pair] of
-// (hi, hi, lo, lo). `lanes` consecutive threads share a column's points (a sixth of the
+// (hi, hi, lo, lo), or per column for the sparse form. `lanes` consecutive threads share a column's points (a sixth of the
 // group's operations or so each: the chain of loads is what the kernel waits for).
 __global__ void __launch_bounds__(256) k_bte_sums(BteDev d, const BteGroup *grp) {
     if (d.ctl->done) return;
@@ -247,6 +372,12 @@ __global__ void __launch_bounds__(256) k_bte_sums(BteDev d, const BteGroup *grp)
             a[x] = df_merge(a[x], v);
         }
     if (part != 0 || col >= 2 * n_pair) return;
+    if (d.n_sparse) {  // [column] of (hi, lo) of the three directions, 32 bytes
+        float4 *o = d.fsum + g.fsum / 3 * 4 + 2 * (int64_t)col;
+        o[0] = make_float4(a[0].x, a[0].y, a[1].x, a[1].y);
+        o[1] = make_float4(a[2].x, a[2].y, 0.f, 0.f);
+        return;
+    }
     float *out = reinterpret_cast<float *>(d.fsum + g.fsum + (col >> 1)) + (col & 1);
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
@@ -306,7 +437,7 @@ __global__ void k_bte_update(BteDev d) {
         fn[i] = d.fn[base + i];
         double v = 0.0;
         if (r >= 0 && !(q < kFreqTolD)) {
-            const double *p = d.part + (int64_t)r * d.split * 3 + x;
+            const double *p = d.part + (d.n_sparse ? (int64_t)d.part_first[r] : (int64_t)r * d.split) * 3 + x;
             for (int c = 0; c < d.ranges[r]; ++c) v += p[c * 3];
             v = -v / q;
         }
@@ -509,8 +640,26 @@ cudaError_t launch_bte_compact(int n, int64_t ld, int n_row, const BteRow *rows,
     return cudaGetLastError();
 }
 
+cudaError_t launch_bte_count(int n, int64_t ld, int n_row, int stride, const BteRow *rows, const int32_t *rep,
+                             const double *xi, int32_t *nnz, cudaStream_t s) {
+    if (n_row <= 0) return cudaSuccess;
+    k_bte_count<<<(n_row + stride - 1) / stride, 256, 0, s>>>(n, ld, stride, rows, rep, xi, nnz);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_bte_sparse(int n, int64_t ld, int n_row, const BteRow *rows, const int32_t *rep, const double *xi,
+                              const int64_t *first, float2 *val, int32_t *col, cudaStream_t s) {
+    if (n_row <= 0) return cudaSuccess;
+    k_bte_sparse<<<n_row, 256, 0, s>>>(n, ld, rows, rep, xi, first, val, col);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_bte_products(const BteDev &d, const BteItem *items, const int32_t *first, int n_part, const float4 *xi,
                                 cudaStream_t s) {
+    if (d.n_sparse) {
+        k_bte_products_sparse<<<d.n_sparse, 256, 0, s>>>(d);
+        return cudaGetLastError();
+    }
     if (n_part <= 0) return cudaSuccess;
     const cudaError_t e = cudaFuncSetAttribute(k_bte_products, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBteSmem);
     if (e != cudaSuccess) return e;

@@ -292,7 +292,14 @@ struct tdg_ctx {
     int last_ln_tune = 324;  // its launch shape (ln_apply_tune)
     DevBuf<__nv_bfloat16> d_bmat_t;  // transposed real-split matrices (adjoint)
     DevBuf<float> d_ghi, d_glo;      // double-float gradient accumulator (large-cell adjoint)
-    int xi_fmt = -1;  // d_xi_df holds the current Xi (1) or nothing (-1)
+    int xi_fmt = -1;  // d_xi_df holds the current Xi (1), d_sp_val and d_sp_col do (2), or nothing (-1)
+    // the sparse form of Xi (sparse_xi): elements, columns, items and the rows' partial sums
+    DevBuf<float2> d_sp_val;
+    DevBuf<int32_t> d_sp_col, d_sp_ranges, d_sp_first;
+    DevBuf<BteSparseItem> d_sp_items;
+    int n_sp_items = 0;
+    std::vector<BteRow> bte_rows;       // host copies of the rows' places and their groups' F sums
+    std::vector<int64_t> bte_row_fsum;
     // off-diagonal kappa inputs (host copies; uploaded by the first tdg_kappa_offdiag)
     std::vector<double> irr_dyngrad, atom_shift, q_full;
     std::vector<int32_t> op_fmap;
@@ -1849,6 +1856,71 @@ void symmetrize_kappa(const tdg_ctx *c, double *kappa) {
 
 }  // namespace
 
+namespace {
+// Sparse form of Xi's products: compacted matrices from kSparseBytes on (below, they stay in L2
+// and an iteration is latency; the count and its copy would cost more than they give) of which
+// less than kSparseDensity is not zero. Solves in us, sparse and dense, by the density of Xi:
+// 0.20 (perovskite 16^3) 1335 and 2053, 0.27 (perovskite 12^3) 581 and 756, 0.53 (16^3, one
+// width for all) 2140 and 1901, 0.68 (40-atom cell 4^3) 1057 and 919, 0.82 (rocksalt 24^3, one
+// width) 20 970 and 12 430.
+constexpr int64_t kSparseBytes = (int64_t)128 << 20;
+constexpr double kSparseDensity = 0.4;
+constexpr int kSparseSample = 31;  // the rows of the first estimate: every 31st, of all modes in turn
+
+// Builds the sparse form where the rule takes it; made says whether it did.
+int sparse_xi(tdg_ctx *c, bool &made) {
+    made = false;
+    const int n = c->n, nr = c->n_row;
+    const int64_t ncol = (int64_t)c->N * n;
+    cudaStream_t s = c->stream;
+    if (c->bte_n_xi * (int64_t)sizeof(float4) < kSparseBytes) return kOk;
+    DevBuf<int32_t> d_nnz;
+    CUDA_TRY(d_nnz.alloc(nr));
+    std::vector<int32_t> nnz(nr);
+    double density = 0.0;
+    // an estimate on some rows, then the count of all
+    for (int stride : {kSparseSample, 1}) {
+        const int m = (nr + stride - 1) / stride;
+        CUDA_TRY(launch_bte_count(n, ncol, nr, stride, c->d_bte_rows.p, c->orbits.rep, c->d_xi.p, d_nnz.p, s));
+        CUDA_TRY(copy_async(nnz.data(), d_nnz.p, sizeof(int32_t) * m, cudaMemcpyDeviceToHost, s));
+        CUDA_TRY(cudaStreamSynchronize(s));
+        int64_t some = 0, of = 0;
+        for (int i = 0; i < m; ++i) {
+            some += nnz[i];
+            of += c->bte_rows[(size_t)i * stride].n_col;
+        }
+        density = of ? (double)some / (double)of : 1.0;
+        if (density >= kSparseDensity) return kOk;
+    }
+    std::vector<int64_t> first(nr);
+    std::vector<int32_t> ranges(nr), part(nr);
+    std::vector<BteSparseItem> items;
+    int64_t at = 0;
+    for (int r = 0; r < nr; ++r) {
+        first[r] = at;
+        part[r] = (int32_t)items.size();
+        for (int32_t k = 0; k < nnz[r]; k += kBteSparseItem)
+            items.push_back({at + k, c->bte_row_fsum[r], std::min(kBteSparseItem, nnz[r] - k), 0});
+        ranges[r] = (int32_t)items.size() - part[r];
+        at += nnz[r];
+    }
+    if (items.empty()) return kOk;
+    DevBuf<int64_t> d_first;
+    CUDA_TRY(d_first.upload(first.data(), first.size(), s));
+    CUDA_TRY(c->d_sp_val.alloc((size_t)at));
+    CUDA_TRY(c->d_sp_col.alloc((size_t)at));
+    CUDA_TRY(c->d_sp_items.upload(items.data(), items.size(), s));
+    CUDA_TRY(c->d_sp_ranges.upload(ranges.data(), ranges.size(), s));
+    CUDA_TRY(c->d_sp_first.upload(part.data(), part.size(), s));
+    CUDA_TRY(launch_bte_sparse(n, ncol, nr, c->d_bte_rows.p, c->orbits.rep, c->d_xi.p, d_first.p, c->d_sp_val.p,
+                               c->d_sp_col.p, s));
+    CUDA_TRY(cudaStreamSynchronize(s));  // the uploads' host arrays and d_first go out of scope
+    c->n_sp_items = (int)items.size();
+    made = true;
+    return kOk;
+}
+}  // namespace
+
 extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double tol, double *kappa_sma,
                          double *kappa_iter, double *fn_out, int32_t *n_iter) {
     XferScope xs(c ? c->xfer : nullptr);
@@ -1900,17 +1972,29 @@ extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double 
             c->bte_split = pl.split;
             c->bte_groups = ng;
             c->bte_sum_threads = pl.sum_threads;
-            CUDA_TRY(c->d_fsum.alloc((size_t)pl.n_fsum));
+            CUDA_TRY(c->d_fsum.alloc((size_t)pl.n_fsum / 3 * 4));
             c->bte_n_xi = pl.n_xi;
+            c->bte_rows = pl.rows;
+            c->bte_row_fsum.assign(nr, 0);
+            for (int r = 0; r < nr; ++r)
+                for (const BteGroup &g : pl.groups)
+                    if (g.rep0 == pl.rows[r].rep0) c->bte_row_fsum[r] = g.fsum / 3 * 4;
             CUDA_TRY(c->d_bte_items.upload(pl.items.data(), pl.items.size(), s));
         }
         // the products take the representatives' columns of Xi as double-float pairs
-        if (c->xi_fmt != 1) {
+        if (c->xi_fmt < 0) {
+            bool made = false;
+            const int sst = sparse_xi(c, made);
+            if (sst) return sst;
+            if (made) c->xi_fmt = 2;
+        }
+        if (c->xi_fmt < 0) {
             CUDA_TRY(c->d_xi_df.alloc((size_t)c->bte_n_xi));
             CUDA_TRY(launch_bte_compact(n, ncol, nr, c->d_bte_rows.p, c->orbits.rep, c->d_xi.p, c->d_xi_df.p, s));
             c->xi_fmt = 1;
         }
-        CUDA_TRY(c->d_part.alloc((size_t)nr * c->bte_split * 3));
+        const bool sparse = c->xi_fmt == 2;
+        CUDA_TRY(c->d_part.alloc(sparse ? (size_t)c->n_sp_items * 3 : (size_t)nr * c->bte_split * 3));
         CUDA_TRY(c->d_fn.alloc(nfn));
         if (c->d_full_op.n == 0) {
             CUDA_TRY(c->d_full_op.upload(c->full_op.data(), N, s));
@@ -1962,7 +2046,14 @@ extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double 
         bd.sqtol = kSqTol;
         bd.split = c->bte_split;
         bd.part = c->d_part.p;
-        bd.ranges = c->d_bte_ranges.p;
+        bd.ranges = sparse ? c->d_sp_ranges.p : c->d_bte_ranges.p;
+        if (sparse) {
+            bd.n_sparse = c->n_sp_items;
+            bd.sparse = c->d_sp_items.p;
+            bd.sp_val = c->d_sp_val.p;
+            bd.sp_col = c->d_sp_col.p;
+            bd.part_first = c->d_sp_first.p;
+        }
         bd.rows_by_group = c->d_by_group.p;
         bd.img_off = c->d_img_off.p;
         bd.img = c->d_bte_img.p;

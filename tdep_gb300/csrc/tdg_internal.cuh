@@ -405,9 +405,28 @@ cudaError_t launch_bte_images(int n_full, int n_op, int n_group, int max_orb, co
 // The representatives' columns of the symmetrised Xi as double-float column pairs.
 cudaError_t launch_bte_compact(int n, int64_t ld, int n_row, const BteRow *rows, const int32_t *rep, const double *xi,
                                float4 *out, cudaStream_t s);
+// Sparse form of the representatives' columns: the non-zero elements of every row in ascending
+// column order, as (hi, lo) pairs with their column (representative x modes). An item is up to
+// kBteSparseItem elements of one row, with the group's F sums.
+constexpr int kBteSparseItem = 2048;
+struct BteSparseItem {
+    int64_t first, fsum;
+    int32_t count, unused;
+};
+// Non-zero elements of every stride-th row: nnz[i] of row i stride.
+cudaError_t launch_bte_count(int n, int64_t ld, int n_row, int stride, const BteRow *rows, const int32_t *rep,
+                             const double *xi, int32_t *nnz, cudaStream_t s);
+// The non-zero elements of row r from first[r] on.
+cudaError_t launch_bte_sparse(int n, int64_t ld, int n_row, const BteRow *rows, const int32_t *rep, const double *xi,
+                              const int64_t *first, float2 *val, int32_t *col, cudaStream_t s);
 struct BteDev {
     int32_t n_irr, n_mode, n_row, maxiter;
     int32_t split;                    // partial sums per row and direction in part
+    int32_t n_sparse;                 // items of the sparse form, 0 with the dense one
+    const BteSparseItem *sparse;
+    const float2 *sp_val;             // its elements and their columns
+    const int32_t *sp_col;
+    const int32_t *part_first;        // [n_row] first partial sum of the row (sparse form; split is not used)
     double tol, sqtol;
     double *part;                     // [n_row][split][3] partial products of Xi and fbb
     const int32_t *ranges;            // [n_row] partial sums of the row
