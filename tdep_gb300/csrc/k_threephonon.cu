@@ -249,10 +249,11 @@ __global__ void __launch_bounds__(threads_for(N), min_blocks_for(N, sizeof(R) ==
 
     // the next q-triplet's record is loaded one iteration ahead, so that the per-mode loads
     // of an iteration wait for one round trip to memory instead of two
-    TripletRec rec_next = blockIdx.x < a.n_trip ? a.trip[blockIdx.x] : TripletRec{};
-    for (int t = blockIdx.x; t < a.n_trip; t += gridDim.x) {
+    const int n_trip = a.n_trip_dev ? *a.n_trip_dev : a.n_trip;
+    TripletRec rec_next = (int)blockIdx.x < n_trip ? a.trip[blockIdx.x] : TripletRec{};
+    for (int t = blockIdx.x; t < n_trip; t += gridDim.x) {
         const TripletRec rec = rec_next;
-        if (t + (int)gridDim.x < a.n_trip) rec_next = a.trip[t + gridDim.x];
+        if (t + (int)gridDim.x < n_trip) rec_next = a.trip[t + gridDim.x];
         const int f1 = m.irr_full[rec.q1];
         const int q2 = rec.q2, q3 = rec.q3;
         const int i2 = m.full_irr[q2], i3 = m.full_irr[q3];
@@ -749,6 +750,62 @@ cudaError_t launch_adj_prec(const ThreePhArgs &a, int grid, size_t extra, cudaSt
     }
 }
 
+// The q-triplets with a mode triplet inside an 8-sigma window: a thread per q-triplet, the
+// screen of k_threephonon (a superset of it: no degeneracy rules, the windows compared as
+// squares) to the first hit. The fused kernel spends a CTA's loads and barriers on every
+// q-triplet before it knows that nothing survives, and 59 % of rocksalt 24^3 are such: call 11.3
+// -> 9.4 ms (2.0 million q-triplets, mixed); rocksalt 12^3 in FP64 1400 -> 1278 us (33 490).
+template <int N>
+__global__ void __launch_bounds__(128) k_threephonon_prescreen(ThreePhArgs a, TripletRec *live, int32_t *count) {
+    const int t = blockIdx.x * 128 + threadIdx.x, lane = threadIdx.x & 31;
+    const PhononDev &P = a.ph;
+    const MeshDev &m = a.mesh;
+    bool any = false;
+    TripletRec rec{};
+    if (t < a.n_trip) {
+        rec = a.trip[t];
+        const uint32_t mask = a.cand_mask[(size_t)rec.cand * 4];
+        const float2 *w1 = P.omega_hl + (size_t)m.irr_full[rec.q1] * N, *w2 = P.omega_hl + (size_t)rec.q2 * N,
+                     *w3 = P.omega_hl + (size_t)rec.q3 * N;
+        const bool fixed = P.integrationtype == 1;
+        const float *g1 = P.sigsq32 + (size_t)rec.q1 * N, *g2 = P.sigsq32 + (size_t)m.full_irr[rec.q2] * N,
+                    *g3 = P.sigsq32 + (size_t)m.full_irr[rec.q3] * N;
+        // 64.2 > (8 * 1.001)^2; a fixed width counts once
+        const float sf = fixed ? 64.2f * (float)P.sigma_fixed * (float)P.sigma_fixed : 0.f, sc = fixed ? 0.f : 64.2f;
+        float o2[N], o3[N], s2[N], s3[N];
+#pragma unroll
+        for (int b = 0; b < N; ++b) {
+            o2[b] = w2[b].x;
+            o3[b] = w3[b].x;
+            s2[b] = sc * g2[b];
+            s3[b] = sc * g3[b] + sf;
+        }
+        for (int b1 = 0; b1 < N && !any; ++b1) {
+            const float o1 = w1[b1].x, s1 = sc * g1[b1];
+            // NaN (omega below 1e-9 Ha) fails every comparison
+            if (!((mask >> b1) & 1u) || a.rows.rowidx[(size_t)rec.q1 * N + b1] < 0 || o1 != o1) continue;
+#pragma unroll
+            for (int b2 = 0; b2 < N; ++b2) {
+                const float p = o1 + o2[b2], d = o1 - o2[b2], s12 = s1 + s2[b2];
+#pragma unroll
+                for (int b3 = 0; b3 < N; ++b3) {
+                    // om1 + om2 + om3 is never the smallest of the four mismatches
+                    const float x = fminf(fminf(fabsf(p - o3[b3]), fabsf(d + o3[b3])), fabsf(d - o3[b3])) -
+                                    1e-6f * (p + o3[b3]);
+                    any |= x <= 0.f || x * x <= s12 + s3[b3];
+                }
+            }
+        }
+    }
+    const uint32_t bal = __ballot_sync(0xffffffffu, any);
+    int at = 0;
+    if (lane == 0 && bal) at = atomicAdd(count, __popc(bal));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (any) live[at + __popc(bal & ((1u << lane) - 1u))] = rec;
+}
+
+constexpr int64_t kPrescreenTriplets = 16384;
+
 // Sums of n_slice slices of `pitch` entries, 32 entries and 8 groups of slices per block (one
 // thread per entry had left most of the chip idle, and its FP64 additions bound it: 73 us for
 // 456 slices of 30 105 entries). Slices in FP32 are summed in double-float (exact to ~2^-44),
@@ -821,6 +878,26 @@ bool threephonon_plan_fits(int n, int n_fc) {
 
 size_t threephonon_smem_bytes(int n, int precision, int) {
     return make_layout(n, precision == 0 ? sizeof(double2) : sizeof(float2)).total;
+}
+
+// Up to 6 modes most q-triplets of a fine mesh have no survivor; from 9 modes on nearly all have one
+// (12 modes, 9^3: 99 %; 15 modes, 8^3: 99 %), and width type 6 is not screened by squares. The pass
+// gives 120 us at 33 490 q-triplets and costs a memset and a launch, some 6 us: the line is where
+// it gives several times that.
+bool threephonon_prescreen_for(int n, int integrationtype, int64_t n_trip) {
+    return (n == 3 || n == 6) && integrationtype != 6 && n_trip >= kPrescreenTriplets;
+}
+
+cudaError_t launch_threephonon_prescreen(const ThreePhArgs &a, TripletRec *live, int32_t *count, cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int32_t), s);
+    if (e != cudaSuccess || a.n_trip <= 0) return e;
+    const unsigned grid = (unsigned)((a.n_trip + 127) / 128);
+    switch (a.mesh.n_mode) {
+        case 3: k_threephonon_prescreen<3><<<grid, 128, 0, s>>>(a, live, count); break;
+        case 6: k_threephonon_prescreen<6><<<grid, 128, 0, s>>>(a, live, count); break;
+        default: return cudaErrorNotSupported;
+    }
+    return cudaGetLastError();
 }
 
 cudaError_t launch_threephonon(const ThreePhArgs &a, int precision, int n_sm, int ctas_per_sm, cudaStream_t s) {

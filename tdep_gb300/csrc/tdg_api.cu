@@ -236,6 +236,8 @@ struct tdg_ctx {
     DevBuf<unsigned long long> d_utotal;
     DevBuf<int4> d_qdesc;
     DevBuf<TripletRec> d_trip;
+    DevBuf<TripletRec> d_trip_live;  // those that may have a survivor (launch_threephonon_prescreen)
+    DevBuf<int32_t> d_live_count;
     DevBuf<int2> d_red;
     // four-phonon enumeration, samples (list a drives the symmetrisation) and kernel scratch
     DevBuf<int4> d_cand4, d_red4;
@@ -1539,9 +1541,23 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
             ta.n_trip = std::min(ntrip, std::max(ntrip / 8, 64 * c->n_sm * std::max(maxps, 1)));
             CUDA_TRY(tune_pick(key, cand, 0, [&](int v) { return fused(ta, v); }, s, cps, tuned));
             if (tuned) CUDA_TRY(rezero_outputs(c, nr, ld, s));
+            const bool pre = !use_tc && threephonon_prescreen_for(n, a.ph.integrationtype, ntrip);
+            if (pre) {
+                CUDA_TRY(c->d_trip_live.alloc((size_t)ntrip));
+                CUDA_TRY(c->d_live_count.alloc(1));
+            }
             gk << (use_tc ? "t" : "f") << cps << '/' << std::string(reinterpret_cast<const char *>(&a), sizeof a);
-            body3 = [&, fused]() { return fused(a, cps); };
-            launches += plan ? 2 : 1;
+            if (pre) gk << '/' << (const void *)c->d_trip_live.p << '/' << (const void *)c->d_live_count.p;
+            body3 = [&, fused, pre]() -> cudaError_t {
+                if (!pre) return fused(a, cps);
+                const cudaError_t ep = launch_threephonon_prescreen(a, c->d_trip_live.p, c->d_live_count.p, s);
+                if (ep != cudaSuccess) return ep;
+                ThreePhArgs la = a;
+                la.trip = c->d_trip_live.p;
+                la.n_trip_dev = c->d_live_count.p;
+                return fused(la, cps);
+            };
+            launches += (plan ? 2 : 1) + (pre ? 1 : 0);
             const int used = (cps > 0 && cps < maxps) ? cps : maxps;
             c->last_launch[0] = (int)std::min<int64_t>((int64_t)c->n_sm * used, std::max(ntrip, 1));
             c->last_launch[1] = used;

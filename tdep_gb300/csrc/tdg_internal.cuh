@@ -146,6 +146,7 @@ struct ThreePhArgs {
     Fc3Dev fc;
     const TripletRec *trip;
     int32_t n_trip;
+    const int32_t *n_trip_dev;  // not null: the number of q-triplets is here (at most n_trip)
     const int2 *red;
     const uint32_t *cand_mask;  // [n_mask*4] distinct row masks, indexed by TripletRec::cand
     double *gamma;              // [n_row]
@@ -172,6 +173,10 @@ struct ThreePhArgs {
 };
 // ctas_per_sm: persistent grid of n_sm * ctas_per_sm CTAs (0 or more than fit: as many as fit).
 cudaError_t launch_threephonon(const ThreePhArgs &a, int precision, int n_sm, int ctas_per_sm, cudaStream_t s);
+// The q-triplets of a.trip that may have a survivor, in any order, and their number (zeroed by the
+// call); for the mode counts and width types of threephonon_prescreen_for.
+bool threephonon_prescreen_for(int n, int integrationtype, int64_t n_trip);
+cudaError_t launch_threephonon_prescreen(const ThreePhArgs &a, TripletRec *live, int32_t *count, cudaStream_t s);
 // CTAs of the fused kernel per SM (resident_ctas; 0 if the configuration is not supported);
 // api and count (may be null) receive resident_ctas's two figures.
 int threephonon_max_per_sm(int n, int precision, int *api = nullptr, int *count = nullptr);
