@@ -118,53 +118,40 @@ __device__ __forceinline__ void k3_skip_masks(const K3Smem &S) {
     }
 }
 
-// Live bits of the four Gaussians of every b3 of one (b1, b2): the FP32 screen against
-// the 8-sigma window of lo_gauss with a relative margin of 1e-3 and an absolute margin far
-// above FP32 rounding (a Gaussian the screen drops is exactly 0 in the reference). Returns
-// the number of surviving mode triplets; the live bits of b3 are packed 4 per b3 into
-// lo (b3 < 8), hi (b3 < 16) and x (b3 < 18).
+// The b3 of one (b1, b2) that some Gaussian reaches, as bits: the FP32 screen against the
+// 8-sigma window of lo_gauss with a relative margin of 1e-3 and an absolute margin far above
+// FP32 rounding (a Gaussian the screen drops is exactly 0 in the reference). Which of the four
+// Gaussians is left to the survivors' own evaluation (k3_survivors_f32): here the smallest of
+// the mismatches |om1 + om2 - om3|, |om1 - om2 + om3|, |om1 - om2 - om3| (om1 + om2 + om3 is never
+// below the last) is compared by squares, a dozen instructions per mode triplet and no square
+// root, where the live bits of all four had taken three times that (perovskite 16^3: call 8.66 ->
+// 8.47 ms; 10^3 forward and backward 3174 -> 3057 us).
 template <int N>
-__device__ __forceinline__ int k3_screen(const K3Smem &S, int it, float sigfix32, int b1, int b2, uint32_t &live_lo,
-                                         uint32_t &live_hi, uint32_t &live_x) {
-    constexpr uint32_t kAll = (N >= 32) ? 0xffffffffu : ((1u << N) - 1u);
-    live_lo = live_hi = live_x = 0u;
-    int nsurv = 0;
-    const bool skip12 = S.rowid[b1] < 0 || ((S.zmask[0] | S.m12[b1]) >> b2) & 1u;
-    const uint32_t allowed = skip12 ? 0u : (kAll & ~(S.zmask[1] | S.m13[b1] | S.m23[b2]));
-    const float f_o1 = S.fo1[b1], f_o2 = S.fo2[b2];
+__device__ __forceinline__ uint32_t k3_screen(const K3Smem &S, int it, float sigfix32, int b1, int b2) {
+    constexpr uint32_t kAll = (1u << N) - 1u;
+    if (S.rowid[b1] < 0 || (((S.zmask[0] | S.m12[b1]) >> b2) & 1u)) return 0u;
+    const uint32_t allowed = kAll & ~(S.zmask[1] | S.m13[b1] | S.m23[b2]);
+    if (it == 6) return allowed;  // the -it 6 width can cancel in FP32: not screened
+    // 64.2 > (8 * 1.001)^2; a fixed width counts once
+    const float o1 = S.fo1[b1], o2 = S.fo2[b2], p = o1 + o2, d = o1 - o2;
+    const float scale = it == 1 ? 0.f : 64.2f;
+    const float w12 = it == 1 ? 64.2f * sigfix32 * sigfix32 : 64.2f * (S.fs1[b1] + S.fs2[b2]);
+    uint32_t hit = 0u;
 #pragma unroll
     for (int b3 = 0; b3 < N; ++b3) {
-        if (!((allowed >> b3) & 1u)) continue;
-        const float f_o3 = S.fo3[b3];
-        float sg = 0.f;
-        if (it == 1) sg = sigfix32;
-        else if (it == 2) sg = sqrt_screen(S.fs1[b1] + S.fs2[b2] + S.fs3[b3]);
-        const float win = 8.0f * sg * 1.001f + 1e-6f * (f_o1 + f_o2 + f_o3);
-        uint32_t live = 15u;  // the -it 6 width can cancel in FP32: not screened
-        if (it != 6) {
-            live = (fabsf(f_o1 + f_o2 - f_o3) <= win ? 1u : 0u) | (fabsf(f_o1 - f_o2 + f_o3) <= win ? 2u : 0u) |
-                   (fabsf(f_o1 - f_o2 - f_o3) <= win ? 4u : 0u) | (f_o1 + f_o2 + f_o3 <= win ? 8u : 0u);
-        }
-        if (live) {
-            ++nsurv;
-            if (b3 < 8) live_lo |= live << (4 * b3);
-            else if (b3 < 16) live_hi |= live << (4 * (b3 - 8));
-            else live_x |= live << (4 * (b3 - 16));
-        }
+        const float o3 = S.fo3[b3];
+        const float x = fmaxf(fminf(fminf(fabsf(p - o3), fabsf(d + o3)), fabsf(d - o3)) - 1e-6f * (p + o3), 0.f);
+        if (x * x <= fmaf(scale, S.fs3[b3], w12)) hit |= 1u << b3;
     }
-    return nsurv;
+    return hit & allowed;
 }
 
-// Queue entries of one (b1, b2) from its live bits, starting at position k.
+// Queue entries of the hits of one (b1, b2), starting at position k.
 template <int N>
-__device__ __forceinline__ void k3_enqueue(const K3Smem &S, int b1b2, int k, uint32_t live_lo, uint32_t live_hi,
-                                           uint32_t live_x) {
+__device__ __forceinline__ void k3_enqueue(const K3Smem &S, int b1b2, int k, uint32_t hit) {
 #pragma unroll
-    for (int b3 = 0; b3 < N; ++b3) {
-        const uint32_t live = b3 < 8 ? (live_lo >> (4 * b3)) & 15u
-                                     : (b3 < 16 ? (live_hi >> (4 * (b3 - 8))) & 15u : (live_x >> (4 * (b3 - 16))) & 15u);
-        if (live) S.Q[k++] = (uint32_t)(b1b2 * N + b3) | (live << 16);
-    }
+    for (int b3 = 0; b3 < N; ++b3)
+        if ((hit >> b3) & 1u) S.Q[k++] = (uint32_t)(b1b2 * N + b3);
 }
 
 // FP64 delta weights and occupations of the survivors q0 <= s < q1 of the queue, by full
@@ -227,8 +214,9 @@ __device__ __forceinline__ double k3_width6(const K3Smem &S, const PhononDev &P,
 // om3) from FP32 pairs (centre_diff_f32, as accurate as the FP64 difference rounded to
 // FP32), the width, the exponent and the Gaussian in FP32 (expf), the occupation factors
 // and row weight from FP32 copies made once per mode, F in FP32. Relative error of a weight about 1e-6, against the 1e-5 of the BF16x3
-// contraction.
-template <int N, typename Width6, typename PsiSq, typename Put>
+// contraction. LIVE: the entries carry their live Gaussians; otherwise those whose window holds
+// the FP32 mismatch with the screen's margins.
+template <int N, bool LIVE, typename Width6, typename PsiSq, typename Put>
 __device__ __forceinline__ void k3_survivors_f32(const K3Smem &S, const PhononDev &P, int q0, int q1, float perm,
                                                  Width6 width6, PsiSq psisq, Put put) {
     constexpr int N2 = N * N;
@@ -252,6 +240,11 @@ __device__ __forceinline__ void k3_survivors_f32(const K3Smem &S, const PhononDe
         const float invsig = 1.0f / sigma;
         const float win8 = 8.0f * sigma, h = 0.5f * invsig * invsig, cg = kSqrt2PiInvF * invsig;
         const float h1 = S.fo1[b1], l1 = S.fl1[b1], h2 = S.fo2[b2], l2 = S.fl2[b2], h3 = S.fo3[b3], l3 = S.fl3[b3];
+        if constexpr (!LIVE) {
+            const float w = win8 * 1.001f + 1e-6f * (h1 + h2 + h3);
+            live = (fabsf(h1 + h2 - h3) <= w ? 1u : 0u) | (fabsf(h1 - h2 + h3) <= w ? 2u : 0u) |
+                   (fabsf(h1 - h2 - h3) <= w ? 4u : 0u) | (h1 + h2 + h3 <= w ? 8u : 0u);
+        }
         float g[4] = {0.f, 0.f, 0.f, 0.f};
         while (live) {
             const int j = __ffs(live) - 1;

@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(threads_for(N), min_blocks_for(N, sizeof(R) ==
                 if constexpr (sizeof(R) == 8)
                     k3_survivors<N>(S, P, qstart[pass], qstart[pass + 1], perm, width6, psisq, put);
                 else
-                    k3_survivors_f32<N>(S, P, qstart[pass], qstart[pass + 1], (float)perm, width6, psisq, put);
+                    k3_survivors_f32<N, true>(S, P, qstart[pass], qstart[pass + 1], (float)perm, width6, psisq, put);
                 if (pass + 1 < PASSES) __syncthreads();  // B and the next T1 slabs
             } else {
                 // d L / d|Psi_b|^2 = lam[row(b1)] * nred * dF_b/d|Psi_b|^2 (Gamma += nred * sum F);
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(threads_for(N), min_blocks_for(N, sizeof(R) ==
                 if constexpr (sizeof(R) == 8)
                     k3_survivors<N>(S, P, qstart[pass], qstart[pass + 1], perm, width6_again, psisq, put);
                 else
-                    k3_survivors_f32<N>(S, P, qstart[pass], qstart[pass + 1], (float)perm, width6_again, psisq, put);
+                    k3_survivors_f32<N, true>(S, P, qstart[pass], qstart[pass + 1], (float)perm, width6_again, psisq, put);
             }
         }
         if constexpr (ADJ) {

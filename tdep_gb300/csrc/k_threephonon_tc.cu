@@ -426,14 +426,12 @@ __global__ void __launch_bounds__(kTcThreads, ADJ ? 3 : 4) k_threephonon_tc(Thre
         if (!ok) break;
         tc::fence_before_sync();
         // ---- FP32 screen of the Gaussians, survivors queued, FP32 weights, FP64 sums ----
-        uint32_t live_lo = 0u, live_hi = 0u, live_x = 0u;
-        int nsurv = 0;
         const int b1 = mrow >> 4, b2 = mrow & 15;
         const bool mine = b1 < N && b2 < N;
-        if (mine) nsurv = k3_screen<N>(S, it, sigfix32, b1, b2, live_lo, live_hi, live_x);
+        const uint32_t hit = mine ? k3_screen<N>(S, it, sigfix32, b1, b2) : 0u;
         int nq = 0;
-        const int off = block_exclusive_scan(nsurv, S.wsum, nq);  // contains barriers: the operands are dead
-        if (mine && nsurv) k3_enqueue<N>(S, b1 * N + b2, off, live_lo, live_hi, live_x);
+        const int off = block_exclusive_scan(__popc(hit), S.wsum, nq);  // contains barriers: the operands are dead
+        if (hit) k3_enqueue<N>(S, b1 * N + b2, off, hit);
         // the forward pass reads F only where the row and column bits are set (entries written
         // by this q-triplet's survivors); the adjoint reads all of it
         if constexpr (ADJ)
@@ -441,7 +439,7 @@ __global__ void __launch_bounds__(kTcThreads, ADJ ? 3 : 4) k_threephonon_tc(Thre
         __syncthreads();
         const auto width6 = [&](int x1, int x2, int x3) { return k3_width6(S, P, x1, x2, x3); };
         if constexpr (!ADJ) {
-            k3_survivors_f32<N>(
+            k3_survivors_f32<N, false>(
                 S, P, 0, nq, (float)perm, width6, [&](uint32_t qv) -> float { return psq[qv & 0xffffu]; },
                 [&](uint32_t qv, float f) {
                     const int idx = (int)(qv & 0xffffu);
@@ -456,7 +454,7 @@ __global__ void __launch_bounds__(kTcThreads, ADJ ? 3 : 4) k_threephonon_tc(Thre
             // equivalent triplets); W = G conj(Psi); Q[abc] = sum_b W_b E1[a,b1] E2[b,b2] E3[c,b3]
             // by three GEMMs against the real-split E^T images (W E3^T over b3, then E2^T over
             // b2, then E1^T over b1); d L / d mwm_t(i,j,k) = 2 Re(phase_t Q[3a1+i][3a2+j][3a3+k]).
-            k3_survivors_f32<N>(S, P, 0, nq, (float)perm, width6, [](uint32_t) -> float { return 1.0f; },
+            k3_survivors_f32<N, false>(S, P, 0, nq, (float)perm, width6, [](uint32_t) -> float { return 1.0f; },
                                 [&](uint32_t qv, float f) {
                                     const int idx = (int)(qv & 0xffffu);
                                     S.Ff[idx] = f;
