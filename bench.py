@@ -4,7 +4,7 @@ Default workload (the configuration the benchmark spec's targets are stated on): 5-ato
 perovskite (15 modes), 16x16x16 Gamma-centred mesh, adaptive Gaussian smearing, T = 300 K,
 seeded per-q1 q' samples of uneven sizes (200-4000 points) in one persistent launch,
 seeded Lennard-Jones + Born-Mayer force constants, mixed precision (tensor-core or FP32
-contraction, FP64 delta weights and accumulation). The same line carries the
+contraction, FP32 delta weights, FP64 accumulation). The same line carries the
 three-plus-four-phonon leg, the adjoint ratio and, as a sub-record, the 2-atom rocksalt
 24x24x24 configuration.
 
@@ -106,28 +106,26 @@ def setup(cfg_name, precision="mixed"):
     return cfg, prob, opts, lists
 
 
-# DRAM bytes (read + write) of one launch of the fused kernel, keyed by workload and path (0 the
-# SIMT kernel k_threephonon, 1 the tensor-core kernel k_threephonon_tc), from
+# DRAM bytes (read + write) of one pass of the fused kernel, with the screening pass before it
+# where there is one, keyed by workload and path (0 the SIMT kernel k_threephonon, 1 the
+# tensor-core kernel k_threephonon_tc), from
 # `ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k regex:k_threephonon`
-# on `python bench.py --profile --config <name> --steps 1 --warmup 1` (a one-pass capture),
-# summarised in profiles/. The tensor-core kernel's figure for perovskite16 is its perovskite12
-# capture (224.8 MB for 19404 q-triplets) scaled by the q-triplets of one launch (101233):
-# its traffic is the Xi row scatter, which grows with the q-triplets.
-TRAFFIC_PER_LAUNCH = {("rocksalt16", 0): 40_693_760, ("rocksalt24", 0): 460_600_000,
+# on `python bench.py --profile --config <name> --steps 1 --warmup 1` (a one-pass capture).
+TRAFFIC_PER_LAUNCH = {("rocksalt16", 0): 40_103_296, ("rocksalt24", 0): 452_435_968,
                       ("perovskite16", 0): 1_098_100_000, ("perovskite12", 1): 224_781_312,
-                      ("perovskite16", 1): 1_172_700_000}
+                      ("perovskite16", 1): 1_112_205_312}
 KERNEL_NAMES = {
-    0: "k_threephonon (fused pretransform, FP32 SIMT contraction, FP64 delta weights)",
+    0: "k_threephonon (fused pretransform, FP32 SIMT contraction of the survivors, FP32 delta weights, FP64 sums)",
     1: "k_threephonon_tc (fused pretransform, tcgen05 BF16x3 contraction with FP32 accumulation in tensor "
        "memory, FP32 delta weights, FP64 sums)",
-    2: "large-cell stage: phases, pretransform, 3 tcgen05 BF16x3 GEMM stages, FP64 delta kernel (time of the "
+    2: "large-cell stage: phases, pretransform, 3 tcgen05 BF16x3 GEMM stages, FP32 delta kernel (time of the "
        "whole stage)"}
 PRECISION_NOTES = {
-    0: "mixed: FP32 pretransform+contraction, FP64 delta weights/occupations/accumulation",
+    0: "mixed: FP32 pretransform+contraction, FP32 delta weights/occupations, FP64 sums/accumulation",
     1: "mixed: FP32 pretransform, BF16x3 tensor-core contraction with FP32 accumulation, FP32 delta weights "
-       "of the survivors (FP64 centre differences), FP64 sums/accumulation",
-    2: "mixed: FP32 pretransform, BF16x3 tensor-core contraction with FP32 accumulation, FP64 delta "
-       "weights/occupations/accumulation"}
+       "of the survivors (centre differences from FP32 pairs), FP64 sums/accumulation",
+    2: "mixed: FP32 pretransform, BF16x3 tensor-core contraction with FP32 accumulation, FP32 delta "
+       "weights/occupations, double-float block sums, FP64 accumulation"}
 
 
 class ClockSampler:
