@@ -208,7 +208,7 @@ __global__ void k_bte_compact(int n, int64_t ld, int n_row, const BteRow *rows, 
 // perovskite 20 % at 16^3). Where few are left a row is the list of its non-zero elements, 12
 // bytes each, and the F sums are gathered, 32 bytes per column from L2: rocksalt 24^3, 75
 // iterations, call 22.9 -> 12.0 ms: an iteration takes 51 us where the dense products had
-// alone taken some 195.
+// alone taken 217.
 // A CTA takes an item of up to 2048 elements of a row, four gathers in flight per thread; the
 // items' sums are added in order by k_bte_update.
 __global__ void __launch_bounds__(256) k_bte_products_sparse(BteDev d) {
@@ -278,7 +278,8 @@ __global__ void __launch_bounds__(256) k_bte_count(int n, int64_t ld, int stride
     __syncthreads();
     int c = 0;
 #pragma unroll 4
-    for (int col = threadIdx.x; col < q.n_col; col += 256) c += bte_element(xi + (int64_t)r * ld, rep, q, n, col) != 0.0;
+    for (int col = threadIdx.x; col < q.n_col; col += 256)
+        c += bte_element(xi + (int64_t)r * ld, rep, q, n, col) != 0.0;
     c = __reduce_add_sync(0xffffffffu, c);
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(&total, c);
     __syncthreads();
