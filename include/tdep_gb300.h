@@ -169,6 +169,12 @@ int tdg_check_mma(int32_t variant, int32_t n, const float *a, const float *b, fl
  * of lo_gauss inside its 8-sigma window), so tests can bound its error. */
 int tdg_check_exp(const double *t, int32_t n, double *out);
 
+/* Diagnostic, no counterpart in the reference: of the device allocations that this thread's
+ * calls on contexts make from now on, number `after` (from 0) fails as one does on a full
+ * device, once; -1 takes that back. For tests of what a call leaves behind when it runs out
+ * of memory. */
+int tdg_check_alloc_failure(int64_t after);
+
 /* Create a context on CUDA device `device` and upload the problem (replaces the
  * allocations of scattering.f90:85-212). Fails with TDG_ERR_DEVICE without a GPU. */
 int tdg_create(tdg_ctx **out, const tdg_problem *prob, int device);

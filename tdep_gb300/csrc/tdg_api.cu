@@ -50,6 +50,10 @@ thread_local std::unique_ptr<int32_t[]> tl_slist;  // shared three-phonon sample
 thread_local size_t tl_slist_cap = 0;
 thread_local cudaStream_t tl_stream = nullptr;
 thread_local cudaMemPool_t tl_pool = nullptr;
+// tdg_check_alloc_failure: allocations on this thread before the one that asks for more memory
+// than any device has, -1 none
+thread_local int64_t tl_alloc_left = -1;
+constexpr size_t kTooMuch = (size_t)1 << 50;
 
 struct PoolScope {
     cudaStream_t ps;
@@ -110,17 +114,20 @@ struct DevBuf {
         if (count <= n && p) return cudaSuccess;
         release();
         if (count == 0) count = 1;
+        const size_t bytes = tl_alloc_left >= 0 && tl_alloc_left-- == 0 ? kTooMuch : count * sizeof(T);
         cudaError_t e;
         if (tl_pool && tl_stream) {
-            e = cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), count * sizeof(T), tl_pool, tl_stream);
+            e = cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), bytes, tl_pool, tl_stream);
             if (e == cudaSuccess) st = tl_stream;
         } else {
-            e = cudaMalloc(&p, count * sizeof(T));
+            e = cudaMalloc(&p, bytes);
         }
-        if (e == cudaSuccess)
+        if (e == cudaSuccess) {
             n = count;
-        else
+        } else {
             p = nullptr;
+            cudaGetLastError();  // returned here; the next launch's check must not find it again
+        }
         return e;
     }
     cudaError_t upload(const T *h, size_t count, cudaStream_t s) {
@@ -371,6 +378,11 @@ extern "C" int tdg_check_exp(const double *t, int32_t n, double *out) {
     CUDA_TRY(dout.alloc(n));
     CUDA_TRY(launch_exp_neg_check(dt.p, n, dout.p, dtab.p, nullptr));
     CUDA_TRY(cudaMemcpy(out, dout.p, sizeof(double) * n, cudaMemcpyDeviceToHost));
+    return kOk;
+}
+
+extern "C" int tdg_check_alloc_failure(int64_t after) {
+    tl_alloc_left = after < 0 ? -1 : after;
     return kOk;
 }
 
