@@ -1375,7 +1375,8 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
             chk(c->d_cand.alloc(nc));
             int maxL = 0;
             for (const auto &d : qdesc) maxL = std::max(maxL, d.y);
-            chk(launch_build_candidates(c->d_qdesc.p, nirr, maxL, c->d_list3.p, c->d_cand.p, s));
+            if (e == cudaSuccess)
+                chk(launch_build_candidates(c->d_qdesc.p, nirr, maxL, c->d_list3.p, c->d_cand.p, s));
         }
     }
     if (o->isotope) {

@@ -1,4 +1,6 @@
 """Calls on a context whose earlier call ran out of device memory (tdg_check_alloc_failure)."""
+from itertools import count
+
 import numpy as np
 import pytest
 
@@ -27,3 +29,48 @@ def test_the_next_call_does_not_find_the_error_again(configs):
     sr.close()
     # the same non-negative sums in the order in which the device adds them
     np.testing.assert_allclose(got, ref, rtol=1e-12, atol=0)
+
+
+def run(sr, opts, lists):
+    return {"linewidth": sr.generate(opts, lists), "xi": sr.Xi}
+
+
+def every_failure(prob, opts, lists, steps=run):
+    """Fails allocation 0, 1, 2, ... of the calls in `steps`, each on a new context, until none is
+    left, and compares the same calls made again with those of a context without a failure.
+    Returns how many failed."""
+    sr = ScatteringRates(prob)
+    ref = steps(sr, opts, lists)
+    sr.close()
+    for after in count():
+        N.lib().tdg_release_cached_memory(0)  # the context before holds these calls' values in its blocks
+        sr = ScatteringRates(prob)
+        N.lib().tdg_check_alloc_failure(after)
+        try:
+            steps(sr, opts, lists)
+            failed = False
+        except N.TdgError as e:
+            assert e.code == 8
+            failed = True
+        finally:
+            N.lib().tdg_check_alloc_failure(-1)
+        if not failed:
+            sr.close()
+            return after
+        got = steps(sr, opts, lists)
+        sr.close()
+        for k, v in ref.items():
+            # FP64 sums of up to 1e4 terms in the order in which the device adds them; gradients
+            # are summed in FP32
+            tol = 1e-5 if k == "grad" else 1e-9
+            np.testing.assert_allclose(got[k], v, rtol=tol, atol=1e-2 * tol * np.abs(v).max(),
+                                       err_msg=f"{k}, allocation {after}")
+
+
+# samples that go up as they are (fcc 4^3), and one per q1 (more than 65 536 entries: fcc 10^3)
+@pytest.mark.parametrize("name,mesh,precision", [("fcc", 4, "fp64"), ("fcc", 10, "fp64"), ("rocksalt", 4, "mixed"),
+                                                 ("fluorite", 4, "mixed")])
+def test_generate_after_a_failed_allocation(configs, name, mesh, precision):
+    prob = Problem.load(configs[name], (mesh,) * 3)
+    opts = Options(precision=precision, isotopescattering=False)
+    assert every_failure(prob, opts, QLists.monte_carlo(prob, opts)) > 10
