@@ -220,6 +220,7 @@ struct tdg_ctx {
     // isotope scattering: magnitudes of the eigenvector components (first use), screen columns
     DevBuf<double> d_iso_mag;
     DevBuf<float2> d_iso_col;
+    bool iso_mag_ready = false;
     int L = 1, lmul[3] = {1, 1, 1};
     // scattering state
     int n_row = 0;
@@ -1381,9 +1382,10 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
     }
     if (o->isotope) {
         chk(c->d_iso_col.alloc((size_t)ld));
-        if (c->d_iso_mag.n == 0) {
+        if (!c->iso_mag_ready) {
             chk(c->d_iso_mag.alloc((size_t)ld * n));
             if (e == cudaSuccess) chk(launch_iso_mag(ld * n, c->d_egv.p, c->d_iso_mag.p, s));
+            c->iso_mag_ready = e == cudaSuccess;  // where an earlier step has failed it is not filled
         }
     }
     if (o->fourthorder) {

@@ -74,3 +74,10 @@ def test_generate_after_a_failed_allocation(configs, name, mesh, precision):
     prob = Problem.load(configs[name], (mesh,) * 3)
     opts = Options(precision=precision, isotopescattering=False)
     assert every_failure(prob, opts, QLists.monte_carlo(prob, opts)) > 10
+
+
+def test_isotopes_after_a_failed_allocation(configs):
+    prob = Problem.load(configs["rocksalt"], (4, 4, 4))
+    prob.mass_disorder = 1e-4 * (1.0 + np.arange(prob.n_atom))
+    opts = Options(thirdorder=False)
+    assert every_failure(prob, opts, QLists.per_irreducible(prob)) > 5
