@@ -298,6 +298,10 @@ struct tdg_ctx {
     DevBuf<double> d_scf, d_qs_bte, d_F0, d_bte_change;
     DevBuf<int32_t> d_deg_irr, d_dm_irr, d_chain, d_star_ptr, d_star, d_arrived;
     DevBuf<BteCtl> d_ctl;
+    // set once every buffer of a table is there (one alone says nothing of those after it): the
+    // operations of the full mesh, the degenerate sets and stars of tdg_kappa, the inputs of
+    // tdg_kappa_offdiag, the transposed matrices of the large-cell adjoint
+    bool full_ops_ready = false, bte_tables_ready = false, offdiag_ready = false, bmat_t_ready = false;
     bool last_ln = false;  // the last tdg_scattering took the large-cell (tensor-core) path
     int last_ln_tune = 324;  // its launch shape (ln_apply_tune)
     DevBuf<__nv_bfloat16> d_bmat_t;  // transposed real-split matrices (adjoint)
@@ -2027,15 +2031,16 @@ extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double 
         const bool sparse = c->xi_fmt == 2;
         CUDA_TRY(c->d_part.alloc(sparse ? (size_t)c->n_sp_items * 3 : (size_t)nr * c->bte_split * 3));
         CUDA_TRY(c->d_fn.alloc(nfn));
-        if (c->d_full_op.n == 0) {
+        if (!c->full_ops_ready) {
             CUDA_TRY(c->d_full_op.upload(c->full_op.data(), N, s));
             CUDA_TRY(c->d_op_cart.upload(c->op_cart.data(), c->op_cart.size(), s));
+            c->full_ops_ready = true;
         }
         // The whole iteration runs on the device (kappa.f90:382-490): the three Xi
         // products, then the scalar recurrences and the foldout (k_bte_update), in chunks of kBteChunk
         // iterations between host checks of the done flag; a chunk is replayed as a CUDA
         // graph from its second use. Fn goes up once and comes back once.
-        if (c->d_deg_irr.n == 0) {
+        if (!c->bte_tables_ready) {
             std::vector<int32_t> dg((size_t)nirr * n), dm((size_t)nirr * n * n);
             for (int q1 = 0; q1 < nirr; ++q1) {
                 const int f = c->irr_full[q1] - 1;
@@ -2056,6 +2061,7 @@ extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double 
             CUDA_TRY(c->d_chain.upload(chain.data(), chain.size(), s));
             CUDA_TRY(c->d_star_ptr.upload(sp.data(), sp.size(), s));
             CUDA_TRY(c->d_star.upload(star.data(), star.size(), s));
+            c->bte_tables_ready = true;
         }
         CUDA_TRY(c->d_scf.alloc((size_t)maxiter));
         CUDA_TRY(c->d_ctl.alloc(1));
@@ -2242,10 +2248,11 @@ int adjoint_large_cell(tdg_ctx *c, const std::vector<double> &lam, double *mwm_b
     const int n = c->n, N = c->N, ntrip = c->last_ntrip;
     const int64_t nm = (int64_t)c->n_fc3 * 27;
     CUDA_TRY(c->d_lam.upload(lam.data(), lam.size(), s));
-    if (c->d_bmat_t.n == 0) {
+    if (!c->bmat_t_ready) {
         const int kp = ln_kp(n);
         CUDA_TRY(c->d_bmat_t.alloc((size_t)N * 2 * kp * kp));
         CUDA_TRY(launch_ln_bmat(n, N, c->d_egvs32.p, c->d_bmat_t.p, true, s));
+        c->bmat_t_ready = true;
     }
     CUDA_TRY(c->d_ghi.alloc(nm));
     CUDA_TRY(c->d_glo.alloc(nm));
@@ -2675,13 +2682,13 @@ extern "C" int tdg_kappa_offdiag(tdg_ctx *c, const tdg_opts *o, double *kappa_of
     cudaStream_t s = c->stream;
     const int n = c->n, nirr = c->nirr;
     const size_t nn = (size_t)n * n;
-    if (c->d_grad.n == 0) {
+    if (!c->offdiag_ready) {
         CUDA_TRY(c->d_grad.upload(reinterpret_cast<const double2 *>(c->irr_dyngrad.data()), (size_t)nirr * 3 * nn, s));
         CUDA_TRY(c->d_shift.upload(c->atom_shift.data(), c->atom_shift.size(), s));
         CUDA_TRY(c->d_fmap.upload(c->op_fmap.data(), c->op_fmap.size(), s));
         CUDA_TRY(c->d_qfull.upload(c->q_full.data(), c->q_full.size(), s));
         CUDA_TRY(c->d_irr_weight.upload(c->irr_weight.data(), c->irr_weight.size(), s));
-        if (c->d_op_cart.n == 0) CUDA_TRY(c->d_op_cart.upload(c->op_cart.data(), c->op_cart.size(), s));
+        CUDA_TRY(c->d_op_cart.upload(c->op_cart.data(), c->op_cart.size(), s));
         // (point, operation) items of the per-operation kernels, point-major
         std::vector<int2> items;
         std::vector<int32_t> iptr(nirr + 1, 0);
@@ -2697,6 +2704,7 @@ extern "C" int tdg_kappa_offdiag(tdg_ctx *c, const tdg_opts *o, double *kappa_of
         const size_t w = offdiag_work_elems(n, nirr, c->od_items);
         if (w) CUDA_TRY(c->d_odwork.alloc(w));
         CUDA_TRY(c->d_odS.alloc((size_t)nirr * 9));
+        c->offdiag_ready = true;
     }
     // linewidths and heat capacities of the irreducible modes (kappa.f90:252-278)
     std::vector<double> lwcv(2 * (size_t)nirr * n);

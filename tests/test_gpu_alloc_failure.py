@@ -81,3 +81,17 @@ def test_isotopes_after_a_failed_allocation(configs):
     prob.mass_disorder = 1e-4 * (1.0 + np.arange(prob.n_atom))
     opts = Options(thirdorder=False)
     assert every_failure(prob, opts, QLists.per_irreducible(prob)) > 5
+
+
+def solve(sr, opts, lists):
+    out = run(sr, opts, lists)
+    out["kappa_sma"], out["kappa_iter"] = sr.kappa(opts)
+    out["kappa_offdiag"] = sr.kappa_offdiag(opts)
+    return out
+
+
+@pytest.mark.parametrize("name", ["fcc", "rocksalt"])
+def test_solve_after_a_failed_allocation(configs, name):
+    prob = Problem.load(configs[name], (4, 4, 4))
+    opts = Options(precision="mixed")
+    assert every_failure(prob, opts, QLists.monte_carlo(prob, opts), solve) > 40
