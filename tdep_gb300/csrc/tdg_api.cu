@@ -850,13 +850,14 @@ int ln_batch_setup(tdg_ctx *c, const MeshDev &mesh, const PhononDev &ph, const R
         CUDA_TRY(launch_ln_bmat(n, N, c->d_egvs32.p, c->d_bmat.p, false, s));
         c->bmat_ready = true;
     }
-    const __nv_bfloat16 *old = c->d_lnx.p;
+    // padding of the operand planes (component rows a >= n, positions with an index >= n)
+    // must read as zero; no kernel writes it. A new buffer is a larger one: its address may be
+    // that of the one before.
+    const size_t had = c->d_lnx.n;
     CUDA_TRY(c->d_lnx.alloc(4 * (size_t)plane * nbmax));
+    if (c->d_lnx.n != had) CUDA_TRY(cudaMemsetAsync(c->d_lnx.p, 0, sizeof(__nv_bfloat16) * c->d_lnx.n, s));
     CUDA_TRY(c->d_psi.alloc((size_t)nbmax * n * n * n));
     CUDA_TRY(c->d_lnph.alloc((size_t)nbmax * c->n_fc3));
-    // padding of the operand planes (component rows a >= n, positions with an index >= n)
-    // must read as zero; no kernel writes it
-    if (c->d_lnx.p != old) CUDA_TRY(cudaMemsetAsync(c->d_lnx.p, 0, sizeof(__nv_bfloat16) * c->d_lnx.n, s));
     const size_t slots = c->d_lnx.n / (4 * (size_t)plane);
     std::memset(&b, 0, sizeof b);  // kernel-argument bytes are compared as graph keys
     b.mesh = mesh;

@@ -42,6 +42,7 @@ def every_failure(prob, opts, lists, steps=run):
     sr = ScatteringRates(prob)
     ref = steps(sr, opts, lists)
     sr.close()
+    assert all(np.abs(v).max() > 0 for v in ref.values())
     for after in count():
         N.lib().tdg_release_cached_memory(0)  # the context before holds these calls' values in its blocks
         sr = ScatteringRates(prob)
@@ -95,3 +96,16 @@ def test_solve_after_a_failed_allocation(configs, name):
     prob = Problem.load(configs[name], (4, 4, 4))
     opts = Options(precision="mixed")
     assert every_failure(prob, opts, QLists.monte_carlo(prob, opts), solve) > 40
+
+
+def fit(sr, opts, lists):
+    lw = sr.generate(opts, lists)
+    return {"linewidth": lw, "xi": sr.Xi, "grad": sr.adjoint_fc3(opts, np.ones_like(lw))}
+
+
+# the fused kernels and, without symmetry, the large-cell path with padded operand planes
+@pytest.mark.parametrize("name,mesh", [("rocksalt", 4), ("fluorite", 4), ("supercell", 3)])
+def test_gradient_after_a_failed_allocation(configs, name, mesh):
+    prob = Problem.load(configs[name], (mesh,) * 3)
+    opts = Options(precision="mixed", isotopescattering=False)
+    assert every_failure(prob, opts, QLists.monte_carlo(prob, opts), fit) > 20
