@@ -271,6 +271,8 @@ int tdg_mc_qlists(const tdg_problem *prob, const tdg_opts *opts, int32_t *n_row,
  *   [9] equivalent-triplet and -quartet entries.
  * Four-phonon scattering supports up to 5 atoms (15 modes) in the primitive cell,
  * three-phonon up to 6 atoms.
+ * A call with a bad argument leaves the context's last scattering as it was. One that fails
+ * later (device memory, a kernel) leaves none: the calls that need it say so.
  */
 int tdg_scattering(tdg_ctx *ctx, const tdg_opts *opts, const tdg_qlists *lists,
                    double *linewidth, double *qs, double *stats);

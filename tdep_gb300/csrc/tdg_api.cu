@@ -240,7 +240,7 @@ struct tdg_ctx {
     DevBuf<uint32_t> d_mask;
     DevBuf<int32_t> d_nt, d_nrd, d_toff, d_roff, d_tmp, d_list3, d_rlen;
     DevBuf<int64_t> d_rbeg;
-    DevBuf<int32_t> d_row_of, d_copies, d_ucnt, d_uoff;  // union_candidates
+    DevBuf<int32_t> d_row_of, d_copies, d_ucnt, d_uoff;  // union_count, union_write
     DevBuf<unsigned long long> d_utotal;
     DevBuf<int4> d_qdesc;
     DevBuf<TripletRec> d_trip;
@@ -954,14 +954,24 @@ cudaError_t rezero_outputs(tdg_ctx *c, int64_t nr, int64_t ld, cudaStream_t s) {
 namespace {
 // Total length of the three-phonon lists up to which they go to the device as they are.
 constexpr int64_t kShortLists = 1 << 16;
-// Copies counted at a time (rows x points) by union_candidates.
+// Copies counted at a time (rows x points) by union_count.
 constexpr int64_t kUnionCounts = (int64_t)1 << 28;
+// Those kept for the next call (16 MB).
+constexpr size_t kKeptCounts = (size_t)1 << 22;
 
-// Three-phonon candidates and their row masks (d_cand, d_mask) from samples that differ
-// between the rows of a q1. row_of: first row of every q1. Nothing of the context's last
-// scattering is touched before the lists have been found good.
-int union_candidates(tdg_ctx *c, const tdg_qlists *ql, const std::vector<int> &row_of, const std::vector<int64_t> &rbeg,
-                     const std::vector<int32_t> &rlen, const std::vector<int32_t> &row_b1, int64_t &nc) {
+// Three-phonon candidates and their row masks from samples that differ between the rows of a q1:
+// union_count checks the lists and counts, union_write fills d_cand and d_mask, which the
+// adjoint of the last scattering still reads, so it comes after the last argument check.
+// row_of: first row of every q1. part: whole q1 at a time, as many as kUnionCounts holds.
+cudaError_t union_count_part(tdg_ctx *c, const std::vector<int> &row_of, const std::vector<int> &part, size_t k) {
+    const int r0 = row_of[part[k]];
+    return launch_union_count(c->N, r0, row_of[part[k + 1]] - r0, c->d_rbeg.p, c->d_rlen.p, c->d_list3.p, c->d_copies.p,
+                              c->d_status.p, c->stream);
+}
+
+int union_count(tdg_ctx *c, const tdg_qlists *ql, const std::vector<int> &row_of, const std::vector<int64_t> &rbeg,
+                const std::vector<int32_t> &rlen, const std::vector<int32_t> &row_b1, std::vector<int> &part,
+                int64_t &nc) {
     cudaStream_t s = c->stream;
     const int N = c->N, nirr = c->nirr, nr = ql->n_row;
     const int64_t all = (int64_t)nirr * N;
@@ -969,8 +979,7 @@ int union_candidates(tdg_ctx *c, const tdg_qlists *ql, const std::vector<int> &r
     auto chk = [&](cudaError_t x) {
         if (e == cudaSuccess) e = x;
     };
-    // whole q1 at a time, as many as kUnionCounts holds
-    std::vector<int> part{0};
+    part.assign(1, 0);
     int64_t most = 0;
     for (int q1 = 0; q1 < nirr; ++q1) {
         const int64_t rows = row_of[q1 + 1] - row_of[part.back()];
@@ -991,13 +1000,8 @@ int union_candidates(tdg_ctx *c, const tdg_qlists *ql, const std::vector<int> &r
     if (e != cudaSuccess) return set_error(kErrDevice, std::string("allocation/upload failed: ") + cudaGetErrorString(e));
     CUDA_TRY(cudaMemsetAsync(c->d_status.p, 0, sizeof(int32_t), s));
     CUDA_TRY(cudaMemsetAsync(c->d_utotal.p, 0, sizeof(unsigned long long), s));
-    auto count = [&](size_t k) {
-        const int r0 = row_of[part[k]];
-        return launch_union_count(N, r0, row_of[part[k + 1]] - r0, c->d_rbeg.p, c->d_rlen.p, c->d_list3.p, c->d_copies.p,
-                                  c->d_status.p, s);
-    };
     for (size_t k = 0; k + 1 < part.size(); ++k) {
-        CUDA_TRY(count(k));
+        CUDA_TRY(union_count_part(c, row_of, part, k));
         CUDA_TRY(launch_union_copies(N, part[k], part[k + 1] - part[k], row_of[part[k]], c->d_row_of.p, c->d_copies.p,
                                      c->d_ucnt.p, c->d_utotal.p, s));
     }
@@ -1011,15 +1015,21 @@ int union_candidates(tdg_ctx *c, const tdg_qlists *ql, const std::vector<int> &r
     if (total >= ((unsigned long long)1 << 31) - 1)
         return set_error(kErrBadDim, "too many three-phonon candidates for one call");
     nc = (int64_t)total;
-    chk(c->d_cand.alloc((size_t)nc));
-    chk(c->d_mask.alloc(4 * (size_t)nc));
-    if (e != cudaSuccess) return set_error(kErrDevice, std::string("allocation failed: ") + cudaGetErrorString(e));
-    for (size_t k = 0; k + 1 < part.size(); ++k) {
-        if (part.size() > 2) CUDA_TRY(count(k));  // one part: still counted
-        CUDA_TRY(launch_union_write(N, part[k], part[k + 1] - part[k], row_of[part[k]], c->d_row_of.p, c->d_row_b1.p,
-                                    c->d_copies.p, c->d_uoff.p, c->d_cand.p, c->d_mask.p, s));
-    }
     return kOk;
+}
+
+cudaError_t union_write(tdg_ctx *c, const std::vector<int> &row_of, const std::vector<int> &part, int64_t nc) {
+    cudaError_t e = c->d_cand.alloc((size_t)nc);
+    if (e == cudaSuccess) e = c->d_mask.alloc(4 * (size_t)nc);
+    for (size_t k = 0; e == cudaSuccess && k + 1 < part.size(); ++k) {
+        if (part.size() > 2) e = union_count_part(c, row_of, part, k);  // one part: still counted
+        if (e == cudaSuccess)
+            e = launch_union_write(c->N, part[k], part[k + 1] - part[k], row_of[part[k]], c->d_row_of.p, c->d_row_b1.p,
+                                   c->d_copies.p, c->d_uoff.p, c->d_cand.p, c->d_mask.p, c->stream);
+    }
+    // up to 1 GB that only these two steps use
+    if (c->d_copies.n > kKeptCounts) c->d_copies.release();
+    return e;
 }
 }  // namespace
 
@@ -1134,7 +1144,7 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
     // uploaded once per q1 and the candidates (q1, q2, mask of every row of q1) are formed
     // on the device, in sample order. Otherwise the candidates are, per q1, the union of
     // its rows' samples, with the set of rows that sampled q2 as a bit mask, formed on the
-    // device from the uploaded lists (union_candidates). A q-point that a row samples k times (the
+    // device from the uploaded lists (union_count, union_write). A q-point that a row samples k times (the
     // reference's sampler only avoids repeating the previous point, so this happens when the
     // Monte-Carlo grid does not divide the mesh) is counted k times, as the reference does:
     // the j-th copy of a candidate carries the rows that sampled the point at least j times.
@@ -1147,8 +1157,9 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
     std::vector<int4> qdesc;                // shared path: per q1 (list start, length, first candidate, mask)
     bool shared = true;
     int64_t nc64 = 0;
+    std::vector<int> qr0, part;             // rows with samples of their own: first row per q1, parts
     if (o->thirdorder) {
-        std::vector<int> qr0(nirr + 1, nr);
+        qr0.assign(nirr + 1, nr);
         for (int r = nr - 1; r >= 0; --r) qr0[rq1[r]] = r;
         for (int q1 = nirr - 1; q1 >= 0; --q1)
             if (qr0[q1] == nr) qr0[q1] = qr0[q1 + 1];
@@ -1234,7 +1245,7 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
                 rbeg[r] = ql->ptr3[r];
                 rlen[r] = (int32_t)(ql->ptr3[r + 1] - ql->ptr3[r]);
             }
-            st = union_candidates(c, ql, qr0, rbeg, rlen, rb1, nc64);
+            st = union_count(c, ql, qr0, rbeg, rlen, rb1, part, nc64);
             if (st) return st;
         }
         for (const auto &t : table) masks.insert(masks.end(), t.begin(), t.end());
@@ -1351,6 +1362,8 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
     auto chk = [&](cudaError_t x) {
         if (e == cudaSuccess) e = x;
     };
+    // from here on buffers of the last scattering are replaced: without this one's end there is none
+    c->have_scattering = false;
     chk(c->d_be.upload(be.data(), be.size(), s));
     chk(c->d_sigsq.upload(sigsq.data(), sigsq.size(), s));
     std::vector<float> sigsq32(sigsq.begin(), sigsq.end());
@@ -1383,6 +1396,8 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
             for (const auto &d : qdesc) maxL = std::max(maxL, d.y);
             if (e == cudaSuccess)
                 chk(launch_build_candidates(c->d_qdesc.p, nirr, maxL, c->d_list3.p, c->d_cand.p, s));
+        } else if (e == cudaSuccess) {
+            chk(union_write(c, qr0, part, nc64));
         }
     }
     if (o->isotope) {

@@ -109,3 +109,43 @@ def test_gradient_after_a_failed_allocation(configs, name, mesh):
     prob = Problem.load(configs[name], (mesh,) * 3)
     opts = Options(precision="mixed", isotopescattering=False)
     assert every_failure(prob, opts, QLists.monte_carlo(prob, opts), fit) > 20
+
+
+def test_gradient_of_the_scattering_before_a_failed_one(configs):
+    """Until a call replaces what the last one left, its gradient stays; from then on there is none
+    to ask for, whatever the call comes to."""
+    prob = Problem.load(configs["fluorite"], (4, 4, 4))
+    opts = Options(precision="mixed", isotopescattering=False)
+    few = QLists.per_irreducible(prob, samples3={q: np.array([1, 5, 9]) for q in range(1, prob.n_irr + 1)})
+    many = QLists.monte_carlo(prob, opts)
+    wrong = QLists.per_irreducible(prob, samples3={q: np.array([1, 5, 9]) for q in range(1, prob.n_irr + 1)})
+    wrong.list3[-1] = prob.n_full + 1
+    refused = kept = 0
+    for after in count():
+        sr = ScatteringRates(prob)
+        bar = np.ones_like(sr.generate(opts, few))
+        ref = sr.adjoint_fc3(opts, bar)
+        with pytest.raises(N.TdgError) as e:
+            sr.generate(opts, wrong)
+        assert e.value.code == 5
+        np.testing.assert_array_equal(sr.adjoint_fc3(opts, bar), ref)
+        N.lib().tdg_check_alloc_failure(after)
+        try:
+            sr.generate(opts, many)
+            failed = False
+        except N.TdgError as x:
+            assert x.code == 8
+            failed = True
+        finally:
+            N.lib().tdg_check_alloc_failure(-1)
+        if failed:
+            try:
+                np.testing.assert_array_equal(sr.adjoint_fc3(opts, bar), ref)
+                kept += 1
+            except N.TdgError as x:
+                assert x.code == 5
+                refused += 1
+        sr.close()
+        if not failed:
+            break
+    assert refused > 3 and kept > 0
