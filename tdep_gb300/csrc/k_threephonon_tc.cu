@@ -475,13 +475,13 @@ __global__ void __launch_bounds__(kTcThreads, ADJ ? 3 : 4) k_threephonon_tc(Thre
                             sum += wr[(int64_t)(e < N2 ? pr.x : pr.y) * N + bb];
                         }
                     }
-                    XA[e] = split_df(2.0 * (e < N2 ? S.om2 : S.om3)[bb] * sum * S.inv1[eb1]);
+                    XA[e] = split_df(2.0 * a.xi_bar_scale * (e < N2 ? S.om2 : S.om3)[bb] * sum * S.inv1[eb1]);
                 }
                 __syncthreads();
             }
             // G = cot F with cot an FP32 pair, one rounding to FP32: an FP64 product and two
             // conversions for each of the n^3 entries had taken a 64th-rate pipe 5 000 cycles
-            // of every q-triplet
+            // of every q-triplet. The caller keeps lam and xi_bar in the range of such pairs.
             float gw[16];
 #pragma unroll
             for (int b3 = 0; b3 < 16; ++b3) gw[b3] = 0.f;

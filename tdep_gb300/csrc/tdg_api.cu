@@ -277,6 +277,7 @@ struct tdg_ctx {
     // recomputed raw terms, and work arrays; fn_iter: c->Fn is an iterative solution
     DevBuf<double> d_xi_bar, d_od_raw, d_gam_tmp, d_zv, d_yv, d_xpart, d_tf, d_xtf;
     bool xi_bar_ready = false, fn_iter = false;
+    double xi_bar_top = 0.0;  // no element of d_xi_bar is larger
     int last_prec = 0;
     // large-cell path: real-split eigenvector matrices (built once), operand planes, Psi, phases
     DevBuf<__nv_bfloat16> d_bmat, d_lnx;
@@ -2513,6 +2514,10 @@ extern "C" int tdg_kappa_iter_vjp(tdg_ctx *c, const tdg_opts *o, const double *k
     chk(c->d_od_raw.alloc((size_t)nr * ncol));
     chk(c->d_gam_tmp.alloc((size_t)nr));
     if (e != cudaSuccess) return set_error(kErrDevice, std::string("allocation failed: ") + cudaGetErrorString(e));
+    double ztop = 0.0, ttop = 0.0;
+    for (double v : z) ztop = std::max(ztop, std::fabs(v));
+    for (double v : tf) ttop = std::max(ttop, std::fabs(v));
+    c->xi_bar_top = 3.0 * ztop * ttop;
     CUDA_TRY(copy_async(c->d_zv.p, z.data(), sizeof(double) * z.size(), cudaMemcpyHostToDevice, s));
     CUDA_TRY(cudaMemsetAsync(c->d_od_raw.p, 0, sizeof(double) * (size_t)nr * ncol, s));
     CUDA_TRY(cudaMemsetAsync(c->d_gam_tmp.p, 0, sizeof(double) * nr, s));
@@ -2585,6 +2590,17 @@ extern "C" int tdg_adjoint_fc3(tdg_ctx *c, const tdg_opts *o, const double *lw_b
     const bool use_tc = c->last_path == 1 && o->precision != TDG_PREC_FP64 && o->tensor_cores != 2 &&
                         !(tc_env && tc_env[0] == '0') && threephonon_tc_supported(n, o->precision, c->n_fc3) &&
                         c->tc_plan.slots > 0;
+    // The tensor-core adjoint takes its cotangents as FP32 pairs. The gradient is linear in them: where
+    // the largest is outside 2^+-60 they go in scaled by a power of two, which comes off in FP64.
+    int shift = 0;
+    if (use_tc) {
+        double top = c->xi_bar_ready ? c->xi_bar_top : 0.0;
+        for (double v : lam) top = std::max(top, std::fabs(v));
+        if (top > 0.0 && std::isfinite(top) && std::abs(std::ilogb(top)) > 60) {
+            shift = std::min(1000, std::max(-1000, -std::ilogb(top)));
+            for (double &v : lam) v = std::ldexp(v, shift);
+        }
+    }
     // the CTA's gradient slice lives in shared memory when it is small enough (SIMT)
     const bool acc_smem = !use_tc && (size_t)c->n_fc3 * 27 * sizeof(double) <= 48 * 1024;
     const int grid = use_tc ? threephonon_tc_adjoint_grid(n, c->n_sm, ntrip, c->n_fc3)
@@ -2630,6 +2646,7 @@ extern "C" int tdg_adjoint_fc3(tdg_ctx *c, const tdg_opts *o, const double *lw_b
     a.mwm_bar = c->d_slices.p;
     a.acc_in_smem = acc_smem ? 1 : 0;
     a.xi_bar = c->xi_bar_ready ? c->d_xi_bar.p : nullptr;
+    a.xi_bar_scale = std::ldexp(1.0, shift);
     if (use_tc) {
         if (!c->tc_eimg_t_ready) {
             CUDA_TRY(c->d_tc_eimg_t.alloc((size_t)c->N * 4096));
@@ -2663,7 +2680,10 @@ extern "C" int tdg_adjoint_fc3(tdg_ctx *c, const tdg_opts *o, const double *lw_b
     if (st) return st;
     for (int sidx = 0; sidx < c->n_fc3; ++sidx) {
         const int t = c->fc3_perm[sidx];
-        for (int k = 0; k < 27; ++k) mwm_bar[(size_t)t * 27 + k] = dev[(size_t)sidx * 27 + k];
+        for (int k = 0; k < 27; ++k) {
+            const double v = dev[(size_t)sidx * 27 + k];
+            mwm_bar[(size_t)t * 27 + k] = shift ? std::ldexp(v, -shift) : v;
+        }
     }
     if (stats) {
         float ms_all = 0.f, ms_k = 0.f;

@@ -158,6 +158,7 @@ struct ThreePhArgs {
     double *mwm_bar;            // FP64 slices, zeroed before the launch
     int32_t acc_in_smem;        // accumulate the CTA's slice in shared memory, store it once
     const double *xi_bar;       // adjoint only, may be null: cotangent of the raw three-phonon
+    double xi_bar_scale;  // power of two on xi_bar (the tensor-core adjoint; lam carries it already)
                                 // row terms of Xi ([n_row * n_full*n], tdg_kappa_iter_vjp)
     // pretransform plan of the fused kernel launched (pretransform_plan; FP32 force constants):
     // plan_slots x (its threads) values, 4 force constants per slot, and words; plan_slots 0:
