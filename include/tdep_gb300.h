@@ -223,6 +223,18 @@ int tdg_last_path(tdg_ctx *ctx, int32_t *path);
  * path. */
 int tdg_last_launch(tdg_ctx *ctx, int32_t *shape);
 
+/* Forms chosen by rules on sizes in the context's last calls (no reference counterpart):
+ * routes[0] 1 where the last tdg_scattering left q-triplets out before the fused kernel, else
+ * 0; routes[1] the parts in which it merged the samples of rows that do not share one, 0
+ * where they do; routes[2] the products of the last iterative tdg_kappa, 1 over all columns of
+ * Xi kept, 2 over the non-zero elements; -1 before such a call. */
+int tdg_last_routes(tdg_ctx *ctx, int32_t *routes);
+
+/* Diagnostic, no counterpart in the reference: the counts (rows times mesh points) up to which
+ * this context merges the samples of several rows at a time, so that a test reaches more than
+ * one part on a small mesh; 0 restores the default. */
+int tdg_check_union_counts(tdg_ctx *ctx, int64_t counts);
+
 /*
  * Launch-shape autotuner (no reference counterpart). The first scattering call that needs a
  * launch shape for its mode count, precision and device (the persistent grid of the fused

@@ -113,6 +113,7 @@ SIGNATURES = {
     "tdg_device_count": (C.c_int, []),
     "tdg_check_exp": (C.c_int, [_f64p, C.c_int32, _f64p]),
     "tdg_check_alloc_failure": (C.c_int, [C.c_int64]),
+    "tdg_check_union_counts": (C.c_int, [C.c_void_p, C.c_int64]),
     "tdg_check_mma": (C.c_int, [C.c_int32, C.c_int32, _f32p, _f32p, _f32p]),
     "tdg_create": (C.c_int, [C.POINTER(C.c_void_p), C.POINTER(TdgProblem), C.c_int]),
     "tdg_destroy": (None, [C.c_void_p]),
@@ -128,6 +129,7 @@ SIGNATURES = {
                                       _f64p]),
     "tdg_kappa_iter_vjp": (C.c_int, [C.c_void_p, C.POINTER(TdgOpts), _f64p, C.c_int32, C.c_double, _f64p, _i32p]),
     "tdg_last_path": (C.c_int, [C.c_void_p, C.POINTER(C.c_int32)]),
+    "tdg_last_routes": (C.c_int, [C.c_void_p, _i32p]),
     "tdg_last_launch": (C.c_int, [C.c_void_p, _i32p]),
     "tdg_pool_usage": (C.c_int, [C.c_int, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]),
     "tdg_natural_isotopes": (C.c_int, [C.c_char_p, C.c_int32, C.POINTER(C.c_double), C.POINTER(C.c_double)]),

@@ -212,6 +212,8 @@ struct tdg_ctx {
     // fused three-phonon launch of the last scattering call: grid, CTAs per SM used, the
     // runtime's occupancy figure and the register/shared-memory count (-1 before any)
     int last_launch[4] = {-1, -1, -1, -1};
+    int last_routes[3] = {-1, -1, -1};  // tdg_last_routes
+    int64_t union_counts = 0;           // tdg_check_union_counts, 0 for kUnionCounts
     DevBuf<double2> tw;
     DevBuf<float2> tw32;
     DevBuf<double> d_exp2tab, d_invom;
@@ -487,6 +489,18 @@ extern "C" int tdg_last_path(tdg_ctx *c, int32_t *path) {
 extern "C" int tdg_last_launch(tdg_ctx *c, int32_t *shape) {
     if (!c || !shape) return set_error(kErrParam, "tdg_last_launch: null argument");
     for (int i = 0; i < 4; ++i) shape[i] = c->last_path == 2 ? -1 : c->last_launch[i];
+    return kOk;
+}
+
+extern "C" int tdg_last_routes(tdg_ctx *c, int32_t *routes) {
+    if (!c || !routes) return set_error(kErrParam, "tdg_last_routes: null argument");
+    for (int i = 0; i < 3; ++i) routes[i] = c->last_routes[i];
+    return kOk;
+}
+
+extern "C" int tdg_check_union_counts(tdg_ctx *c, int64_t counts) {
+    if (!c || counts < 0) return set_error(kErrParam, "tdg_check_union_counts: bad argument");
+    c->union_counts = counts;
     return kOk;
 }
 
@@ -984,7 +998,7 @@ int union_count(tdg_ctx *c, const tdg_qlists *ql, const std::vector<int> &row_of
     int64_t most = 0;
     for (int q1 = 0; q1 < nirr; ++q1) {
         const int64_t rows = row_of[q1 + 1] - row_of[part.back()];
-        if (rows * N > kUnionCounts && q1 > part.back()) part.push_back(q1);
+        if (rows * N > (c->union_counts > 0 ? c->union_counts : kUnionCounts) && q1 > part.back()) part.push_back(q1);
         most = std::max<int64_t>(most, row_of[q1 + 1] - row_of[part.back()]);
     }
     part.push_back(nirr);
@@ -1365,6 +1379,8 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
     };
     // from here on buffers of the last scattering are replaced: without this one's end there is none
     c->have_scattering = false;
+    c->last_routes[0] = 0;
+    c->last_routes[1] = o->thirdorder && !shared ? (int)part.size() - 1 : 0;
     chk(c->d_be.upload(be.data(), be.size(), s));
     chk(c->d_sigsq.upload(sigsq.data(), sigsq.size(), s));
     std::vector<float> sigsq32(sigsq.begin(), sigsq.end());
@@ -1578,6 +1594,7 @@ extern "C" int tdg_scattering(tdg_ctx *c, const tdg_opts *o, const tdg_qlists *q
             CUDA_TRY(tune_pick(key, cand, 0, [&](int v) { return fused(ta, v); }, s, cps, tuned));
             if (tuned) CUDA_TRY(rezero_outputs(c, nr, ld, s));
             const bool pre = !use_tc && threephonon_prescreen_for(n, a.ph.integrationtype, ntrip);
+            c->last_routes[0] = pre ? 1 : 0;
             if (pre) {
                 CUDA_TRY(c->d_trip_live.alloc((size_t)ntrip));
                 CUDA_TRY(c->d_live_count.alloc(1));
@@ -2046,6 +2063,7 @@ extern "C" int tdg_kappa(tdg_ctx *c, const tdg_opts *o, int32_t maxiter, double 
             c->xi_fmt = 1;
         }
         const bool sparse = c->xi_fmt == 2;
+        c->last_routes[2] = c->xi_fmt;
         CUDA_TRY(c->d_part.alloc(sparse ? (size_t)c->n_sp_items * 3 : (size_t)nr * c->bte_split * 3));
         CUDA_TRY(c->d_fn.alloc(nfn));
         if (!c->full_ops_ready) {

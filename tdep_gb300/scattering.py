@@ -410,6 +410,12 @@ class ScatteringRates:
         return {"grid": int(v[0]), "ctas_per_sm": int(v[1]), "occupancy_api": int(v[2]),
                 "occupancy_count": int(v[3])}
 
+    def last_routes(self) -> dict:
+        """Forms chosen by rules on sizes in the last calls (tdg_last_routes)."""
+        v = np.zeros(3, np.int32)
+        N.check(self._lib.tdg_last_routes(self._ctx, N.ptr(v, C.c_int32)), "tdg_last_routes")
+        return {"prescreen": int(v[0]), "sample_parts": int(v[1]), "bte_products": int(v[2])}
+
     def graph_counts(self) -> list[int]:
         """Direct runs, CUDA-graph recordings and replays of the three-phonon kernels on this
         context (tdg_graph_counts)."""
