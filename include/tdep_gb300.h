@@ -269,6 +269,13 @@ int tdg_mc_qlists(const tdg_problem *prob, const tdg_opts *opts, int32_t *n_row,
                   int32_t *row_q1, int32_t *row_b1, int64_t *ptr3, int32_t *list3,
                   int64_t *ptr4, int32_t *list4a, int32_t *list4b);
 
+/* Diagnostic, no counterpart in the reference: n_row samples of tdg_mc_qlists on a grid that is the
+ * mesh ([n_row][grid[0]*grid[1]*grid[2]]) and the eight words of the stream after them. A row
+ * with a word below low_word is drawn point by point, which tdg_mc_qlists does below 2^24, once
+ * in 10^12 words; the samples do not depend on it. CPU only. */
+int tdg_check_mesh_samples(const int32_t grid[3], int32_t seed, int32_t n_row, uint64_t low_word, int32_t *list,
+                           uint64_t next[8]);
+
 /*
  * The scattering rates (scattering.f90:58-358): isotope, three-phonon, four-phonon and
  * boundary linewidths for every row, degeneracy averaging, and the symmetrised

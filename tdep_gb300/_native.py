@@ -114,6 +114,7 @@ SIGNATURES = {
     "tdg_check_exp": (C.c_int, [_f64p, C.c_int32, _f64p]),
     "tdg_check_alloc_failure": (C.c_int, [C.c_int64]),
     "tdg_check_union_counts": (C.c_int, [C.c_void_p, C.c_int64]),
+    "tdg_check_mesh_samples": (C.c_int, [_i32p, C.c_int32, C.c_int32, C.c_uint64, _i32p, C.POINTER(C.c_uint64)]),
     "tdg_check_mma": (C.c_int, [C.c_int32, C.c_int32, _f32p, _f32p, _f32p]),
     "tdg_create": (C.c_int, [C.POINTER(C.c_void_p), C.POINTER(TdgProblem), C.c_int]),
     "tdg_destroy": (None, [C.c_void_p]),

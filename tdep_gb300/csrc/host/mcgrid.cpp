@@ -115,7 +115,8 @@ void draw_grid(const McGrid &g, int32_t *out, Mt64 &rng) {
 // at on all threads. Returns the rows that are done and leaves rng at the next one's start:
 // all rows, but for one draw in 10^12. (Drawn point by point, the two million points of a
 // five-atom 12^3 mesh took 30 ms.)
-int mesh_samples(const McGrid &g, int n_row, int32_t *list, Mt64 &rng) {
+// low: 2^24 as a word, 2^-40 as a draw.
+int mesh_samples(const McGrid &g, int n_row, int32_t *list, Mt64 &rng, uint64_t low_word) {
     const int64_t words = 3 * (int64_t)g.npoints;
     const int batch = (int)std::max<int64_t>(1, (1 << 18) / words);
     constexpr int kN = Mt64::kN;
@@ -134,7 +135,7 @@ int mesh_samples(const McGrid &g, int n_row, int32_t *list, Mt64 &rng) {
         parallel_for(nr, [&](int64_t r) {
             const uint64_t *w = blocks.data() + at + r * words;
             uint64_t hit = 0;
-            for (int64_t i = 0; i < words; ++i) hit |= (uint64_t)(Mt64::temper(w[i]) < ((uint64_t)1 << 24));
+            for (int64_t i = 0; i < words; ++i) hit |= (uint64_t)(Mt64::temper(w[i]) < low_word);
             low[r] = hit != 0;
             int32_t *out = list + (r0 + r) * (int64_t)g.npoints;
             for (int q = 0; q < g.npoints; ++q) out[q] = q + 1;
@@ -148,6 +149,18 @@ int mesh_samples(const McGrid &g, int n_row, int32_t *list, Mt64 &rng) {
         if (done < nr) return r0 + done;
     }
     return n_row;
+}
+
+// The samples of n_row rows on a grid that is the mesh, rows with a low draw point by point.
+constexpr uint64_t kLowWord = (uint64_t)1 << 24;
+void mesh_lists(const McGrid &g, int n_row, int32_t *list, Mt64 &rng, uint64_t low_word) {
+    for (int first = 0; first < n_row;) {
+        first += mesh_samples(g, n_row - first, list + (size_t)first * g.npoints, rng, low_word);
+        if (first < n_row) {
+            draw_grid(g, list + (size_t)first * g.npoints, rng);
+            ++first;
+        }
+    }
 }
 
 }  // namespace
@@ -196,12 +209,9 @@ extern "C" int tdg_mc_qlists(const tdg_problem *p, const tdg_opts *o, int32_t *n
         if (o->thirdorder) ptr3[r + 1] = (int64_t)(r + 1) * g3.npoints;
         if (o->fourthorder) ptr4[r + 1] = (int64_t)(r + 1) * g4.npoints;
     }
-    while (mesh3 && first < nr) {
-        first += mesh_samples(g3, nr - first, list3 + (size_t)first * g3.npoints, rng);
-        if (first < nr) {
-            draw_grid(g3, list3 + (size_t)first * g3.npoints, rng);
-            ++first;
-        }
+    if (mesh3) {
+        mesh_lists(g3, nr, list3, rng, kLowWord);
+        first = nr;
     }
     for (int r = first; r < nr; ++r) {
         if (o->thirdorder) draw_grid(g3, list3 + (size_t)r * g3.npoints, rng);
@@ -210,5 +220,17 @@ extern "C" int tdg_mc_qlists(const tdg_problem *p, const tdg_opts *o, int32_t *n
             draw_grid(g4, list4b + (size_t)r * g4.npoints, rng);
         }
     }
+    return kOk;
+}
+
+extern "C" int tdg_check_mesh_samples(const int32_t grid[3], int32_t seed, int32_t n_row, uint64_t low_word,
+                                      int32_t *list, uint64_t next[8]) {
+    using namespace tdg;
+    if (!grid || !list || !next || n_row < 0 || grid[0] < 1 || grid[1] < 1 || grid[2] < 1 || grid[0] > 4096 ||
+        grid[1] > 4096 || grid[2] > 4096 || seed <= 0)
+        return set_error(kErrParam, "tdg_check_mesh_samples: bad argument");
+    Mt64 rng(tdep_seed_word(seed));
+    mesh_lists(make_grid(grid, grid), n_row, list, rng, low_word);
+    for (int i = 0; i < 8; ++i) next[i] = rng.next();
     return kOk;
 }
