@@ -227,7 +227,8 @@ int tdg_last_launch(tdg_ctx *ctx, int32_t *shape);
  * routes[0] 1 where the last tdg_scattering left q-triplets out before the fused kernel, else
  * 0; routes[1] the parts in which it merged the samples of rows that do not share one, 0
  * where they do; routes[2] the products of the last iterative tdg_kappa, 1 over all columns of
- * Xi kept, 2 over the non-zero elements; -1 before such a call. */
+ * Xi kept, 2 over the non-zero elements; routes[3] the q-triplets that were not left out, read
+ * from the device, -1 where routes[0] is not 1; all -1 before such a call. */
 int tdg_last_routes(tdg_ctx *ctx, int32_t *routes);
 
 /* Diagnostic, no counterpart in the reference: the counts (rows times mesh points) up to which

@@ -495,6 +495,11 @@ extern "C" int tdg_last_launch(tdg_ctx *c, int32_t *shape) {
 extern "C" int tdg_last_routes(tdg_ctx *c, int32_t *routes) {
     if (!c || !routes) return set_error(kErrParam, "tdg_last_routes: null argument");
     for (int i = 0; i < 3; ++i) routes[i] = c->last_routes[i];
+    routes[3] = -1;
+    if (c->last_routes[0] != 1 || !c->have_scattering) return kOk;
+    CUDA_TRY(cudaSetDevice(c->device));
+    CUDA_TRY(copy_async(routes + 3, c->d_live_count.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(cudaStreamSynchronize(c->stream));
     return kOk;
 }
 

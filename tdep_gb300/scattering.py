@@ -412,9 +412,9 @@ class ScatteringRates:
 
     def last_routes(self) -> dict:
         """Forms chosen by rules on sizes in the last calls (tdg_last_routes)."""
-        v = np.zeros(3, np.int32)
+        v = np.zeros(4, np.int32)
         N.check(self._lib.tdg_last_routes(self._ctx, N.ptr(v, C.c_int32)), "tdg_last_routes")
-        return {"prescreen": int(v[0]), "sample_parts": int(v[1]), "bte_products": int(v[2])}
+        return {"prescreen": int(v[0]), "sample_parts": int(v[1]), "bte_products": int(v[2]), "live_triplets": int(v[3])}
 
     def graph_counts(self) -> list[int]:
         """Direct runs, CUDA-graph recordings and replays of the three-phonon kernels on this

@@ -55,7 +55,9 @@ def test_triplets_left_out_before_the_fused_kernel(configs, name, mesh, it, take
     opts = Options(integrationtype=it, isotopescattering=False, precision=precision)
     sr = ScatteringRates(prob)
     sr.generate(opts, QLists.monte_carlo(prob, opts))
-    assert sr.last_routes()["prescreen"] == taken
+    routes = sr.last_routes()
+    assert routes["prescreen"] == taken
+    assert 0 < routes["live_triplets"] < sr.stats["triplets"] if taken else routes["live_triplets"] == -1
     sr.close()
 
 
