@@ -16,7 +16,7 @@
 // table of exp(-2 pi i K / L), L = lcm of the mesh dimensions.
 //
 // With adaptive widths few mode triplets have a Gaussian inside its 8-sigma window (2 % at
-// rocksalt 24^3, 3-12 % at 9 to 15 modes), and at two atoms 59 % of the q-triplets have none,
+// rocksalt 24^3, 3-12 % at 9 to 15 modes), and at two atoms 67 % (12^3) to 76 % (24^3) of the q-triplets have none,
 // so the screen comes before the contraction and the contraction is driven by it:
 //   1. every mode triplet and each of the four Gaussians of get_dirac is screened in FP32
 //      against the window, with a relative margin of 1e-3 and an absolute margin far above
@@ -753,8 +753,8 @@ cudaError_t launch_adj_prec(const ThreePhArgs &a, int grid, size_t extra, cudaSt
 // The q-triplets with a mode triplet inside an 8-sigma window: a thread per q-triplet, the
 // screen of k_threephonon (a superset of it: no degeneracy rules, the windows compared as
 // squares) to the first hit. The fused kernel spends a CTA's loads and barriers on every
-// q-triplet before it knows that nothing survives, and 59 % of rocksalt 24^3 are such: call 11.3
-// -> 9.4 ms (2.0 million q-triplets, mixed); rocksalt 12^3 in FP64 1400 -> 1278 us (33 490).
+// q-triplet before it knows that nothing survives, and 76 % of rocksalt 24^3 are such: device time of
+// the call 7.5..8.0 -> 5.2 ms (2.0 million q-triplets, mixed).
 template <int N>
 __global__ void __launch_bounds__(128) k_threephonon_prescreen(ThreePhArgs a, TripletRec *live, int32_t *count) {
     const int t = blockIdx.x * 128 + threadIdx.x, lane = threadIdx.x & 31;
@@ -804,7 +804,7 @@ __global__ void __launch_bounds__(128) k_threephonon_prescreen(ThreePhArgs a, Tr
     if (any) live[at + __popc(bal & ((1u << lane) - 1u))] = rec;
 }
 
-constexpr int64_t kPrescreenTriplets = 16384;
+constexpr int64_t kPrescreen6 = 16384, kPrescreen3 = 1 << 20;
 
 // Sums of n_slice slices of `pitch` entries, 32 entries and 8 groups of slices per block (one
 // thread per entry had left most of the chip idle, and its FP64 additions bound it: 73 us for
@@ -880,12 +880,21 @@ size_t threephonon_smem_bytes(int n, int precision, int) {
     return make_layout(n, precision == 0 ? sizeof(double2) : sizeof(float2)).total;
 }
 
-// Up to 6 modes most q-triplets of a fine mesh have no survivor; from 9 modes on nearly all have one
-// (12 modes, 9^3: 99 %; 15 modes, 8^3: 99 %), and width type 6 is not screened by squares. The pass
-// gives 120 us at 33 490 q-triplets and costs a memset and a launch, some 6 us: the line is where
-// it gives several times that.
+// From 9 modes on nearly all q-triplets have a survivor (12 modes, 9^3: 99 %; 15 modes, 8^3: 99 %),
+// and width type 6 is not screened by squares. Device time of the call in us, without and with
+// the pass:
+//   6 modes, adaptive  3 260 q-triplets (42 % left): FP64 246, 214; mixed 158, 153
+//                     11 620 (37 %): 426, 374; 210, 180.  33 490 (33 %): 804, 710; 325, 264
+//                    181 902 (29 %): 3031, 2750; 984, 731.  2.0 million (24 %): 24 640, 23 800; 7745, 5190
+//   6 modes, one width  3 260 (85 %): 290, 290; 159, 165.  33 490 (85 %): 1657, 1564; 418, 395
+//   3 modes, adaptive 82 611 (48 %): 894, 884; 432, 436.  365 333 (43 %): 3250, 3250; 1400, 1428
+//                      2.0 million (39 %): 15 790, 15 000; 6790, 6490
+//   3 modes, one width, none left out: 82 611: 1721, 1718; 790, 797
+// so at 6 modes from some 16 000 q-triplets on, at 3 modes, where the fused kernel's loads and
+// barriers are few, with adaptive widths from a million on.
 bool threephonon_prescreen_for(int n, int integrationtype, int64_t n_trip) {
-    return (n == 3 || n == 6) && integrationtype != 6 && n_trip >= kPrescreenTriplets;
+    if (n == 6) return integrationtype != 6 && n_trip >= kPrescreen6;
+    return n == 3 && integrationtype == 2 && n_trip >= kPrescreen3;
 }
 
 cudaError_t launch_threephonon_prescreen(const ThreePhArgs &a, TripletRec *live, int32_t *count, cudaStream_t s) {

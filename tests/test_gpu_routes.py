@@ -46,9 +46,11 @@ def test_one_context_from_sparse_to_dense_products_and_back(configs):
     shared.close()
 
 
-# 16 384 q-triplets and more at 3 and 6 modes, fixed and adaptive widths; fewer; width type 6; 9 modes
-@pytest.mark.parametrize("name,mesh,it,taken", [("rocksalt", 12, 2, 1), ("rocksalt", 12, 1, 1), ("fcc", 14, 2, 1),
-                                                ("rocksalt", 6, 2, 0), ("rocksalt", 12, 6, 0), ("fluorite", 12, 2, 0)])
+# 16 384 q-triplets and more at 6 modes, fixed and adaptive widths; fewer; width type 6; a million and
+# more at 3 modes, adaptive widths; fewer; one width; 9 modes
+@pytest.mark.parametrize("name,mesh,it,taken", [("rocksalt", 12, 2, 1), ("rocksalt", 12, 1, 1), ("rocksalt", 6, 2, 0),
+                                                ("rocksalt", 12, 6, 0), ("fcc", 23, 2, 1), ("fcc", 14, 2, 0),
+                                                ("fcc", 23, 1, 0), ("fluorite", 12, 2, 0)])
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_triplets_left_out_before_the_fused_kernel(configs, name, mesh, it, taken, precision):
     prob = Problem.load(configs[name], (mesh,) * 3)
@@ -79,3 +81,22 @@ def test_samples_merged_in_parts(configs, counts, parts):
     # FP64 sums of a few thousand terms in another order
     np.testing.assert_allclose(lw, ref, rtol=1e-10, atol=1e-13 * np.abs(ref).max())
     assert (np.abs(xi - xi_ref) <= 1e-9 * np.abs(xi_ref).max()).all()
+
+
+def test_three_modes_with_triplets_left_out_match_the_oracle(configs):
+    prob = Problem.load(configs["fcc"], (23, 23, 23))
+    opts = Options(isotopescattering=False)
+    lists = QLists.monte_carlo(prob, opts)
+    sr = ScatteringRates(prob)
+    lw = sr.generate(opts, lists)
+    lw32 = sr.generate(Options(**{**opts.__dict__, "precision": "mixed"}), lists)
+    assert sr.last_routes()["prescreen"] == 1
+    sr.close()
+    # the rows of six points over the zone; a point's linewidths are averaged over degenerate
+    # modes, which leaves their sum
+    for q1 in np.linspace(2, prob.n_irr, 6).astype(int):
+        rows = np.nonzero(lists.row_q1 == q1)[0]
+        gamma, _, _ = orc.scattering(prob, opts, lists, rows=(rows[0], rows[-1] + 1))
+        np.testing.assert_allclose(lw[q1 - 1].sum(), gamma.sum(), rtol=1e-10)
+        # FP32 products and weights 1e-6 of a term, exponents of up to 32 amplify to 4e-6
+        np.testing.assert_allclose(lw32[q1 - 1].sum(), gamma.sum(), rtol=1e-4)
