@@ -213,8 +213,8 @@ __device__ __forceinline__ double k3_width6(const K3Smem &S, const PhononDev &P,
 // The same in FP32 for the mixed-precision kernels: the centre differences om1 - (+-om2 +-
 // om3) from FP32 pairs (centre_diff_f32, as accurate as the FP64 difference rounded to
 // FP32), the width, the exponent and the Gaussian in FP32 (expf), the occupation factors
-// and row weight from FP32 copies made once per mode, F in FP32. Relative error of a weight about 1e-6, against the 1e-5 of the BF16x3
-// contraction. LIVE: the entries carry their live Gaussians; otherwise those whose window holds
+// and row weight from FP32 copies made once per mode, F in FP32. Relative error of a weight
+// about 1e-6, against the 1e-5 of the BF16x3 contraction. LIVE: the entries carry their live Gaussians; otherwise those whose window holds
 // the FP32 mismatch with the screen's margins.
 template <int N, bool LIVE, typename Width6, typename PsiSq, typename Put>
 __device__ __forceinline__ void k3_survivors_f32(const K3Smem &S, const PhononDev &P, int q0, int q1, float perm,

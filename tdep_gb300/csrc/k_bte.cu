@@ -15,8 +15,9 @@ namespace tdg {
 namespace {
 
 // Two double-float accumulators (s, sl: high and low parts, one per column of a pair) +=
-// x * f for the columns' elements (x, xl) and F values (f, fl); nx = -x. The scalar form per component: p = x f, pe = fma(x, f, -p), cross = fma(x, fl,
-// xl f), TwoSum of s and p, sl += (e + pe) + cross. A subtraction a - b is fma(b, -1, a),
+// x * f for the columns' elements (x, xl) and F values (f, fl); nx = -x. The scalar form per
+// component: p = x f, pe = fma(x, f, -p), cross = fma(x, fl, xl f), TwoSum of s and p,
+// sl += (e + pe) + cross. A subtraction a - b is fma(b, -1, a),
 // rounded once as a - b is.
 __device__ __forceinline__ void df2_fma(float2 &s, float2 &sl, float2 x, float2 nx, float2 xl, float2 f, float2 fl) {
     const float2 m1 = make_float2(-1.f, -1.f);
@@ -207,8 +208,8 @@ __global__ void k_bte_compact(int n, int64_t ld, int n_row, const BteRow *rows, 
 // shrinks with the mesh (rocksalt: 21 % of the elements are not zero at 12^3, 3.2 % at 24^3;
 // perovskite 20 % at 16^3). Where few are left a row is the list of its non-zero elements, 12
 // bytes each, and the F sums are gathered, 32 bytes per column from L2: rocksalt 24^3, 75
-// iterations, call 22.9 -> 12.0 ms: an iteration takes 51 us where the dense products had
-// alone taken 217.
+// iterations, call 22.9 -> 12.0 ms: an iteration takes 48 us where the dense products had
+// alone taken 217; perovskite 16^3 102 us.
 // A CTA takes an item of up to 2048 elements of a row, four gathers in flight per thread; the
 // items' sums are added in order by k_bte_update.
 __global__ void __launch_bounds__(256) k_bte_products_sparse(BteDev d) {
@@ -345,8 +346,9 @@ __global__ void k_bte_images(int n_full, int n_op, const BteGroup *grp, const in
 }
 
 // F summed over the orbits of every group, as the products read it: [direction][column pair] of
-// (hi, hi, lo, lo), or per column for the sparse form. `lanes` consecutive threads share a column's points (a sixth of the
-// group's operations or so each: the chain of loads is what the kernel waits for).
+// (hi, hi, lo, lo), or per column for the sparse form. `lanes` consecutive threads share a
+// column's points (a sixth of the group's operations or so each: the chain of loads is what the
+// kernel waits for).
 __global__ void __launch_bounds__(256) k_bte_sums(BteDev d, const BteGroup *grp) {
     if (d.ctl->done) return;
     const BteGroup g = grp[blockIdx.y];

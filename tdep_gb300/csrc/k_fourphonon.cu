@@ -23,8 +23,8 @@
 // FP32 frequency pairs and the sums over modes in double-float, so that nothing per
 // quadruplet touches the FP64 pipe, which at 2 lanes per clock and SM was 83 % of this
 // kernel's time with FP64 centre differences and conversions).
-//   Measured: perovskite 8^3, 27 x 27 pairs, mixed 4.18 -> 1.75 ms (issue and shared-memory bound); rocksalt 8^3 FP64 1.13 ->
-// 0.79 ms (91 % of the FP64 pipe).
+//   Measured: perovskite 8^3, 27 x 27 pairs, mixed 4.18 -> 1.75 ms (issue and shared-memory
+// bound); rocksalt 8^3 FP64 1.13 -> 0.79 ms (91 % of the FP64 pipe).
 #include <cuda_runtime.h>
 
 #include <type_traits>

@@ -118,7 +118,8 @@ __global__ void __launch_bounds__(256) k_isotope(MeshDev m, PhononDev ph, const 
             strength = fma(fa * fa, disorder[a], strength);
         }
         const double dx = om1 - om2;
-        const double f0 = strength * prefactor * om1 * om2 * (exp_neg(dx * dx * 0.5 * invsig * invsig, ph.exp2tab) * kSqrt2PiInv * invsig);
+        const double gauss = exp_neg(dx * dx * 0.5 * invsig * invsig, ph.exp2tab) * kSqrt2PiInv * invsig;
+        const double f0 = strength * prefactor * om1 * om2 * gauss;
         if (f0 != 0.0) xi[(int64_t)r * ld + j] += f0 * om2 * inv1;
         sum += f0;
     }

@@ -16,8 +16,8 @@
 // table of exp(-2 pi i K / L), L = lcm of the mesh dimensions.
 //
 // With adaptive widths few mode triplets have a Gaussian inside its 8-sigma window (2 % at
-// rocksalt 24^3, 3-12 % at 9 to 15 modes), and at two atoms 67 % (12^3) to 76 % (24^3) of the q-triplets have none,
-// so the screen comes before the contraction and the contraction is driven by it:
+// rocksalt 24^3, 3-12 % at 9 to 15 modes), and at two atoms 67 % (12^3) to 76 % (24^3) of the
+// q-triplets have none, so the screen comes before the contraction and the contraction is driven by it:
 //   1. every mode triplet and each of the four Gaussians of get_dirac is screened in FP32
 //      against the window, with a relative margin of 1e-3 and an absolute margin far above
 //      FP32 rounding (a Gaussian the screen drops is exactly 0 in the reference); the

@@ -1933,10 +1933,15 @@ void symmetrize_kappa(const tdg_ctx *c, double *kappa) {
 namespace {
 // Sparse form of Xi's products: compacted matrices from kSparseBytes on (below, they stay in L2
 // and an iteration is latency; the count and its copy would cost more than they give) of which
-// less than kSparseDensity is not zero. Solves in us, sparse and dense, by the density of Xi:
-// 0.20 (perovskite 16^3) 1335 and 2053, 0.27 (perovskite 12^3) 581 and 756, 0.53 (16^3, one
-// width for all) 2140 and 1901, 0.68 (40-atom cell 4^3) 1057 and 919, 0.82 (rocksalt 24^3, one
-// width) 20 970 and 12 430.
+// less than kSparseDensity is not zero. Solves of a new matrix in us, sparse and dense, by the
+// density, at 12, 32 and 80 iterations:
+//   0.23 (rocksalt 18^3)    1323 and 1343,  2229 and 2758,  4633 and 6380
+//   0.32 (fcc 28^3)         3031 and 2939,  5715 and 6434,  12 370 and 14 990
+//   0.35 (perovskite 13^3)  1418 and 1292,  2580 and 2662,  5599 and 6127
+//   0.385 (rocksalt 18^3)   1551 and 1364,  2809 and 2783,  5991 and 6419
+//   0.41 (fcc 28^3)         3446 and 2987,  6696 and 6457,  14 670 and 15 030
+//   0.45 (rocksalt 18^3)    1646 and 1364,  3019 and 2794,  6490 and 6425
+// The two meet at 0.25, 0.38 and 0.43; the usual solution takes 10 to 75 iterations.
 constexpr int64_t kSparseBytes = (int64_t)128 << 20;
 constexpr double kSparseDensity = 0.4;
 constexpr int kSparseSample = 31;  // the rows of the first estimate: every 31st, of all modes in turn
